@@ -27,7 +27,7 @@
 namespace pgl {
 
 constexpr int kEmThreads = 512;
-constexpr int kStageFloats = 19200;  // floats per pipeline stage (two stages, 150 KB)
+constexpr int kStageFloats = 19968;  // floats per pipeline stage (two stages, 156 KB)
 
 // E-step passes shared between blocks.  Every block owns a board and a ring of
 // chunk slots in global memory.  For each E-step pass the home block publishes
@@ -38,7 +38,7 @@ constexpr int kStageFloats = 19200;  // floats per pipeline stage (two stages, 1
 // ring, from where the home block's loader warp copies them into the stages
 // with bulk copies.  The consumer warps add the chunks in chunk order.
 constexpr int kMaxStages = 8;                          // consumer pipeline stages
-constexpr int kMaxChunk = 768;                         // E-step samples per chunk at most (chunk divisor 1)
+constexpr int kMaxChunk = 416;                         // E-step samples per chunk at most (13 producer warps)
 constexpr uint32_t kRingFloats = 65536;                // ring per block (256 KB)
 constexpr uint32_t kRingMaxSlots = 64;
 constexpr unsigned long long kWaitNs = 2000000000ull;  // longest wait before the launch fails
@@ -50,8 +50,7 @@ constexpr uint32_t kMaxSharedChunks = kGrabMask - 4096u;
 enum EmError { kErrNone = 0, kErrChunkWait = 1, kErrSlotWait = 2, kErrCopyWait = 3, kErrLeafTooLarge = 4 };
 
 struct __align__(16) BoardParams {  // one pass as its home block publishes it
-  float4 lobeA[kMaxK + kMaxK / kLanes];
-  float2 lobeB[kMaxK];
+  float4 lobeP[3 * kMaxK / 2];
   const float4 *dirw;
   uint32_t count, seqBase, cnt, pad;
 };
@@ -81,6 +80,8 @@ struct EmShared {
   __align__(16) float pbuf[2 * kStageFloats];  // the two pipeline stages
   __align__(16) float4 lobeA[kMaxK + kMaxK / kLanes];  // mean direction, kappa (entry k + k / 8)
   float2 lobeB[kMaxK];                // normalisation, weight
+  __align__(16) float4 lobeP[3 * kMaxK / 2];  // E-step passes: two lobes per three entries, see pack_pairs
+  __align__(16) float ones[kMaxChunk + 48];  // the factor row of the chains that sum a_k w
   float lobeWInv[kMaxK];              // RN(1 / weight) for div_rcp
   float xch[2][kMaxK];
   uint32_t rcpTab[2048];
@@ -118,7 +119,7 @@ struct EmShared {
   float splitN0[kMaxK];                     // split passes: chi-square counts at the pass start
 };
 static_assert(offsetof(EmShared, pbuf) % 16 == 0 && offsetof(EmShared, lobeA) % 16 == 0 &&
-                  offsetof(EmShared, hp) % 16 == 0 && offsetof(EmShared, full) % 8 == 0,
+                  offsetof(EmShared, hp) % 16 == 0 && offsetof(EmShared, ones) % 16 == 0 && offsetof(EmShared, full) % 8 == 0,
               "128-bit shared loads");
 
 // cycle accounting of thread 0 (LeafProfile)
@@ -750,6 +751,19 @@ __device__ void pack_lobes(EmShared &S, int Kp) {
   }
 }
 
+// The lobe parameters of an E-step pass by pairs of lobes, for packed
+// arithmetic: {x0, x1, y0, y1}, {z0, z1, kappa0, kappa1}, {norm0, norm1, w0, w1}.
+__device__ void pack_pairs(EmShared &S, int Kp) {
+  const int i = int(threadIdx.x);
+  if (2 * i < Kp) {
+    const VMMState &v = S.vmm;
+    const int k = 2 * i;
+    S.lobeP[3 * i] = make_float4(v.mx[k], v.mx[k + 1], v.my[k], v.my[k + 1]);
+    S.lobeP[3 * i + 1] = make_float4(v.mz[k], v.mz[k + 1], v.kappa[k], v.kappa[k + 1]);
+    S.lobeP[3 * i + 2] = make_float4(v.norm[k], v.norm[k + 1], v.w[k], v.w[k + 1]);
+  }
+}
+
 // One producer lane's view of a sample: the E-step terms of its 8 lobes
 // (vector v), then the sample pdf and 1/pdf shared by all parts.
 struct PartTerms {
@@ -1229,46 +1243,30 @@ __device__ __forceinline__ unsigned long long grab_word(uint32_t gen, uint32_t c
 __device__ __forceinline__ uint32_t grab_gen(unsigned long long w) { return uint32_t(w >> (2 * kGrabIdxBits)); }
 __device__ __forceinline__ uint32_t grab_chunks(unsigned long long w) { return uint32_t(w >> kGrabIdxBits) & kGrabMask; }
 __device__ __forceinline__ uint32_t grab_next(unsigned long long w) { return uint32_t(w) & kGrabMask; }
-// Chunk shape of an E-step pass with `cnt` lobe vectors: consumers need
-// 4 Kp + 5 chains in three warps (chain_role), one warp loads
-// chunks made by other blocks, producers get
-// the remaining warps (P threads, one chunk of C = P / parts samples).  A
-// chunk holds rows of RS = C + 4 floats (RS / 4 odd, so the consumers'
-// 128-bit loads of 8 consecutive rows hit distinct banks): a_k for k < Kp
-// (the soft assignment t_k / pdf of valid samples, 0 otherwise), the
-// direction x, y, z, the weight of valid samples, then w log(pdf) and the
-// four unassigned-sample terms.
+// Chunk shape of an E-step pass with `cnt` lobe vectors: a consumer warp per
+// lobe vector and one for the per-sample rows (chain_role), one warp that
+// loads chunks made by other blocks, the rest produce, a sample per thread,
+// so that a chunk is one round of the producers.  A chunk holds rows of
+// RS = C + 4 floats (RS / 4 odd, so the 128-bit loads of 8 consecutive rows
+// hit distinct banks): a_k for k < Kp (the soft assignment t_k / pdf of valid
+// samples, 0 otherwise), the direction x, y, z, the weight of valid samples,
+// then w log(pdf) and the four unassigned-sample terms.
 struct EStepShape {
-  int cnt, Kp, parts, P, cons0, consWarps, C, C0, RS, stageFloats, stages, slots;
+  int cnt, Kp, P, cons0, consWarps, C, RS, stageFloats, stages, slots;
 };
-// Chunk k of a pass covers samples [chunk_begin, chunk_begin + chunk_size):
-// the first chunk is one producer round (the leaf's own producers make it
-// while helper blocks are still picking up the pass, and the consumers wait
-// for it), the others C samples.
-__device__ __forceinline__ uint32_t chunk_begin(const EStepShape &e, uint32_t k) {
-  return k == 0 ? 0u : uint32_t(e.C0) + (k - 1u) * uint32_t(e.C);
-}
-__device__ __forceinline__ int chunk_size(const EStepShape &e, uint32_t k) { return k == 0 ? e.C0 : e.C; }
+// Chunk k of a pass covers samples [chunk_begin, chunk_begin + C).
+__device__ __forceinline__ uint32_t chunk_begin(const EStepShape &e, uint32_t k) { return k * uint32_t(e.C); }
 __device__ __forceinline__ uint32_t chunk_count(const EStepShape &e, uint32_t count) {
-  return count <= uint32_t(e.C0) ? 1u : 1u + (count - uint32_t(e.C0) + uint32_t(e.C) - 1u) / uint32_t(e.C);
+  return (count + uint32_t(e.C) - 1u) / uint32_t(e.C);
 }
 __device__ __forceinline__ EStepShape estep_shape(int cnt, const EmTuning &tune) {
   EStepShape e;
   e.cnt = cnt;
   e.Kp = cnt * kLanes;
-  e.parts = cnt == 3 ? 4 : cnt;
-  e.consWarps = 3;  // a w and (d_x a) w | (d_y a) w and (d_z a) w | per-sample rows
+  e.consWarps = cnt == 4 ? 3 : cnt + 1;  // see chain_role
   e.cons0 = kEmThreads - 32 * e.consWarps;  // consumers: threads [cons0, 512)
   e.P = e.cons0 - 32;                       // producers [0, P), then the loader warp
-  // as many producer rounds per chunk as keep two stages in the pipeline
-  // buffer, up to kMaxChunk samples: a consumer warp spends a few hundred
-  // cycles per chunk outside its chains
-  const int slots = e.P / e.parts;
-  const int fit = (2 * kStageFloats / 2) / (e.Kp + 9) - 4;  // C + 4 floats per row, two stages
-  int rounds = min(kMaxChunk, fit) / slots;
-  rounds = rounds < 1 ? 1 : rounds;
-  e.C = ((rounds * slots) / tune.chunkDiv) & ~7;
-  e.C0 = min(e.C, slots & ~7);
+  e.C = (min(e.P, kMaxChunk) / tune.chunkDiv) & ~15;  // chains take 16 samples at a time
   e.RS = e.C + 4;
   e.stageFloats = (e.Kp + 9) * e.RS;
   e.stages = min(min(kMaxStages, tune.stageCap), 2 * kStageFloats / e.stageFloats);
@@ -1276,51 +1274,106 @@ __device__ __forceinline__ EStepShape estep_shape(int cnt, const EmTuning &tune)
   return e;
 }
 
+// Two lobes' E-step terms w norm fexp(kappa min(cos - 1, 0)) of direction d.
+// The multiplications are packed (each component rounds as its own multiply),
+// the additions are not: the compiler contracts a packed multiply and a packed
+// addition into one rounding.  The exponential's argument is not positive (or NaN):
+// below -100 the result is 0 either way, so the argument is clamped there
+// (NaN kept) and the scale's exponent clamped at 0; the rest is fexp's.
+__device__ __forceinline__ float2 pair_terms(float4 xy, float4 zk, float4 nw, V3 d) {
+  const float ln2Part1 = float(0.6931457519), ln2Part2 = float(1.4286067653e-6);
+  float2 c = __fmul2_rn(make_float2(d.z, d.z), make_float2(zk.x, zk.y));
+  c = __ffma2_rn(make_float2(d.y, d.y), make_float2(xy.z, xy.w), c);
+  c = __ffma2_rn(make_float2(d.x, d.x), make_float2(xy.x, xy.y), c);
+  // fminf(NaN, 0) is 0, as the reference's MINPS
+  float2 v = __fmul2_rn(make_float2(zk.z, zk.w), make_float2(fminf(c.x - 1.0f, 0.0f), fminf(c.y - 1.0f, 0.0f)));
+  asm("max.NaN.f32 %0, %0, 0fC2C80000;" : "+f"(v.x));  // -100
+  asm("max.NaN.f32 %0, %0, 0fC2C80000;" : "+f"(v.y));
+  const float2 sc = __fmul2_rn(v, make_float2(1.44269502162933349609375f, 1.44269502162933349609375f));
+  const float t0 = __fadd_rd(sc.x, 12582912.0f), t1 = __fadd_rd(sc.y, 12582912.0f);  // floor, see fexp
+  const float2 kr = make_float2(t0 - 12582912.0f, t1 - 12582912.0f);
+  const uint32_t e0 = uint32_t(max(int(f2u(t0)) - (0x4B400000 - 127), 0)) << 23;
+  const uint32_t e1 = uint32_t(max(int(f2u(t1)) - (0x4B400000 - 127), 0)) << 23;
+  float2 m = __fmul2_rn(kr, make_float2(ln2Part1, ln2Part1));
+  float2 x = make_float2(v.x - m.x, v.y - m.y);
+  m = __fmul2_rn(kr, make_float2(ln2Part2, ln2Part2));
+  x = make_float2(x.x - m.x, x.y - m.y);
+  float2 r = __fmul2_rn(x, make_float2(2.7555381529964506626129150390625e-4f, 2.7555381529964506626129150390625e-4f));
+  const float coeff[7] = {1.304379315115511417388916015625e-3f, 8.378830738365650177001953125e-3f,
+                          4.16539050638675689697265625e-2f, 0.166668415069580078125f,
+                          0.4999999105930328369140625f, 1.0f, 1.0f};
+#pragma unroll
+  for (int i = 0; i < 7; ++i) {
+    r = make_float2(r.x + coeff[i], r.y + coeff[i]);
+    r = i < 6 ? __fmul2_rn(x, r) : __fmul2_rn(r, make_float2(u2f(e0), u2f(e1)));
+  }
+  return __fmul2_rn(make_float2(nw.z, nw.w), __fmul2_rn(make_float2(nw.x, nw.y), r));
+}
+
 // Producers: `nthreads` threads (index t) fill chunk `chunk` into G (a stage
-// or a ring slot).  A sample's `parts` lanes are adjacent, so every warp holds
-// whole samples; rounds of nthreads / parts samples cover the chunk.
-template <bool kRing>
-__device__ void produce_estep_chunk(const EmShared &S, const EStepShape &e, const float4 *dirw, uint32_t count,
-                                    uint32_t chunk, float *G, int t, int nthreads) {
-  const int per = nthreads / e.parts;
-  const int v = t % e.parts;
-  const int RS = e.RS, Kp = e.Kp;
-  const int size = chunk_size(e, chunk);
+// or a ring slot), a sample per thread with the terms of all its lobes in
+// registers: the lobe vectors' sums stay in order without shuffles, the 32
+// lobes give independent work to cover the exponentials' latency, the lobe
+// parameters are broadcast loads and a warp stores whole rows.  Issue bound:
+// 30 FP32 operations and about as many issue slots per lobe, 15 cycles per
+// sample at 32 lobes alone on an SM.  A lane per lobe vector and sample, with
+// shuffles between the vectors, held a leaf of 30 lobes that no other block
+// helps at 39 cycles per sample and pass; it now takes 28.
+template <int kCnt>
+__device__ __noinline__ void produce_estep_rows(const EmShared &S, const EStepShape &e, const float4 *dirw,
+                                                uint32_t count, uint32_t chunk, float *G, int t, int nthreads) {
+  constexpr int Kp = kCnt * kLanes;
+  const int RS = e.RS;
   const uint32_t first = chunk_begin(e, chunk);
-  for (int base = 0; base < size; base += per) {
-    const int s = base + t / e.parts;
+  for (int s = t; s < e.C; s += nthreads) {
     const uint32_t idx = first + uint32_t(s);
-    const bool have = s < size && idx < count;
+    const bool have = idx < count;
     const float4 dw = have ? __ldcg(dirw + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
     const V3 d = mk(dw.x, dw.y, dw.z);
-    PartTerms T;
-    part_terms(S, e.cnt, e.parts, v, have, d, T);
-    if (s < size) {
-      const bool valid = have && T.valid;
-      if (v < e.cnt) {
+    float2 term[Kp / 2], p[kLanes / 2];
 #pragma unroll
-        for (int j = 0; j < kLanes; ++j) G[(v * kLanes + j) * RS + s] = valid ? T.t[j] * T.inv : 0.0f;
+    for (int v = 0; v < kCnt; ++v)
+#pragma unroll
+      for (int j = 0; j < kLanes / 2; ++j) {
+        const int i = v * (kLanes / 2) + j;
+        term[i] = pair_terms(S.lobeP[3 * i], S.lobeP[3 * i + 1], S.lobeP[3 * i + 2], d);
+        p[j] = v == 0 ? term[i] : make_float2(p[j].x + term[i].x, p[j].y + term[i].y);
       }
-      if (v == 0) {
-        const float w = dw.w;
-        const bool un = have && !T.valid;
-        float *X = G + Kp * RS + s;
-        X[0] = d.x;
-        X[RS] = d.y;
-        X[2 * RS] = d.z;
-        X[3 * RS] = valid ? w : 0.0f;
-        // the log-likelihood only drives the convergence test (its relative
-        // change against 0.005); it is not stored, so the single-precision
-        // logf (<= 1 ulp) stands in for the C library's here
-        X[4 * RS] = valid ? w * logf(T.pdf) : 0.0f;
-        X[5 * RS] = un ? w : 0.0f;
-        X[6 * RS] = un ? d.x * w : 0.0f;
-        X[7 * RS] = un ? d.y * w : 0.0f;
-        X[8 * RS] = un ? d.z * w : 0.0f;
-      }
+    const float pdf = ((p[0].x + p[0].y) + (p[1].x + p[1].y)) + ((p[2].x + p[2].y) + (p[3].x + p[3].y));  // reduce8
+    const bool valid = have && pdf > 1e-16f;
+    const float inv = valid ? rcp_avx2_tab(pdf, S.rcpTab) : 0.0f;
+    float *row = G + s;
+#pragma unroll
+    for (int i = 0; i < Kp / 2; ++i) {
+      const float2 a = __fmul2_rn(term[i], make_float2(inv, inv));
+      row[2 * i * RS] = valid ? a.x : 0.0f;
+      row[(2 * i + 1) * RS] = valid ? a.y : 0.0f;
     }
+    const float w = dw.w;
+    const bool un = have && !valid;
+    float *X = row + Kp * RS;
+    X[0] = d.x;
+    X[RS] = d.y;
+    X[2 * RS] = d.z;
+    X[3 * RS] = valid ? w : 0.0f;
+    // the log-likelihood only drives the convergence test (its relative
+    // change against 0.005); it is not stored, so the single-precision
+    // logf (<= 1 ulp) stands in for the C library's here
+    X[4 * RS] = valid ? w * logf(pdf) : 0.0f;
+    X[5 * RS] = un ? w : 0.0f;
+    X[6 * RS] = un ? d.x * w : 0.0f;
+    X[7 * RS] = un ? d.y * w : 0.0f;
+    X[8 * RS] = un ? d.z * w : 0.0f;
   }
-  if (kRing) fence_proxy_async();  // the ring is read by bulk copies
+}
+__device__ __forceinline__ void produce_estep_chunk(const EmShared &S, const EStepShape &e, const float4 *dirw,
+                                                    uint32_t count, uint32_t chunk, float *G, int t, int nthreads) {
+  switch (e.cnt) {
+    case 1: produce_estep_rows<1>(S, e, dirw, count, chunk, G, t, nthreads); break;
+    case 2: produce_estep_rows<2>(S, e, dirw, count, chunk, G, t, nthreads); break;
+    case 3: produce_estep_rows<3>(S, e, dirw, count, chunk, G, t, nthreads); break;
+    default: produce_estep_rows<4>(S, e, dirw, count, chunk, G, t, nthreads); break;
+  }
 }
 
 // A helper takes the next chunk of board `b` (one thread): only when that
@@ -1346,8 +1399,8 @@ __device__ int helper_take(EmShared &S, Board &b, bool paramsLoaded, uint32_t pa
 
 // A helper's chunk of board `b`: wait until its ring slot is free (unless
 // its slot was checked), fill the slot, then publish its sequence number.
-// Warp 15 holds no samples of a chunk (C <= 384 samples in lanes 0..479), so
-// its lane 0 takes the helper's next chunk meanwhile.
+// Warp 15 holds no samples of a chunk (C <= 416), so its lane 0 takes the
+// helper's next chunk meanwhile.
 __device__ void produce_for(EmShared &S, Board &b, float *ring, const EStepShape &e, const float4 *dirw,
                             uint32_t count, uint32_t seqBase, uint32_t chunk, bool exact, uint32_t paramsGen) {
   const int t = threadIdx.x;
@@ -1363,7 +1416,8 @@ __device__ void produce_for(EmShared &S, Board &b, float *ring, const EStepShape
     S.nextExact = x;
     S.hasNext = 1;
   }
-  produce_estep_chunk<true>(S, e, dirw, count, chunk, ring + size_t(slot) * e.stageFloats, t, kEmThreads);
+  produce_estep_chunk(S, e, dirw, count, chunk, ring + size_t(slot) * e.stageFloats, t, kEmThreads);
+  fence_proxy_async();  // the ring is read by bulk copies
   __syncthreads();
   if (t == 0) {
     __threadfence();
@@ -1372,167 +1426,132 @@ __device__ void produce_for(EmShared &S, Board &b, float *ring, const EStepShape
 }
 
 // Consumer side of the sum: a_k w, (d_q a_k) w or a per-sample row, in
-// sample order (the products are those of the reference's E-step).
-// Each chain keeps three groups of four samples in registers: the loads of a
-// group are issued two groups before it is added (a warp issues in order, so
-// loads placed after the dependent adds would wait for them).  The products
-// of two samples share one packed multiply (each component rounded as its
-// own multiply).  The loop is inlined into the consumer's chunk loop (a call
-// per chunk, with the registers it saves and restores, measured 4 % of the
-// first Update's EM launch) and works on 32-bit shared-memory addresses.
+// sample order (the products are those of the reference's E-step).  What
+// bounds a consumer warp is shared memory's way into registers: a warp's load
+// returns 64 bytes per cycle whatever it shares, so a register per lane costs
+// 2 cycles, and loads of 32 distinct rows of 16 bytes keep the data pipe of
+// the whole SM busy for 8 (both measured on one SM).  So a warp holds the four
+// chains of eight lobes, lane 8 q + j the chain q of lobe j, whose loads fetch 128
+// distinct bytes: three registers per sample and chain (a, d, w), 7.3 cycles per
+// sample alone, where a lane per lobe with two chains took 9.3 to 9.9.  With
+// four lobe vectors that would be four warps and 10 cycles (the data pipe again);
+// there a lane holds two lobes and shares their d and w, 11 cycles, and the
+// two warps saved produce (30.5 against 36 cycles per sample and pass in a
+// leaf of 30 lobes that no other block helps, before the producers' packed
+// arithmetic).  The sum of a_k w multiplies by
+// a row of ones, (1 a) w, which keeps its bits and the warp's lanes alike.
+// Sixteen samples per turn, in four groups of four: a group's products are
+// formed, its registers take the loads of the group four further on, then
+// the products are added, so that a load has three groups of additions (50
+// cycles) to arrive.  The products of two samples share one packed multiply
+// (each component rounded as its own multiply).  The last turn's loads run up
+// to 16 floats past the row; their values are not used.  The loop is inlined
+// into the consumer's chunk loop and works on 32-bit shared-memory addresses.
 __device__ __forceinline__ float4 lds4(uint32_t a) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
   return v;
 }
-template <int kKind>  // 0: a w, 1: (d a) w, 2: the value itself
-__device__ __forceinline__ void add_group(float &acc, float4 a, float4 d, float4 w) {
-  if (kKind == 2) {
-    acc += a.x;
-    acc += a.y;
-    acc += a.z;
-    acc += a.w;
-  } else {
-    float2 p0 = make_float2(a.x, a.y), p1 = make_float2(a.z, a.w);
-    if (kKind == 1) {
-      p0 = __fmul2_rn(make_float2(d.x, d.y), p0);
-      p1 = __fmul2_rn(make_float2(d.z, d.w), p1);
+__device__ __forceinline__ void add4(float &acc, float4 v) {
+  acc += v.x;
+  acc += v.y;
+  acc += v.z;
+  acc += v.w;
+}
+__device__ __forceinline__ float4 chain_terms(float4 a, float4 d, float4 w) {
+  const float2 p0 = __fmul2_rn(__fmul2_rn(make_float2(d.x, d.y), make_float2(a.x, a.y)), make_float2(w.x, w.y));
+  const float2 p1 = __fmul2_rn(__fmul2_rn(make_float2(d.z, d.w), make_float2(a.z, a.w)), make_float2(w.z, w.w));
+  return make_float4(p0.x, p0.y, p1.x, p1.y);
+}
+// Rows start at 32-bit shared addresses A0 (A1: the second lobe's), D, W
+// (bytes); n16 samples, a multiple of 16 (past the leaf's last sample the
+// rows hold zeros).
+template <bool kTwo>
+__device__ __forceinline__ float2 chain_rows(uint32_t A0, uint32_t A1, uint32_t D, uint32_t W, int n16, float2 acc) {
+  float4 a[4], b[4], d[4], w[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    a[g] = lds4(A0 + 16 * g);
+    if (kTwo) b[g] = lds4(A1 + 16 * g);
+    d[g] = lds4(D + 16 * g);
+    w[g] = lds4(W + 16 * g);
+  }
+#pragma unroll 1
+  for (int s = 0; s < n16; s += 16) {
+    A0 += 64;
+    A1 += 64;
+    D += 64;
+    W += 64;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const float4 p = chain_terms(a[g], d[g], w[g]);
+      a[g] = lds4(A0 + 16 * g);
+      if (kTwo) {
+        const float4 q = chain_terms(b[g], d[g], w[g]);
+        b[g] = lds4(A1 + 16 * g);
+        d[g] = lds4(D + 16 * g);
+        w[g] = lds4(W + 16 * g);
+        acc.x += p.x;
+        acc.y += q.x;
+        acc.x += p.y;
+        acc.y += q.y;
+        acc.x += p.z;
+        acc.y += q.z;
+        acc.x += p.w;
+        acc.y += q.w;
+      } else {
+        d[g] = lds4(D + 16 * g);
+        w[g] = lds4(W + 16 * g);
+        add4(acc.x, p);
+      }
     }
-    p0 = __fmul2_rn(p0, make_float2(w.x, w.y));
-    p1 = __fmul2_rn(p1, make_float2(w.z, w.w));
-    acc += p0.x;
-    acc += p0.y;
-    acc += p1.x;
-    acc += p1.y;
-  }
-}
-template <int kKind>
-__device__ __forceinline__ float4 lds_if(uint32_t a) {
-  return kKind ? lds4(a) : make_float4(0.f, 0.f, 0.f, 0.f);
-}
-// Rows start at 32-bit shared addresses A, D, W (bytes); n4 samples.
-template <int kKind>
-__device__ __forceinline__ float chain_rows(uint32_t A, uint32_t D, uint32_t W, int n4, float acc) {
-  constexpr int kD = kKind == 1, kW = kKind != 2;
-  // rows hold C + 4 >= 12 floats: the first two groups can be read even
-  // when n4 is smaller
-  float4 a0 = lds4(A), d0 = lds_if<kD>(D), w0 = lds_if<kW>(W);
-  float4 a1 = lds4(A + 16), d1 = lds_if<kD>(D + 16), w1 = lds_if<kW>(W + 16);
-  int s = 0;
-  for (; s + 12 <= n4; s += 12) {
-    const uint32_t o2 = uint32_t(s + 8) * 4u;
-    const float4 a2 = lds4(A + o2), d2 = lds_if<kD>(D + o2), w2 = lds_if<kW>(W + o2);
-    add_group<kKind>(acc, a0, d0, w0);
-    const uint32_t o3 = uint32_t(s + 12 < n4 ? s + 12 : 0) * 4u;
-    a0 = lds4(A + o3);
-    d0 = lds_if<kD>(D + o3);
-    w0 = lds_if<kW>(W + o3);
-    add_group<kKind>(acc, a1, d1, w1);
-    const uint32_t o4 = uint32_t(s + 16 < n4 ? s + 16 : 0) * 4u;
-    a1 = lds4(A + o4);
-    d1 = lds_if<kD>(D + o4);
-    w1 = lds_if<kW>(W + o4);
-    add_group<kKind>(acc, a2, d2, w2);
-  }
-  if (s < n4) add_group<kKind>(acc, a0, d0, w0);
-  if (s + 4 < n4) add_group<kKind>(acc, a1, d1, w1);
-  if (s + 8 < n4) {
-    const uint32_t o2 = uint32_t(s + 8) * 4u;
-    add_group<kKind>(acc, lds4(A + o2), lds_if<kD>(D + o2), lds_if<kW>(W + o2));
   }
   return acc;
 }
-// Two chains of lobe k in one consumer thread, so that the thread reads the
-// a_k row once for both: kind 0 sums a_k w and (d_x a_k) w, kind 1 sums
-// (d_y a_k) w and (d_z a_k) w.  The two chains' additions alternate (each
-// chain still adds its terms in sample order, one rounding per addition).
-template <int kKind>
-__device__ __forceinline__ void add_group2(float &acc0, float &acc1, float4 a, float4 d0, float4 d1, float4 w) {
-  const float2 a01 = make_float2(a.x, a.y), a23 = make_float2(a.z, a.w);
-  const float2 w01 = make_float2(w.x, w.y), w23 = make_float2(w.z, w.w);
-  float2 p01, p23;
-  if (kKind == 0) {
-    p01 = __fmul2_rn(a01, w01);
-    p23 = __fmul2_rn(a23, w23);
-  } else {
-    p01 = __fmul2_rn(__fmul2_rn(make_float2(d0.x, d0.y), a01), w01);
-    p23 = __fmul2_rn(__fmul2_rn(make_float2(d0.z, d0.w), a23), w23);
+__device__ __forceinline__ float value_rows(uint32_t R, int n16, float acc) {
+  float4 a[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) a[g] = lds4(R + 16 * g);
+#pragma unroll 1
+  for (int s = 0; s < n16; s += 16) {
+    R += 64;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const float4 p = a[g];
+      a[g] = lds4(R + 16 * g);
+      add4(acc, p);
+    }
   }
-  const float2 q01 = __fmul2_rn(__fmul2_rn(make_float2(d1.x, d1.y), a01), w01);
-  const float2 q23 = __fmul2_rn(__fmul2_rn(make_float2(d1.z, d1.w), a23), w23);
-  acc0 += p01.x;
-  acc1 += q01.x;
-  acc0 += p01.y;
-  acc1 += q01.y;
-  acc0 += p23.x;
-  acc1 += q23.x;
-  acc0 += p23.y;
-  acc1 += q23.y;
+  return acc;
 }
-// Rows start at 32-bit shared addresses A, D0 (kind 1 only), D1, W (bytes);
-// n4 samples; three groups of four samples in flight as in chain_rows.
-template <int kKind>
-__device__ __forceinline__ float2 chain_rows2(uint32_t A, uint32_t D0, uint32_t D1, uint32_t W, int n4, float2 acc) {
-  constexpr int kD0 = kKind == 1;
-  float a0c = acc.x, a1c = acc.y;
-  float4 a0 = lds4(A), e0 = lds_if<kD0>(D0), f0 = lds4(D1), w0 = lds4(W);
-  float4 a1 = lds4(A + 16), e1 = lds_if<kD0>(D0 + 16), f1 = lds4(D1 + 16), w1 = lds4(W + 16);
-  int s = 0;
-  for (; s + 12 <= n4; s += 12) {
-    const uint32_t o2 = uint32_t(s + 8) * 4u;
-    const float4 a2 = lds4(A + o2), e2 = lds_if<kD0>(D0 + o2), f2 = lds4(D1 + o2), w2 = lds4(W + o2);
-    add_group2<kKind>(a0c, a1c, a0, e0, f0, w0);
-    const uint32_t o3 = uint32_t(s + 12 < n4 ? s + 12 : 0) * 4u;
-    a0 = lds4(A + o3);
-    e0 = lds_if<kD0>(D0 + o3);
-    f0 = lds4(D1 + o3);
-    w0 = lds4(W + o3);
-    add_group2<kKind>(a0c, a1c, a1, e1, f1, w1);
-    const uint32_t o4 = uint32_t(s + 16 < n4 ? s + 16 : 0) * 4u;
-    a1 = lds4(A + o4);
-    e1 = lds_if<kD0>(D0 + o4);
-    f1 = lds4(D1 + o4);
-    w1 = lds4(W + o4);
-    add_group2<kKind>(a0c, a1c, a2, e2, f2, w2);
-  }
-  if (s < n4) add_group2<kKind>(a0c, a1c, a0, e0, f0, w0);
-  if (s + 4 < n4) add_group2<kKind>(a0c, a1c, a1, e1, f1, w1);
-  if (s + 8 < n4) {
-    const uint32_t o2 = uint32_t(s + 8) * 4u;
-    add_group2<kKind>(a0c, a1c, lds4(A + o2), lds_if<kD0>(D0 + o2), lds4(D1 + o2), lds4(W + o2));
-  }
-  return make_float2(a0c, a1c);
-}
-// The chains of consumer thread c: three consumer warps, lane k of the first
-// summing a_k w and (d_x a_k) w, lane k of the second (d_y a_k) w and
-// (d_z a_k) w, lanes 0-4 of the third the five per-sample rows; other lanes
-// are idle (kind -1).  Every a_k row is read by one lane only; the direction
-// and weight rows are read by whole warps at one address (broadcasts).
+// The chains of consumer thread c: lane 8 q + j of chain warp v holds lobe
+// 8 v + j, with four lobe vectors lobes 16 v + j and 16 v + 8 + j; q = 0 is the
+// sum of a_k w, q = 1..3 of (d_q a_k) w.  Lanes 0-4 of the last warp hold the
+// five per-sample rows (kind 2; the other lanes repeat the last of them).
 struct ChainRole {
-  int kind, k, q;
+  int kind, k, q;  // 0: lobes k and k + 8; 1: lobe k; 2: row k
 };
 __device__ __forceinline__ ChainRole chain_role(const EStepShape &e, int c) {
   const int cw = c >> 5, lane = c & 31;
-  ChainRole r{-1, 0, 0};
-  if (cw < 2) {
-    if (lane < e.Kp) r = ChainRole{cw, lane, 0};
-  } else if (cw == 2 && lane < 5) {
-    r = ChainRole{2, lane, 0};
-  }
-  return r;
+  if (cw + 1 == e.consWarps) return ChainRole{2, min(lane, 4), 0};
+  return e.cnt == 4 ? ChainRole{0, 2 * cw * kLanes + (lane & 7), lane >> 3}
+                    : ChainRole{1, cw * kLanes + (lane & 7), lane >> 3};
 }
-__device__ __forceinline__ void estep_chunk_chain(const float *B, const EStepShape &e, const ChainRole &role, int n4,
-                                                  float2 &acc) {
+__device__ __forceinline__ void estep_chunk_chain(const EmShared &S, const float *B, const EStepShape &e,
+                                                  const ChainRole &role, int n16, float2 &acc) {
   const int Kp = e.Kp;
   const uint32_t base = smem_u32(B), row = uint32_t(e.RS) * 4u;
-  const uint32_t A = base + uint32_t(role.k) * row, X = base + uint32_t(Kp) * row, W = base + uint32_t(Kp + 3) * row;
-  if (role.kind == 0) {
-    acc = chain_rows2<0>(A, X, X, W, n4, acc);
-  } else if (role.kind == 1) {
-    acc = chain_rows2<1>(A, X + row, X + 2u * row, W, n4, acc);
-  } else if (role.kind == 2) {
-    const uint32_t R = base + uint32_t(Kp + 4 + role.k) * row;
-    acc.x = chain_rows<2>(R, R, R, n4, acc.x);
+  if (role.kind != 2) {
+    const uint32_t X = base + uint32_t(Kp) * row, W = X + 3u * row;
+    // the row of ones starts four banks after the z row, so the four
+    // direction rows of a warp's load lie in distinct banks
+    const uint32_t ones = smem_u32(S.ones);
+    const uint32_t D = role.q == 0 ? ones + ((X + 3u * row - ones) & 127u) : X + uint32_t(role.q - 1) * row;
+    const uint32_t A = base + uint32_t(role.k) * row;
+    if (role.kind == 0) acc = chain_rows<true>(A, A + uint32_t(kLanes) * row, D, W, n16, acc);
+    else acc = chain_rows<false>(A, A, D, W, n16, acc);
+  } else {
+    acc.x = value_rows(base + uint32_t(Kp + 4 + role.k) * row, n16, acc.x);
   }
 }
 
@@ -1561,15 +1580,15 @@ __device__ __forceinline__ float2 consume_estep(EmShared &S, const EStepShape &e
     const long long w0 = clock64();
     if (!mbar_wait(&S.full[st], use_parity(S, e, k), &S.abortAt, k, S.err)) break;
     waited += clock64() - w0;
-    const int n = int(min(uint32_t(chunk_size(e, k)), count - chunk_begin(e, k)));
-    estep_chunk_chain(S.pbuf + st * e.stageFloats, e, role, (n + 3) & ~3, acc);
+    const int n = int(min(uint32_t(e.C), count - chunk_begin(e, k)));
+    estep_chunk_chain(S, S.pbuf + st * e.stageFloats, e, role, (n + 15) & ~15, acc);
     __syncwarp();
     if (lane == 0) {
       __threadfence_block();  // this warp's reads of the stage come first
       reinterpret_cast<volatile uint32_t *>(S.warpDone)[r >> 5] = k + 1u;
     }
   }
-  if (r == 32) S.prof.cycWaitE += uint64_t(waited);
+  if (r == 0) S.prof.cycWaitE += uint64_t(waited);
   return acc;
 }
 
@@ -1718,9 +1737,9 @@ __device__ void produce_own(EmShared &S, const EStepShape &e, const LeafSamples 
     const uint32_t k = uint32_t(chunk);
     const int st = int(k % uint32_t(e.stages));
     unsigned long long w = 0;
-    const bool early = t == 0 && alone && !has_error(S.err);
+    const bool early = t == 0 && alone;
     if (early) w = atomicAdd(&b.grab, 1ull);
-    produce_estep_chunk<false>(S, e, L.dirw, L.count, k, S.pbuf + st * e.stageFloats, t, e.P);
+    produce_estep_chunk(S, e, L.dirw, L.count, k, S.pbuf + st * e.stageFloats, t, e.P);
     bar_named(3, e.P);
     if (t == 0) {
       mbar_arrive(&S.full[st]);
@@ -1756,7 +1775,7 @@ __device__ void pass_estep(EmShared &S, const LeafSamples &L) {
     S.abortAt = has_error(S.err) ? 0u : 0xFFFFFFFFu;
   }
   if (tid < kEmThreads / 32) S.warpDone[tid] = 0;
-  pack_lobes(S, Kp);
+  pack_pairs(S, Kp);
   __syncthreads();
   const uint32_t seqBase = S.seqBase;
   if (tid == 0) {  // publish the pass on the board
@@ -1764,8 +1783,7 @@ __device__ void pass_estep(EmShared &S, const LeafSamples &L) {
     const uint32_t gen = S.gen % kGrabGenMask + 1u;
     S.gen = gen;
     BoardParams &bp = b.params[gen & 1u];
-    for (int i = 0; i < Kp + Kp / kLanes; ++i) bp.lobeA[i] = S.lobeA[i];
-    for (int i = 0; i < Kp; ++i) bp.lobeB[i] = S.lobeB[i];
+    for (int i = 0; i < 3 * Kp / 2; ++i) bp.lobeP[i] = S.lobeP[i];
     bp.dirw = L.dirw;
     bp.count = L.count;
     bp.seqBase = seqBase;
@@ -1780,17 +1798,15 @@ __device__ void pass_estep(EmShared &S, const LeafSamples &L) {
   else acc = consume_estep(S, e, N, L.count);
   const long long cyc = clock64() - t0;
   if (tid == 0) S.prof.cycProdE += uint64_t(cyc);
-  if (tid == e.cons0 + 32) S.prof.cycConsE += uint64_t(cyc);
+  if (tid == e.cons0) S.prof.cycConsE += uint64_t(cyc);
   __syncthreads();
   if (tid >= e.cons0) {
     const ChainRole role = chain_role(e, tid - e.cons0);
-    if (role.kind == 0) {
-      S.cur.w[role.k] = acc.x;
-      S.cur.dx[role.k] = acc.y;
-    } else if (role.kind == 1) {
-      S.cur.dy[role.k] = acc.x;
-      S.cur.dz[role.k] = acc.y;
-    } else if (role.kind == 2) {
+    if (role.kind != 2) {
+      float *sum = role.q == 0 ? S.cur.w : role.q == 1 ? S.cur.dx : role.q == 2 ? S.cur.dy : S.cur.dz;
+      sum[role.k] = acc.x;
+      if (role.kind == 0) sum[role.k + kLanes] = acc.y;
+    } else if ((tid & 31) < 5) {
       const int x = role.k;
       if (x == 0) S.ll = acc.x;
       else if (x == 1) S.un.sw = acc.x;
@@ -1911,8 +1927,7 @@ __device__ void help_others(EmShared &S, Board *boards, float *rings, const uint
         if (tid == 0) __threadfence();
         __syncthreads();
         const BoardParams &src = b.params[gen & 1u];
-        for (int i = tid; i < kMaxK + kMaxK / kLanes; i += kEmThreads) S.lobeA[i] = __ldcg(&src.lobeA[i]);
-        for (int i = tid; i < kMaxK; i += kEmThreads) S.lobeB[i] = __ldcg(&src.lobeB[i]);
+        for (int i = tid; i < 3 * kMaxK / 2; i += kEmThreads) S.lobeP[i] = __ldcg(&src.lobeP[i]);
         if (tid == 0) {
           S.hp.dirw = reinterpret_cast<const float4 *>(__ldcg(reinterpret_cast<const unsigned long long *>(&src.dirw)));
           S.hp.count = __ldcg(&src.count);
@@ -2350,6 +2365,7 @@ em_leaf_kernel(const LeafTask *tasks, uint32_t numTasks, unsigned int *queue, Em
   __shared__ uint64_t afterSplit, afterMerge;
   for (int i = threadIdx.x; i < 2048; i += blockDim.x) S.rcpTab[i] = rcp_seed(uint32_t(i));
   for (int i = threadIdx.x; i < 64; i += blockDim.x) S.own[i] = 0;
+  for (int i = threadIdx.x; i < kMaxChunk + 48; i += blockDim.x) S.ones[i] = 1.0f;
   if (threadIdx.x == 0) {
     S.board = boards + blockIdx.x;
     S.ring = rings + size_t(blockIdx.x) * kRingFloats;
