@@ -24,6 +24,22 @@ void check(cudaError_t e, const char *what) {
 // The host C library's expf/cosf/sinf exception table (gen_libm_exceptions.cpp),
 // written by the build next to this library as libm_exceptions.bin, copied
 // to device memory that lives until the process exits.
+// The largest distance, relative to the value, between a listed input's value
+// and the rounding boundary beside the host's result (see LibmTables);
+// results that are not normal floats are left out (they are always looked up).
+template <typename F>
+static float libm_margin(const float2 *v, uint32_t n, F exact) {
+  double worst = 0.0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const double d = exact(double(v[i].x));
+    const float f = float(d), y = v[i].y;
+    if (!(std::fabs(d) >= double(FLT_MIN)) || !std::isfinite(f) || !std::isfinite(y)) continue;
+    const float g = y != f ? y : std::nextafter(f, d > double(f) ? INFINITY : -INFINITY);
+    worst = std::max(worst, std::fabs(d - 0.5 * (double(f) + double(g))) / std::fabs(d));
+  }
+  return float(worst * 1.001);
+}
+
 static LibmTables load_libm_tables() {
   Dl_info info{};
   if (!dladdr(reinterpret_cast<void *>(&load_libm_tables), &info) || !info.dli_fname)
@@ -44,7 +60,22 @@ static LibmTables load_libm_tables() {
     check(cudaMalloc(&d, v.size() * sizeof(float2)), "libm table");
     check(cudaMemcpy(d, v.data(), v.size() * sizeof(float2), cudaMemcpyHostToDevice), "libm table");
   }
-  LibmTables t;
+  LibmTables t{};
+  t.expMargin = libm_margin(v.data(), n[0], [](double x) { return std::exp(x); });
+  t.cosMargin = libm_margin(v.data() + n[0], n[1], [](double x) { return std::cos(x); });
+  if (n[0] > 0) {
+    // about one expf entry per bucket of the float order
+    const uint32_t first = float_key(v[0].x), span = float_key(v[n[0] - 1].x) - first;
+    while ((span >> t.expfShift) >= n[0]) ++t.expfShift;
+    t.expfBuckets = (span >> t.expfShift) + 1;
+    std::vector<uint32_t> at(t.expfBuckets + 1, n[0]);
+    for (uint32_t i = n[0]; i-- > 0;) at[(float_key(v[i].x) - first) >> t.expfShift] = i;
+    for (uint32_t j = t.expfBuckets; j-- > 0;) at[j] = std::min(at[j], at[j + 1]);
+    uint32_t *dAt = nullptr;
+    check(cudaMalloc(&dAt, at.size() * sizeof(uint32_t)), "libm index");
+    check(cudaMemcpy(dAt, at.data(), at.size() * sizeof(uint32_t), cudaMemcpyHostToDevice), "libm index");
+    t.expfAt = dAt;
+  }
   t.expf = d;
   t.cosf = d ? d + n[0] : nullptr;
   t.sinf = d ? d + n[0] + n[1] : nullptr;
