@@ -47,10 +47,16 @@ constexpr uint32_t kGrabMask = (1u << kGrabIdxBits) - 1u;
 constexpr uint32_t kGrabGenMask = (1u << 20) - 1u;
 constexpr uint32_t kMaxSharedChunks = kGrabMask - 4096u;
 
+// Lobe parameters by pairs: entry pair_at(k) + c, three entries per pair of
+// lobes and one of padding per lobe vector, so that lanes on different vectors
+// read distinct banks.
+constexpr int kPairEntries = (3 * kLanes / 2 + 1) * (kMaxK / kLanes);
+__host__ __device__ constexpr int pair_at(int k) { return (k / kLanes) * (3 * kLanes / 2 + 1) + 3 * ((k % kLanes) / 2); }
+
 enum EmError { kErrNone = 0, kErrChunkWait = 1, kErrSlotWait = 2, kErrCopyWait = 3, kErrLeafTooLarge = 4 };
 
 struct __align__(16) BoardParams {  // one pass as its home block publishes it
-  float4 lobeP[3 * kMaxK / 2];
+  float4 lobeP[kPairEntries];
   const float4 *dirw;
   uint32_t count, seqBase, cnt, pad;
 };
@@ -76,13 +82,11 @@ struct EmShared {
   SuffState cur;      // statistics of the current EM iteration
   SuffState temp;     // statistics of a partial refit
   SplitState lsplit;  // split statistics used by the recursive splitting
-  Frame invFrame[kMaxK];
   __align__(16) float pbuf[2 * kStageFloats];  // the two pipeline stages
-  __align__(16) float4 lobeA[kMaxK + kMaxK / kLanes];  // mean direction, kappa (entry k + k / 8)
-  float2 lobeB[kMaxK];                // normalisation, weight
-  __align__(16) float4 lobeP[3 * kMaxK / 2];  // E-step passes: two lobes per three entries, see pack_pairs
+  __align__(16) float4 lobeP[kPairEntries];   // see pack_pairs
+  __align__(16) float4 frameP[kPairEntries];  // split passes: rows x and y of the lobes' inverse frames
   __align__(16) float ones[kMaxChunk + 48];  // the factor row of the chains that sum a_k w
-  float lobeWInv[kMaxK];              // RN(1 / weight) for div_rcp
+  float2 lobeW[kMaxK];  // distance passes: weight, its reciprocal (0: divide)
   float xch[2][kMaxK];
   uint32_t rcpTab[2048];
   float cost[kMaxK][kMaxK];  // merge cost of components i < j (cost[i][j])
@@ -115,10 +119,8 @@ struct EmShared {
   uint32_t nextGen;
   uint32_t scanRem[kEmThreads / 32];
   int scanIdx[kEmThreads / 32];
-  uint32_t validPerWarp[kEmThreads / 32];  // split passes: valid samples per producer warp
-  float splitN0[kMaxK];                     // split passes: chi-square counts at the pass start
 };
-static_assert(offsetof(EmShared, pbuf) % 16 == 0 && offsetof(EmShared, lobeA) % 16 == 0 &&
+static_assert(offsetof(EmShared, pbuf) % 16 == 0 && offsetof(EmShared, lobeP) % 16 == 0 &&
                   offsetof(EmShared, hp) % 16 == 0 && offsetof(EmShared, ones) % 16 == 0 && offsetof(EmShared, full) % 8 == 0,
               "128-bit shared loads");
 
@@ -652,25 +654,15 @@ __device__ void split_merge_stats(SplitState &s, int I, int J, float wI, V3 muI,
 //
 // Distance and split-statistics passes run in the home block as a two-stage
 // pipeline over chunks of samples, with one __syncthreads per chunk and two
-// shared-memory stages:
-//   producers (threads [0, C * parts)): `parts` adjacent lanes per sample, one
-//     SIMD vector of 8 lobes each; the lobe terms in registers, the sample pdf
-//     (vfloat8 lane sums carried from part to part in lobe-vector order, then
-//     the 8-lane reduction), then the finished term of every accumulator for
-//     their lobes written to stage (c & 1);
-//   consumers (threads [P, 512)): one thread per accumulator (for example the
-//     x component of lobe 7's weighted direction sum), adding the chunk in
-//     stage ((c - 1) & 1) in sample order.
-// The consumers keep the reference's summation order (sequential over samples
-// within each SIMD lane).  Samples that the reference skips (pdf <= 1e-16)
-// contribute a term of exactly +-0, which leaves an accumulator unchanged:
-// accumulators start at +0 and a round-to-nearest sum that starts at +0 never
-// becomes -0.  Consumer lanes only load and add, so chain warps do not diverge
-// (chi-square lanes have a warp of their own).  Each pass gives the consumers
-// the warps its chains need and the producers the rest; the chunk size
-// follows from the stage memory and the producer threads.  E-step passes
-// (most of the work) use the same roles, with a loader warp besides, and can
-// take chunks made by other blocks (below).
+// shared-memory stages: producer warps write a chunk's terms to stage (c & 1)
+// while consumer lanes add the chunk in stage ((c - 1) & 1) in sample order,
+// a lane per lobe.  The consumers keep the reference's summation order
+// (sequential over samples within each SIMD lane).  Samples that the reference
+// skips (pdf <= 1e-16) contribute a term of exactly +-0, which leaves an
+// accumulator unchanged: accumulators start at +0 and a round-to-nearest sum
+// that starts at +0 never becomes -0.  E-step passes (most of the work) use the
+// same roles, with a loader warp besides, and can take chunks made by other
+// blocks (below).
 
 struct LeafSamples {
   const float4 *dirw;  // direction xyz, weight
@@ -678,49 +670,6 @@ struct LeafSamples {
   const float *dist;
   uint32_t count;
 };
-
-enum PassKind { kPassDistance = 1, kPassSplit = 2 };  // in-block passes
-
-// Thread roles and stage layout of one pass (the same in every thread).
-struct PassShape {
-  int P;        // threads [P, kEmThreads) consume
-  int parts;    // producer lanes per sample (lobe vectors, 3 rounded to 4)
-  int C;        // samples per chunk
-  int threads;  // producer threads: C * parts, a multiple of 32
-  int R;        // row stride of the per-(lobe, sample) rows: C + 2 floats
-  int stage;    // floats per stage
-};
-template <PassKind kind>
-__device__ __forceinline__ PassShape pass_shape(int Kp, int budget = kStageFloats) {
-  // rows: one per (accumulator, lobe); extra: per-sample arrays
-  int consWarps, rows, extra;
-  if (kind == kPassDistance) {  // 2 Kp chains
-    consWarps = (2 * Kp + 31) / 32;
-    rows = 2 * Kp;
-    extra = 0;
-  } else {  // 5 Kp product chains, two per lane, then (from a warp boundary) Kp chi-square chains
-    consWarps = (5 * Kp + 63) / 64 + 1;
-    rows = 7 * Kp;  // a, a w, three covariance terms, chi, 1/n
-    extra = 1;      // validity
-  }
-  PassShape p;
-  const int cnt = Kp / kLanes;
-  p.parts = cnt == 3 ? 4 : cnt;
-  p.P = kEmThreads - 32 * consWarps;
-  int c = (budget - 2 * rows) / (rows + extra);
-  const int byThreads = p.P / p.parts;
-  c = c < byThreads ? c : byThreads;
-  // C * parts a multiple of 32 (whole warps) and C a multiple of 8.  Rows of
-  // C + 2 floats: (C + 2) / 2 is odd, so the consumers' 64-bit loads of
-  // consecutive rows fall in distinct banks, and rows 8 apart are 16 banks
-  // apart, so two parts of a sample store to distinct banks.
-  const int mult = 32 / p.parts > 8 ? 32 / p.parts : 8;
-  p.C = c - c % mult;
-  p.threads = p.C * p.parts;
-  p.R = p.C + 2;
-  p.stage = rows * p.R + extra * p.C;
-  return p;
-}
 
 // x86 RCPSS from the block's shared copy of the table (per-lane gathers from
 // constant memory would serialise)
@@ -739,391 +688,475 @@ __device__ __forceinline__ float rcp_avx2_tab(float a, const uint32_t *tab) {
   return r * fmaf_(-r, a, 2.0f);
 }
 
-// Lobe parameters packed for the producers' broadcast loads.
-__device__ void pack_lobes(EmShared &S, int Kp) {
-  const int tid = threadIdx.x;
-  if (tid < Kp) {
-    const VMMState &v = S.vmm;
-    // entry k + k / 8: the parts of a sample read lobes k and k + 8 at once
-    S.lobeA[tid + (tid >> 3)] = make_float4(v.mx[tid], v.my[tid], v.mz[tid], v.kappa[tid]);
-    S.lobeB[tid] = make_float2(v.norm[tid], v.w[tid]);
-    S.lobeWInv[tid] = rcp_for_div(v.w[tid]);
-  }
-}
-
-// The lobe parameters of an E-step pass by pairs of lobes, for packed
-// arithmetic: {x0, x1, y0, y1}, {z0, z1, kappa0, kappa1}, {norm0, norm1, w0, w1}.
+// The lobe parameters of a pass by pairs of lobes, for packed arithmetic:
+// {x0, x1, y0, y1}, {z0, z1, kappa0, kappa1}, {norm0, norm1, w0, w1}.
 __device__ void pack_pairs(EmShared &S, int Kp) {
-  const int i = int(threadIdx.x);
-  if (2 * i < Kp) {
+  const int k = 2 * int(threadIdx.x);
+  if (k < Kp) {
     const VMMState &v = S.vmm;
-    const int k = 2 * i;
-    S.lobeP[3 * i] = make_float4(v.mx[k], v.mx[k + 1], v.my[k], v.my[k + 1]);
-    S.lobeP[3 * i + 1] = make_float4(v.mz[k], v.mz[k + 1], v.kappa[k], v.kappa[k + 1]);
-    S.lobeP[3 * i + 2] = make_float4(v.norm[k], v.norm[k + 1], v.w[k], v.w[k + 1]);
+    float4 *o = S.lobeP + pair_at(k);
+    o[0] = make_float4(v.mx[k], v.mx[k + 1], v.my[k], v.my[k + 1]);
+    o[1] = make_float4(v.mz[k], v.mz[k + 1], v.kappa[k], v.kappa[k + 1]);
+    o[2] = make_float4(v.norm[k], v.norm[k + 1], v.w[k], v.w[k + 1]);
   }
 }
 
-// One producer lane's view of a sample: the E-step terms of its 8 lobes
-// (vector v), then the sample pdf and 1/pdf shared by all parts.
-struct PartTerms {
-  float t[kLanes];
-  float pdf, inv;
-  bool valid;
-};
-__device__ __forceinline__ void part_terms(const EmShared &S, int cnt, int parts, int v, bool have, V3 d,
-                                           PartTerms &T) {
-  const unsigned full = 0xFFFFFFFFu;
-  if (have && v < cnt) {
+// Two lobes' terms w norm fexp(kappa min(cos - 1, 0)) of direction d, the
+// multiplications packed.  The exponential's argument is not positive (or
+// NaN): below -100 the result is 0 either way, so the argument is clamped there
+// (NaN kept) and the scale's exponent clamped at 0; the rest is fexp's.
+__device__ __forceinline__ float2 pair_terms(const float4 *P, V3 d) {
+  const float ln2Part1 = float(0.6931457519), ln2Part2 = float(1.4286067653e-6);
+  const float4 xy = P[0], zk = P[1], nw = P[2];
+  float2 c = mul2(f2(d.z), make_float2(zk.x, zk.y));
+  c = fma2(f2(d.y), make_float2(xy.z, xy.w), c);
+  c = fma2(f2(d.x), make_float2(xy.x, xy.y), c);
+  // fminf(NaN, 0) is 0, as the reference's MINPS
+  float2 v = mul2(make_float2(zk.z, zk.w), make_float2(fminf(c.x - 1.0f, 0.0f), fminf(c.y - 1.0f, 0.0f)));
+  asm("max.NaN.f32 %0, %0, 0fC2C80000;" : "+f"(v.x));  // -100
+  asm("max.NaN.f32 %0, %0, 0fC2C80000;" : "+f"(v.y));
+  const float2 sc = mul2(v, f2(1.44269502162933349609375f));
+  const float t0 = __fadd_rd(sc.x, 12582912.0f), t1 = __fadd_rd(sc.y, 12582912.0f);  // floor, see fexp
+  const float2 kr = make_float2(t0 - 12582912.0f, t1 - 12582912.0f);
+  const uint32_t e0 = uint32_t(max(int(f2u(t0)) - (0x4B400000 - 127), 0)) << 23;
+  const uint32_t e1 = uint32_t(max(int(f2u(t1)) - (0x4B400000 - 127), 0)) << 23;
+  float2 m = mul2(kr, f2(ln2Part1));
+  float2 x = make_float2(v.x - m.x, v.y - m.y);
+  m = mul2(kr, f2(ln2Part2));
+  x = make_float2(x.x - m.x, x.y - m.y);
+  float2 r = mul2(x, f2(2.7555381529964506626129150390625e-4f));
+  const float coeff[7] = {1.304379315115511417388916015625e-3f, 8.378830738365650177001953125e-3f,
+                          4.16539050638675689697265625e-2f, 0.166668415069580078125f,
+                          0.4999999105930328369140625f, 1.0f, 1.0f};
 #pragma unroll
-    for (int j = 0; j < kLanes; ++j) {
-      const int k = v * kLanes + j;
-      const float4 A = S.lobeA[k + v];
-      const float2 B = S.lobeB[k];
-      float ct = dot(d, mk(A.x, A.y, A.z));
-      float cm1 = emin(ct - 1.0f, 0.0f);
-      float ev = B.x * fexp(A.w * cm1);
-      T.t[j] = B.y * ev;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < kLanes; ++j) T.t[j] = 0.0f;
+  for (int i = 0; i < 7; ++i) {
+    r = make_float2(r.x + coeff[i], r.y + coeff[i]);
+    r = i < 6 ? mul2(x, r) : mul2(r, make_float2(u2f(e0), u2f(e1)));
   }
-  // lane sums over the lobe vectors in order: ((t0 + t1) + t2) + t3
-  float p[kLanes];
-#pragma unroll
-  for (int j = 0; j < kLanes; ++j) p[j] = T.t[j];
-  for (int step = 1; step < parts; ++step) {
-#pragma unroll
-    for (int j = 0; j < kLanes; ++j) {
-      const float in = __shfl_up_sync(full, p[j], 1);
-      if (v == step) p[j] = in + T.t[j];
-    }
-  }
-  float pdf = 0.0f, inv = 0.0f;
-  bool valid = false;
-  if (v == parts - 1 && have) {
-    pdf = reduce8(p);
-    valid = pdf > 1e-16f;
-    inv = valid ? rcp_avx2_tab(pdf, S.rcpTab) : 0.0f;
-  }
-  const int last = (int(threadIdx.x & 31) - v) + parts - 1;
-  T.pdf = __shfl_sync(full, pdf, last);
-  T.inv = __shfl_sync(full, inv, last);
-  T.valid = __shfl_sync(full, valid ? 1 : 0, last) != 0;
+  return mul2(make_float2(nw.z, nw.w), mul2(make_float2(nw.x, nw.y), r));
 }
 
-struct SampleIn {
-  float4 dw;
-  float x;  // pdf (split pass) or distance (distance pass)
-  bool have;
-};
-template <PassKind kind>
-__device__ __forceinline__ SampleIn load_sample(const LeafSamples &L, uint32_t idx) {
-  SampleIn r;
-  r.have = idx < L.count;
-  r.dw = make_float4(0.f, 0.f, 0.f, 0.f);
-  r.x = 0.0f;
-  if (r.have) {
-    r.dw = L.dirw[idx];
-    if constexpr (kind == kPassDistance) r.x = L.dist[idx];
-    else if constexpr (kind == kPassSplit) r.x = L.pdf[idx];
-  }
-  return r;
-}
-
-// a / b in a function of its own: the rare operands that div_rcp_try leaves
-// over.  As a plain expression behind a condition the division is evaluated
-// for every operand and the result selected afterwards; its slow path for
-// small numerators (most lobes are far from a sample's direction) was then
-// half of a split-statistics pass, and a branch per quotient keeps the eight
-// lobes of a lane from overlapping.  So a lane does its lobes without a
-// branch and then once more those that need it (first Update with 1,048,576
-// samples: split passes 182 -> 105 cycles per sample, distance passes 19 ->
-// 16, the Update 17.7 -> 11.7 ms).
+// a / b in a function of its own: as a plain expression behind a condition the
+// compiler evaluates the division for every operand and selects afterwards,
+// and most lobes are far from a sample's direction, so that most numerators
+// would run its slow path for small operands.
 __device__ __noinline__ float div_plain(float a, float b) { return a / b; }
 
-// Producer: lane v of sample slot s fills its lobes' rows of stage B.  In
-// split passes the running count of valid samples (for the chi-square means'
-// 1/n) needs a prefix over the chunk: warp ballots, then a barrier among the
-// producer threads only (named barrier 1), then `base` (valid samples of the
-// earlier chunks) moves on by the chunk's total.
-template <PassKind kind>
-__device__ __forceinline__ void produce(EmShared &S, const PassShape &sh, int cnt, int Kp, int s, int v,
-                                        const SampleIn &in, float *B, uint32_t &base) {
-  PartTerms T;
-  const V3 d = mk(in.dw.x, in.dw.y, in.dw.z);
-  const float w = in.dw.w;
-  part_terms(S, cnt, sh.parts, v, in.have, d, T);
-  const bool valid = in.have && T.valid;
-  const int R = sh.R;
-  const bool mine = v < cnt;  // this lane has lobes
-  if constexpr (kind == kPassDistance) {
-    // rows k: wts * rcp(distance); rows Kp + k: wts
-    if (mine) {
-      const float sd = valid ? rcp_avx2_tab(in.x, S.rcpTab) : 0.0f;
-      unsigned redo = 0;  // lobes whose quotient div_rcp_try could not give
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+
+// ---- distance passes (WEMFactory.h:1199-1326): per lobe the sums of wts and of
+// wts * rcp(distance), wts = (w a) (a pdf / weight).  A sample per producer
+// thread as in the E-step (below); a chunk holds rows wts_k (0 for skipped
+// samples) and rcp(distance) of RS = C + 4 floats; one consumer warp, lane k
+// summing both chains of lobe k.  22 cycles per sample at 23 lobes, issue bound in
+// the producers; 50 with a lane per lobe vector and two rows per lobe.
+template <int kCnt>
+__device__ __noinline__ void produce_distance(const EmShared &S, int RS, float4 dw, float dist, bool have, float *row) {
+  constexpr int Kp = kCnt * kLanes;
+  const V3 d = mk(dw.x, dw.y, dw.z);
+  const float w = dw.w;
+  float2 term[Kp / 2], p[kLanes / 2];
 #pragma unroll
-      for (int j = 0; j < kLanes; ++j) {
-        const int k = v * kLanes + j;
-        bool ok = true;
-        const float a = T.t[j] * T.inv;
-        float wts = (w * a) * div_rcp_try(a * T.pdf, S.lobeB[k].y, S.lobeWInv[k], ok);
-        if (!valid) wts = 0.0f;
-        redo |= ok ? 0u : 1u << j;
-        B[k * R + s] = wts * sd;
-        B[(Kp + k) * R + s] = wts;
-      }
-      if (valid && redo != 0) {
+  for (int v = 0; v < kCnt; ++v)
 #pragma unroll
-        for (int j = 0; j < kLanes; ++j) {
-          if ((redo >> j & 1u) == 0) continue;
-          const int k = v * kLanes + j;
-          const float a = T.t[j] * T.inv;
-          const float wts = (w * a) * div_plain(a * T.pdf, S.lobeB[k].y);
-          B[k * R + s] = wts * sd;
-          B[(Kp + k) * R + s] = wts;
-        }
-      }
+    for (int j = 0; j < kLanes / 2; ++j) {
+      const int i = v * (kLanes / 2) + j;
+      term[i] = pair_terms(S.lobeP + pair_at(2 * i), d);
+      p[j] = v == 0 ? term[i] : make_float2(p[j].x + term[i].x, p[j].y + term[i].y);
     }
-  } else {
-    // count of valid samples up to and including this one
-    const unsigned full = 0xFFFFFFFFu;
-    const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
-    const unsigned b = __ballot_sync(full, v == 0 && valid);
-    if (lane == 0) S.validPerWarp[warp] = uint32_t(__popc(b));
-    asm volatile("bar.sync 1, %0;" ::"r"(sh.threads) : "memory");
-    uint32_t before = 0, total = 0;
-    for (int q = 0; q < sh.threads / 32; ++q) {
-      const uint32_t n = S.validPerWarp[q];
-      before += q < warp ? n : 0u;
-      total += n;
-    }
-    const uint32_t count = base + before + uint32_t(__popc(b & ((1u << (lane - v)) - 1u))) + 1u;
-    base += total;
-    // rows r Kp + k: a, a w, (a w)(lx lx), (a w)(ly ly), (a w)(lx ly), chi,
-    // RN(1 / n) with n = n0_k + count; then the validity per sample
-    const float spdfv = in.x;
-    const float value = w * spdfv;
-    const float mcEst = S.mcEstimate;
-    // the three divisors are per sample: one reciprocal each, then Markstein
-    const float den1 = mcEst * T.pdf, den2 = ((mcEst * mcEst) * T.pdf) * T.pdf;
-    const float y1 = rcp_for_div(den1), y2 = rcp_for_div(den2), y3 = rcp_for_div(spdfv);
-    if (mine) {
-      const float vv = value * value;
-      unsigned redo = 0;  // lobes with a quotient that div_rcp_try could not give
+  const float pdf = ((p[0].x + p[0].y) + (p[1].x + p[1].y)) + ((p[2].x + p[2].y) + (p[3].x + p[3].y));  // reduce8
+  const bool valid = have && pdf > 1e-16f;
+  const float inv = valid ? rcp_avx2_tab(pdf, S.rcpTab) : 0.0f;
+  row[Kp * RS] = valid ? rcp_avx2_tab(dist, S.rcpTab) : 0.0f;
+  bool redo = false;
 #pragma unroll
-      for (int j = 0; j < kLanes; ++j) {
-        const int k = v * kLanes + j;
-        bool ok = true;
-        const float a = valid ? T.t[j] * T.inv : 0.0f;
-        const float vmf = a * T.pdf;
-        const float pvp = div_rcp_try(vmf * value, den1, y1, ok);
-        float chi = div_rcp_try(vv * vmf, den2, y2, ok);
-        chi -= 2.0f * pvp;
-        chi += vmf;
-        chi = div_rcp_try(chi, spdfv, y3, ok);
-        chi = a > 0.0f ? chi : 0.0f;
-        redo |= ok | !valid ? 0u : 1u << j;
-        const V3 ld = xfm(S.invFrame[k], d);
-        const float aw = a * w;
-        const float n = S.splitN0[k] + float(count);
-        B[k * R + s] = a;
-        B[(Kp + k) * R + s] = valid ? aw : 0.0f;
-        B[(2 * Kp + k) * R + s] = valid ? aw * (ld.x * ld.x) : 0.0f;
-        B[(3 * Kp + k) * R + s] = valid ? aw * (ld.y * ld.y) : 0.0f;
-        B[(4 * Kp + k) * R + s] = valid ? aw * (ld.x * ld.y) : 0.0f;
-        B[(5 * Kp + k) * R + s] = valid ? chi : 0.0f;
-        B[(6 * Kp + k) * R + s] = (valid & (n >= 1e-30f) & (n <= 1e30f)) ? rcp_rn(n) : 0.0f;
-      }
-      if (redo != 0) {
-#pragma unroll
-        for (int j = 0; j < kLanes; ++j) {
-          if ((redo >> j & 1u) == 0) continue;
-          const float a = T.t[j] * T.inv;
-          const float vmf = a * T.pdf;
-          const float pvp = div_plain(vmf * value, den1);
-          float chi = div_plain(vv * vmf, den2);
-          chi -= 2.0f * pvp;
-          chi += vmf;
-          chi = div_plain(chi, spdfv);
-          B[(5 * Kp + v * kLanes + j) * R + s] = a > 0.0f ? chi : 0.0f;
-        }
-      }
-    }
-    if (v == 0) B[7 * Kp * R + s] = valid ? 1.0f : 0.0f;
+  for (int i = 0; i < Kp / 2; ++i) {
+    const float2 wy0 = S.lobeW[2 * i], wy1 = S.lobeW[2 * i + 1];
+    const float2 a = mul2(term[i], f2(inv));
+    const float2 n = mul2(a, f2(pdf));
+    const bool s0 = n.x < kSmallNumerator, s1 = n.y < kSmallNumerator;
+    const float2 q = pair_quotients(n, make_float2(wy0.x, wy1.x), make_float2(wy0.y, wy1.y),
+                                    make_float2(s0 ? 0x1p50f : 1.0f, s1 ? 0x1p50f : 1.0f),
+                                    make_float2(s0 ? 0x1p-50f : 1.0f, s1 ? 0x1p-50f : 1.0f));
+    const float2 wts = mul2(mul2(f2(w), a), q);
+    row[2 * i * RS] = valid ? wts.x : 0.0f;
+    row[(2 * i + 1) * RS] = valid ? wts.y : 0.0f;
+    // a numerator out of range, a weight out of [1e-8, 1e8] (marked by a zero reciprocal)
+    redo |= !(n.x <= 1e15f) | !(n.y <= 1e15f) | (wy0.y == 0.0f) | (wy1.y == 0.0f);
   }
-}
-
-__device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
-__device__ __forceinline__ float4 ld4(const float *p) {  // two 64-bit loads (rows are 8-byte aligned)
-  const float2 a = ld2(p), b = ld2(p + 2);
-  return make_float4(a.x, a.y, b.x, b.y);
-}
-
-// Sum of one row (the terms of one accumulator) in sample order; loads run 8
-// samples ahead of the additions.
-__device__ __forceinline__ void row_chain(const float *row, int n4, float &acc) {
-  int s = 0;
-  if (n4 >= 8) {
-    float4 a = ld4(row), b = ld4(row + 4);
-    for (; s + 8 <= n4; s += 8) {
-      const int sn = s + 16 <= n4 ? s + 8 : s;
-      const float4 a1 = ld4(row + sn), b1 = ld4(row + sn + 4);
-      acc += a.x;
-      acc += a.y;
-      acc += a.z;
-      acc += a.w;
-      acc += b.x;
-      acc += b.y;
-      acc += b.z;
-      acc += b.w;
-      a = a1;
-      b = b1;
-    }
-  }
-  if (s < n4) {
-    const float4 v = ld4(row + s);
-    acc += v.x;
-    acc += v.y;
-    acc += v.z;
-    acc += v.w;
-  }
-}
-
-// Distance pass (WEMFactory.h:1199-1326): lanes c < Kp sum wts * rcp(distance),
-// lanes Kp <= c < 2 Kp sum wts.
-__device__ __forceinline__ void distance_chain(const float *B, const PassShape &sh, int c, int Kp, int n4,
-                                               float &acc) {
-  if (c < 2 * Kp) row_chain(B + c * sh.R, n4, acc);
-}
-
-// Split-statistics pass (Splitter.h:439-523).  Lanes c < 5 Kp sum row c
-// (r = c / Kp: sumAssignedSamples a, sumWeights a w, then the 2D covariance
-// sums (a w)(lx lx), (a w)(ly ly), (a w)(lx ly)).  Chi-square lanes start at
-// the next warp: the running mean chi2 += (chi - chi2) / n over the valid
-// samples, n counting from n0.  Markstein's steps with the producers'
-// y = RN(1 / (n0 + count)) give (chi - chi2) / n exactly (a skipped sample,
-// y = 0, adds +-0) when y belongs to the lane's own running count n (the
-// usual case: n equals n0 + count) and the difference d and the quotient lie
-// in [1e-30, 1e30] (or d is 0).  The chain checks this per group of four
-// samples beside the additions, not between them: the counts, the largest
-// |d| against 1e30 and the smallest non-zero |d| against 1e-30 times the
-// group's last n (so every quotient of the group is in range).  From the
-// first group that fails (rare) the chunk is summed again with divisions,
-// which give the same bits wherever Markstein's steps were exact.
-__device__ __forceinline__ int split_chi_base(int Kp) { return ((5 * Kp + 63) / 64) * 32; }
-__device__ __forceinline__ void split_chain(const float *B, const PassShape &sh, int c, int Kp, int n4, float n0,
-                                            float &acc, float &acc2, float &accN, float &cnt) {
-  const int R = sh.R;
-  const int chiBase = split_chi_base(Kp);
-  if (c < chiBase) {  // rows c and c + chiBase (a row chain costs a few cycles per sample, the chi chain ~50)
-    if (c < 5 * Kp) row_chain(B + c * R, n4, acc);
-    if (c + chiBase < 5 * Kp) row_chain(B + (c + chiBase) * R, n4, acc2);
-  } else if (c < chiBase + Kp) {
-    const int k = c - chiBase;
-    const float *xr = B + (5 * Kp + k) * R, *yr = B + (6 * Kp + k) * R, *vr = B + 7 * Kp * R;
-    const float accStart = acc, nStart = accN;
-    int redoAt = n4;  // first group that failed the range check
-    float accRedo = 0.0f, nRedo = 0.0f;
-    float4 x = ld4(xr), y = ld4(yr), v = ld4(vr);
-    for (int s = 0; s < n4; s += 4) {
-      const int sn = s + 4 < n4 ? s + 4 : s;
-      const float4 x1 = ld4(xr + sn), y1 = ld4(yr + sn), v1 = ld4(vr + sn);
-      const float accG = acc, nG = accN;
-      const float n1 = accN + v.x, n2 = n1 + v.y, n3 = n2 + v.z, n4v = n3 + v.w;
-      const float c1 = cnt + v.x, c2 = c1 + v.y, c3 = c2 + v.z, c4 = c3 + v.w;
-      const bool same = (v.x == 0.0f || n1 == n0 + c1) & (v.y == 0.0f || n2 == n0 + c2) &
-                        (v.z == 0.0f || n3 == n0 + c3) & (v.w == 0.0f || n4v == n0 + c4);
-      const float d1 = x.x - acc;
-      acc = acc + markstein_q(d1, n1, y.x);
-      const float d2 = x.y - acc;
-      acc = acc + markstein_q(d2, n2, y.y);
-      const float d3 = x.z - acc;
-      acc = acc + markstein_q(d3, n3, y.z);
-      const float d4 = x.w - acc;
-      acc = acc + markstein_q(d4, n4v, y.w);
-      const float a1 = fabsf(d1), a2 = fabsf(d2), a3 = fabsf(d3), a4 = fabsf(d4);
-      const float gMax = fmaxf(fmaxf(a1, a2), fmaxf(a3, a4));
-      const float gMin = fminf(fminf(a1 == 0.0f ? INFINITY : a1, a2 == 0.0f ? INFINITY : a2),
-                               fminf(a3 == 0.0f ? INFINITY : a3, a4 == 0.0f ? INFINITY : a4));
-      if ((!same || !(gMax <= 1e30f) || gMin < 1.0000002e-30f * n4v) && redoAt == n4) {
-        redoAt = s;
-        accRedo = accG;
-        nRedo = nG;
-      }
-      accN = n4v;
-      cnt = c4;
-      x = x1;
-      y = y1;
-      v = v1;
-    }
-    if (acc != acc) {
-      redoAt = 0;
-      accRedo = accStart;
-      nRedo = nStart;
-    }
-    if (redoAt < n4) {
-      acc = accRedo;
-      accN = nRedo;
-      for (int s = redoAt; s < n4; ++s) {
-        const float vv = vr[s];
-        accN += vv;
-        if (vv != 0.0f) acc += (xr[s] - acc) / accN;
-      }
+  if (redo && valid) {
+#pragma unroll 1
+    for (int k = 0; k < Kp; ++k) {
+      const float a = __fmul_rn((k & 1) ? pair_terms(S.lobeP + pair_at(k), d).y : pair_terms(S.lobeP + pair_at(k), d).x, inv);
+      row[k * RS] = (w * a) * div_plain(a * pdf, S.lobeW[k].x);
     }
   }
 }
 
-// Runs one distance or split-statistics pass over the leaf's samples in the
-// home block.  `acc`/`accN` are the consumer's accumulators (initialised by
-// the caller); chunk c is made into stage (c & 1) while the consumers add
-// chunk c - 1.
-template <PassKind kind>
-__device__ __noinline__ void run_pass(EmShared &S, const LeafSamples &L, const PassShape &sh, int cnt, float &accOut,
-                                      float &acc2Out, float &accNOut) {
+template <int kCnt>
+__device__ __noinline__ void run_distance(EmShared &S, const LeafSamples &L) {
+  constexpr int Kp = kCnt * kLanes;
+  constexpr int P = kEmThreads - 32;  // one consumer warp
+  constexpr int C = P, RS = C + 4;
+  static_assert((Kp + 1) * RS <= kStageFloats, "a distance chunk fits its stage");
   const int tid = threadIdx.x;
-  float acc = accOut, acc2 = acc2Out, accN = accNOut;  // the chains run on registers
-  const int Kp = cnt * kLanes;
-  const int C = sh.C;
   const uint32_t rounds = (L.count + C - 1) / C;
-  const bool producer = tid < sh.threads;
-  const int s = tid / sh.parts, v = tid % sh.parts;
-  const bool consumer = tid >= sh.P;
-  const int c = tid - sh.P;
-  const int chiK = kind == kPassSplit ? c - split_chi_base(Kp) : -1;
-  const float n0 = (chiK >= 0 && chiK < Kp) ? S.splitN0[chiK] : 0.0f;
-  float count = 0.0f;
-  uint32_t base = 0;
-  SampleIn next;
-  if (producer) next = load_sample<kind>(L, uint32_t(s));
-  long long cycP = 0, cycC = 0;
+  const bool producer = tid < P;
+  float4 dw = make_float4(0.f, 0.f, 0.f, 0.f);
+  float dist = 0.0f;
+  if (producer && uint32_t(tid) < L.count) {
+    dw = L.dirw[tid];
+    dist = L.dist[tid];
+  }
+  const int k = min(tid & 31, Kp - 1);
+  float sumD = 0.0f, sumW = 0.0f;
   for (uint32_t it = 0; it <= rounds; ++it) {
     if (producer && it < rounds) {
-      const long long t0 = clock64();
-      const SampleIn cur = next;
-      if (it + 1 < rounds) next = load_sample<kind>(L, (it + 1) * C + s);
-      produce<kind>(S, sh, cnt, Kp, s, v, cur, S.pbuf + (it & 1) * kStageFloats, base);
-      cycP += clock64() - t0;
+      const uint32_t idx = it * C + uint32_t(tid), nextIdx = idx + C;
+      const float4 cur = dw;
+      const float curDist = dist;
+      if (nextIdx < L.count) {
+        dw = L.dirw[nextIdx];
+        dist = L.dist[nextIdx];
+      }
+      produce_distance<kCnt>(S, RS, cur, curDist, idx < L.count, S.pbuf + (it & 1) * kStageFloats + tid);
     }
-    if (consumer && it >= 1) {
-      const long long t0 = clock64();
-      const uint32_t chunk = it - 1;
-      const int n = int(min(uint32_t(C), L.count - chunk * C));
+    if (!producer && it >= 1) {
+      const uint32_t base = smem_u32(S.pbuf + ((it - 1) & 1) * kStageFloats);
+      uint32_t A = base + uint32_t(k * RS) * 4u, D = base + uint32_t(Kp * RS) * 4u;
+      const int n = int(min(uint32_t(C), L.count - (it - 1) * C));
+      const int n8 = (n + 7) & ~7;
+      float4 a0 = lds4(A), d0 = lds4(D), a1 = lds4(A + 16), d1 = lds4(D + 16);
+#pragma unroll 1
+      for (int s = 0; s < n8; s += 8) {
+        A += 32;
+        D += 32;
+        const float2 p0 = mul2(make_float2(a0.x, a0.y), make_float2(d0.x, d0.y));
+        const float2 p1 = mul2(make_float2(a0.z, a0.w), make_float2(d0.z, d0.w));
+        const float2 p2 = mul2(make_float2(a1.x, a1.y), make_float2(d1.x, d1.y));
+        const float2 p3 = mul2(make_float2(a1.z, a1.w), make_float2(d1.z, d1.w));
+        const float4 v0 = a0, v1 = a1;
+        a0 = lds4(A);  // the last turn's loads run up to 8 floats past the row
+        d0 = lds4(D);
+        a1 = lds4(A + 16);
+        d1 = lds4(D + 16);
+        sumD += p0.x; sumW += v0.x;
+        sumD += p0.y; sumW += v0.y;
+        sumD += p1.x; sumW += v0.z;
+        sumD += p1.y; sumW += v0.w;
+        sumD += p2.x; sumW += v1.x;
+        sumD += p2.y; sumW += v1.y;
+        sumD += p3.x; sumW += v1.z;
+        sumD += p3.y; sumW += v1.w;
+      }
+    }
+    __syncthreads();
+  }
+  if (!producer && (tid & 31) < Kp) {
+    S.xch[0][k] = sumD;
+    S.xch[1][k] = sumW;
+  }
+  __syncthreads();
+}
+
+// ---- split-statistics passes (Splitter.h:439-523).  Producers: kCnt adjacent
+// lanes per sample, one lobe vector each (the vectors' pdf sums carried from
+// lane to lane in order); a chunk holds, per lobe, rows a, x and y of the
+// direction in the lobe's frame, and chi (all 0 for skipped samples), then
+// the rows of the sample's weight and validity.  Rows hold RS floats (a
+// multiple of four, RS / 4 odd) and the parts' blocks of rows start a few banks
+// apart, so that the parts of a sample store to distinct banks.  Consumers: warp 14, lane k
+// summing lobe k's a, a w and (a w)(x x), (a w)(y y), (a w)(x y); warp 15,
+// lane k its running chi-square mean.  The products are formed by the
+// consumers, four rows per lobe in place of seven, which makes chunks of 112 to
+// 448 samples of what were 80 to 200, and the counts' reciprocals by the chi-square
+// lanes.  Bound by the chi-square chain (47 cycles per sample beside the
+// producers' 36 at 24 lobes; 105 while the producers made seven rows a lobe and
+// counted the valid samples between two barriers).
+struct SplitShape {
+  int C, RS, vec, part;  // samples per chunk; floats per row, per lobe vector of rows, per part
+};
+template <int kCnt>
+__device__ constexpr SplitShape split_shape() {
+  constexpr int perWarp = 32 / kCnt;
+  constexpr int C = (kEmThreads / 32 - 2) * perWarp;
+  constexpr int RS = ((C + 4) / 8) * 8 + 4;  // > C, RS / 4 odd
+  return SplitShape{C, RS, kLanes * RS, 4 * kLanes * RS + (kCnt == 2 ? 16 : kCnt == 3 ? 12 : 8)};
+}
+
+template <int kCnt>
+__device__ __noinline__ void produce_split(const EmShared &S, int v, float4 dw, float spdf, bool have, float *B, int s) {
+  constexpr SplitShape sh = split_shape<kCnt>();
+  constexpr int RS = sh.RS;
+  const unsigned full = 0xFFFFFFFFu;
+  const V3 d = mk(dw.x, dw.y, dw.z);
+  const float w = dw.w;
+  const float4 *P = S.lobeP + v * (3 * kLanes / 2 + 1), *F = S.frameP + v * (3 * kLanes / 2 + 1);
+  float2 term[kLanes / 2], p[kLanes / 2];
+#pragma unroll
+  for (int j = 0; j < kLanes / 2; ++j) p[j] = term[j] = pair_terms(P + 3 * j, d);
+#pragma unroll
+  for (int step = 1; step < kCnt; ++step)
+#pragma unroll
+    for (int j = 0; j < kLanes / 2; ++j) {
+      const float x = __shfl_up_sync(full, p[j].x, 1), y = __shfl_up_sync(full, p[j].y, 1);
+      if (v == step) p[j] = make_float2(x + term[j].x, y + term[j].y);
+    }
+  float pdf = ((p[0].x + p[0].y) + (p[1].x + p[1].y)) + ((p[2].x + p[2].y) + (p[3].x + p[3].y));  // reduce8
+  if (kCnt > 1) pdf = __shfl_sync(full, pdf, (int(threadIdx.x) & 31) - v + kCnt - 1);  // the last part's
+  const bool valid = have && pdf > 1e-16f;
+  const float inv = valid ? rcp_avx2_tab(pdf, S.rcpTab) : 0.0f;
+  const float value = w * spdf, vv = value * value;
+  const float mc = S.mcEstimate;
+  const float den1 = mc * pdf, den2 = ((mc * mc) * pdf) * pdf;
+  // bounds within which nothing but a denormal quotient under- or overflows
+  const bool inside = (value == 0.0f || (fabsf(value) >= 1e-4f && fabsf(value) <= 1e4f)) && den1 >= 1e-10f &&
+                      den1 <= 1e4f && spdf >= 1e-6f && spdf <= 1e6f;
+  const float y1 = rcp_newton(den1), y2 = rcp_newton(den2), y3 = rcp_newton(spdf);
+  bool redo = !inside;
+  float *row = B + v * sh.part + s;
+#pragma unroll
+  for (int j = 0; j < kLanes / 2; ++j) {
+    const float2 a = mul2(term[j], f2(inv));
+    const float2 vmf = mul2(a, f2(pdf));
+    const bool s0 = vmf.x < kSmallNumerator, s1 = vmf.y < kSmallNumerator;
+    const float2 up = make_float2(s0 ? 0x1p50f : 1.0f, s1 ? 0x1p50f : 1.0f);
+    const float2 down = make_float2(s0 ? 0x1p-50f : 1.0f, s1 ? 0x1p-50f : 1.0f);
+    const float2 pvp = pair_quotients(mul2(vmf, f2(value)), f2(den1), f2(y1), up, down);
+    float2 chi = pair_quotients(mul2(f2(vv), vmf), f2(den2), f2(y2), up, down);
+    const float2 two = mul2(f2(2.0f), pvp);
+    chi = make_float2((chi.x - two.x) + vmf.x, (chi.y - two.y) + vmf.y);
+    chi = pair_quotients(chi, f2(spdf), f2(y3), up, down);
+    redo |= !(fabsf(chi.x) <= 1e20f) | !(fabsf(chi.y) <= 1e20f);
+    chi = make_float2(a.x > 0.0f ? chi.x : 0.0f, a.y > 0.0f ? chi.y : 0.0f);
+    const float4 f0 = F[3 * j], f1 = F[3 * j + 1], f2v = F[3 * j + 2];
+    const float2 lx = fma2(f2(d.x), make_float2(f0.x, f0.y),
+                                 fma2(f2(d.y), make_float2(f0.z, f0.w), mul2(f2(d.z), make_float2(f1.x, f1.y))));
+    const float2 ly =
+        fma2(f2(d.x), make_float2(f1.z, f1.w),
+                   fma2(f2(d.y), make_float2(f2v.x, f2v.y), mul2(f2(d.z), make_float2(f2v.z, f2v.w))));
+    float *r = row + 2 * j * RS;
+    r[0] = valid ? a.x : 0.0f;
+    r[RS] = valid ? a.y : 0.0f;
+    r += sh.vec;
+    r[0] = valid ? lx.x : 0.0f;
+    r[RS] = valid ? lx.y : 0.0f;
+    r += sh.vec;
+    r[0] = valid ? ly.x : 0.0f;
+    r[RS] = valid ? ly.y : 0.0f;
+    r += sh.vec;
+    r[0] = valid ? chi.x : 0.0f;
+    r[RS] = valid ? chi.y : 0.0f;
+  }
+  if (v == 0) {
+    float *r = B + kCnt * sh.part + s;
+    r[0] = valid ? w : 0.0f;
+    r[RS] = valid ? 1.0f : 0.0f;
+  }
+  if (redo && valid) {
+#pragma unroll 1
+    for (int j = 0; j < kLanes; ++j) {
+      const float2 t = pair_terms(P + 3 * (j / 2), d);
+      const float a = __fmul_rn((j & 1) ? t.y : t.x, inv);
+      const float vmf = a * pdf;
+      const float pvp = div_plain(vmf * value, den1);
+      float chi = div_plain(vv * vmf, den2);
+      chi -= 2.0f * pvp;
+      chi += vmf;
+      chi = div_plain(chi, spdf);
+      row[3 * sh.vec + j * RS] = a > 0.0f ? chi : 0.0f;
+    }
+  }
+}
+
+// Warp 14: five chains per lane over one chunk; A: the lobe's first row
+// (bytes), V: bytes from its a row to its x row and from x to y, W: the weights.
+struct SplitSums {
+  float sa, sw, cx, cy, cz;
+};
+__device__ __forceinline__ void split_sums(uint32_t A, uint32_t V, uint32_t W, int n4, SplitSums &q) {
+  uint32_t X = A + V, Y = X + V;
+  float4 a = lds4(A), x = lds4(X), y = lds4(Y), w = lds4(W);
+#pragma unroll 1
+  for (int s = 0; s < n4; s += 4) {
+    A += 16;
+    X += 16;
+    Y += 16;
+    W += 16;
+    const float4 a1 = lds4(A), x1 = lds4(X), y1 = lds4(Y), w1 = lds4(W);  // the last turn's run past the rows
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float2 ah = h ? make_float2(a.z, a.w) : make_float2(a.x, a.y);
+      const float2 xh = h ? make_float2(x.z, x.w) : make_float2(x.x, x.y);
+      const float2 yh = h ? make_float2(y.z, y.w) : make_float2(y.x, y.y);
+      const float2 wh = h ? make_float2(w.z, w.w) : make_float2(w.x, w.y);
+      const float2 aw = mul2(ah, wh);
+      const float2 xx = mul2(aw, mul2(xh, xh));
+      const float2 yy = mul2(aw, mul2(yh, yh));
+      const float2 xy = mul2(aw, mul2(xh, yh));
+      q.sa += ah.x;
+      q.sw += aw.x;
+      q.cx += xx.x;
+      q.cy += yy.x;
+      q.cz += xy.x;
+      q.sa += ah.y;
+      q.sw += aw.y;
+      q.cx += xx.y;
+      q.cy += yy.y;
+      q.cz += xy.y;
+    }
+    a = a1;
+    x = x1;
+    y = y1;
+    w = w1;
+  }
+}
+
+// Warp 15: the running mean chi2 += (chi - chi2) / n over the valid samples of a
+// chunk, n the lane's running count.  Markstein's steps with y = RN(1 / n)
+// (one Newton step, a group of four samples ahead of the additions) give
+// (chi - chi2) / n exactly (a skipped sample, y = 0, adds +-0) when the
+// difference d and the quotient lie in [1e-30, 1e30] (or d is 0).  The chain
+// is five dependent operations per sample, about 21 cycles; what runs beside
+// it is kept small (31 cycles per sample alone, 47 with the range checks per
+// group and a guarded n): a mean stays between its start and its samples, so
+// their sizes bound d, and the smallest non-zero |d| of the chunk is held against
+// 1e-30 times its last n, so every quotient is in range.  A chunk that fails
+// (rare) is summed again with divisions, which give the same bits wherever
+// Markstein's steps were exact.  kGuard: a count may be 0 before the first valid
+// sample.
+template <bool kGuard>
+__device__ __forceinline__ void chi_counts(float n0, float4 v, float4 &n, float4 &r) {
+  n.x = n0 + v.x;
+  n.y = n.x + v.y;
+  n.z = n.y + v.z;
+  n.w = n.z + v.w;
+  r.x = rcp_newton(kGuard ? fmaxf(n.x, 0.5f) : n.x) * v.x;  // n >= 1 where v is not 0
+  r.y = rcp_newton(kGuard ? fmaxf(n.y, 0.5f) : n.y) * v.y;
+  r.z = rcp_newton(kGuard ? fmaxf(n.z, 0.5f) : n.z) * v.z;
+  r.w = rcp_newton(kGuard ? fmaxf(n.w, 0.5f) : n.w) * v.w;
+}
+template <bool kGuard>
+__device__ __forceinline__ void split_chi(const float *xr, const float *vr, int n4, float &acc, float &accN) {
+  const float accStart = acc, nStart = accN;
+  uint32_t X = smem_u32(xr), V = smem_u32(vr);
+  float hi = fabsf(acc);       // largest |chi|, and the mean at the start
+  uint32_t lo = 0xFFFFFFFFu;  // smallest non-zero |d|, as twice its bits minus one (a zero's are the largest)
+  float4 x = lds4(X), v = lds4(V), n, r;
+  chi_counts<kGuard>(accN, v, n, r);
+  v = lds4(V + 16);
+#pragma unroll 2
+  for (int s = 0; s < n4; s += 4) {
+    X += 16;
+    V += 16;
+    const float4 x1 = lds4(X), v1 = lds4(V + 16);  // the last turns' loads run past the rows
+    float4 nn, rn;
+    chi_counts<kGuard>(n.w, v, nn, rn);
+    const float d1 = x.x - acc;
+    acc = acc + markstein_q(d1, n.x, r.x);
+    const float d2 = x.y - acc;
+    acc = acc + markstein_q(d2, n.y, r.y);
+    const float d3 = x.z - acc;
+    acc = acc + markstein_q(d3, n.z, r.z);
+    const float d4 = x.w - acc;
+    acc = acc + markstein_q(d4, n.w, r.w);
+    hi = fmaxf(fmaxf(hi, fmaxf(fabsf(x.x), fabsf(x.y))), fmaxf(fabsf(x.z), fabsf(x.w)));
+    lo = min(min(lo, min(2u * f2u(d1) - 1u, 2u * f2u(d2) - 1u)), min(2u * f2u(d3) - 1u, 2u * f2u(d4) - 1u));
+    accN = n.w;
+    x = x1;
+    v = v1;
+    n = nn;
+    r = rn;
+  }
+  if (acc != acc || !(hi <= 1e29f) || !(accN <= 1e30f) || lo < 2u * f2u(1.0000002e-30f * accN) - 1u) {
+    acc = accStart;
+    accN = nStart;
+#pragma unroll 1
+    for (int s = 0; s < n4; ++s) {
+      const float vv = vr[s];
+      accN += vv;
+      if (vv != 0.0f) acc += div_plain(xr[s] - acc, accN);
+    }
+  }
+}
+
+template <int kCnt>
+__device__ __noinline__ void run_split(EmShared &S, const LeafSamples &L, SplitState &sp) {
+  constexpr SplitShape sh = split_shape<kCnt>();
+  constexpr int Kp = kCnt * kLanes, C = sh.C, RS = sh.RS;
+  constexpr int P = kEmThreads - 64;
+  static_assert(kCnt * sh.part + 2 * RS <= kStageFloats, "a split chunk fits its stage");
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t rounds = (L.count + C - 1) / C;
+  const bool producer = tid < P;
+  // lane l of producer warp g: part l % kCnt of the warp's sample l / kCnt (three
+  // parts: lanes 30 and 31 follow along and store nothing)
+  constexpr int perWarp = 32 / kCnt;
+  const int v = lane % kCnt, slot = lane / kCnt;
+  const bool spare = slot >= perWarp;
+  const int s = (tid >> 5) * perWarp + slot;
+  float4 dw = make_float4(0.f, 0.f, 0.f, 0.f);
+  float spdf = 0.0f;
+  if (producer && !spare && uint32_t(s) < L.count) {
+    dw = L.dirw[s];
+    spdf = L.pdf[s];
+  }
+  const int k = min(lane, Kp - 1);
+  SplitSums q{};
+  float chi = 0.0f, chiN = 0.0f;
+  if (tid >= P && tid < P + 32) q = SplitSums{sp.sa[k], sp.sw[k], sp.cx[k], sp.cy[k], sp.cz[k]};
+  if (tid >= P + 32) {
+    chi = sp.chi2[k];
+    chiN = sp.n[k];
+  }
+  long long cycP = 0, cycC = 0;
+  for (uint32_t it = 0; it <= rounds; ++it) {
+    const long long t0 = clock64();
+    if (producer) {
+      if (it < rounds) {
+        const uint32_t idx = it * C + uint32_t(s), nextIdx = idx + C;
+        const float4 cur = dw;
+        const float curPdf = spdf;
+        if (!spare && nextIdx < L.count) {
+          dw = L.dirw[nextIdx];
+          spdf = L.pdf[nextIdx];
+        }
+        // a spare lane writes to the row's padding past the chunk's last sample
+        produce_split<kCnt>(S, v, cur, curPdf, !spare && idx < L.count, S.pbuf + (it & 1) * kStageFloats, spare ? RS - 1 : s);
+        cycP += clock64() - t0;
+      }
+    } else if (it >= 1) {
+      const float *B = S.pbuf + ((it - 1) & 1) * kStageFloats;
+      const int n = int(min(uint32_t(C), L.count - (it - 1) * C));
       const int n4 = (n + 3) & ~3;
-      const float *B = S.pbuf + (chunk & 1) * kStageFloats;
-      if constexpr (kind == kPassDistance) distance_chain(B, sh, c, Kp, n4, acc);
-      else split_chain(B, sh, c, Kp, n4, n0, acc, acc2, accN, count);
+      const float *row = B + (k / kLanes) * sh.part + (k % kLanes) * RS, *per = B + kCnt * sh.part;
+      if (tid < P + 32) split_sums(smem_u32(row), uint32_t(sh.vec) * 4u, smem_u32(per), n4, q);
+      else if (__all_sync(0xFFFFFFFFu, chiN + per[RS] >= 0.5f)) split_chi<false>(row + 3 * sh.vec, per + RS, n4, chi, chiN);
+      else split_chi<true>(row + 3 * sh.vec, per + RS, n4, chi, chiN);
       cycC += clock64() - t0;
     }
     __syncthreads();
   }
-  accOut = acc;
-  acc2Out = acc2;
-  accNOut = accN;
-  const int probe = kind == kPassSplit ? split_chi_base(Kp) : 0;
-  if (tid == 0 && kind == kPassSplit) S.prof.cycProdS += uint64_t(cycP);
-  if (c == probe && kind == kPassSplit) S.prof.cycConsS += uint64_t(cycC);
+  if (lane < Kp) {
+    if (tid >= P && tid < P + 32) {
+      sp.sa[k] = q.sa;
+      sp.sw[k] = q.sw;
+      sp.cx[k] = q.cx;
+      sp.cy[k] = q.cy;
+      sp.cz[k] = q.cz;
+    } else if (tid >= P + 32) {
+      sp.chi2[k] = chi;
+      sp.n[k] = chiN;
+    }
+  }
+  if (tid == 0) S.prof.cycProdS += uint64_t(cycP);
+  if (tid == P + 32) S.prof.cycConsS += uint64_t(cycC);
+  __syncthreads();
 }
 
 // ---------------------------------------------------------------- shared E-step passes
@@ -1152,7 +1185,6 @@ __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long l
 __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(unsigned long long *m, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(m)), "r"(count) : "memory");
 }
@@ -1274,42 +1306,6 @@ __device__ __forceinline__ EStepShape estep_shape(int cnt, const EmTuning &tune)
   return e;
 }
 
-// Two lobes' E-step terms w norm fexp(kappa min(cos - 1, 0)) of direction d.
-// The multiplications are packed (each component rounds as its own multiply),
-// the additions are not: the compiler contracts a packed multiply and a packed
-// addition into one rounding.  The exponential's argument is not positive (or NaN):
-// below -100 the result is 0 either way, so the argument is clamped there
-// (NaN kept) and the scale's exponent clamped at 0; the rest is fexp's.
-__device__ __forceinline__ float2 pair_terms(float4 xy, float4 zk, float4 nw, V3 d) {
-  const float ln2Part1 = float(0.6931457519), ln2Part2 = float(1.4286067653e-6);
-  float2 c = __fmul2_rn(make_float2(d.z, d.z), make_float2(zk.x, zk.y));
-  c = __ffma2_rn(make_float2(d.y, d.y), make_float2(xy.z, xy.w), c);
-  c = __ffma2_rn(make_float2(d.x, d.x), make_float2(xy.x, xy.y), c);
-  // fminf(NaN, 0) is 0, as the reference's MINPS
-  float2 v = __fmul2_rn(make_float2(zk.z, zk.w), make_float2(fminf(c.x - 1.0f, 0.0f), fminf(c.y - 1.0f, 0.0f)));
-  asm("max.NaN.f32 %0, %0, 0fC2C80000;" : "+f"(v.x));  // -100
-  asm("max.NaN.f32 %0, %0, 0fC2C80000;" : "+f"(v.y));
-  const float2 sc = __fmul2_rn(v, make_float2(1.44269502162933349609375f, 1.44269502162933349609375f));
-  const float t0 = __fadd_rd(sc.x, 12582912.0f), t1 = __fadd_rd(sc.y, 12582912.0f);  // floor, see fexp
-  const float2 kr = make_float2(t0 - 12582912.0f, t1 - 12582912.0f);
-  const uint32_t e0 = uint32_t(max(int(f2u(t0)) - (0x4B400000 - 127), 0)) << 23;
-  const uint32_t e1 = uint32_t(max(int(f2u(t1)) - (0x4B400000 - 127), 0)) << 23;
-  float2 m = __fmul2_rn(kr, make_float2(ln2Part1, ln2Part1));
-  float2 x = make_float2(v.x - m.x, v.y - m.y);
-  m = __fmul2_rn(kr, make_float2(ln2Part2, ln2Part2));
-  x = make_float2(x.x - m.x, x.y - m.y);
-  float2 r = __fmul2_rn(x, make_float2(2.7555381529964506626129150390625e-4f, 2.7555381529964506626129150390625e-4f));
-  const float coeff[7] = {1.304379315115511417388916015625e-3f, 8.378830738365650177001953125e-3f,
-                          4.16539050638675689697265625e-2f, 0.166668415069580078125f,
-                          0.4999999105930328369140625f, 1.0f, 1.0f};
-#pragma unroll
-  for (int i = 0; i < 7; ++i) {
-    r = make_float2(r.x + coeff[i], r.y + coeff[i]);
-    r = i < 6 ? __fmul2_rn(x, r) : __fmul2_rn(r, make_float2(u2f(e0), u2f(e1)));
-  }
-  return __fmul2_rn(make_float2(nw.z, nw.w), __fmul2_rn(make_float2(nw.x, nw.y), r));
-}
-
 // Producers: `nthreads` threads (index t) fill chunk `chunk` into G (a stage
 // or a ring slot), a sample per thread with the terms of all its lobes in
 // registers: the lobe vectors' sums stay in order without shuffles, the 32
@@ -1336,7 +1332,7 @@ __device__ __noinline__ void produce_estep_rows(const EmShared &S, const EStepSh
 #pragma unroll
       for (int j = 0; j < kLanes / 2; ++j) {
         const int i = v * (kLanes / 2) + j;
-        term[i] = pair_terms(S.lobeP[3 * i], S.lobeP[3 * i + 1], S.lobeP[3 * i + 2], d);
+        term[i] = pair_terms(S.lobeP + pair_at(2 * i), d);
         p[j] = v == 0 ? term[i] : make_float2(p[j].x + term[i].x, p[j].y + term[i].y);
       }
     const float pdf = ((p[0].x + p[0].y) + (p[1].x + p[1].y)) + ((p[2].x + p[2].y) + (p[3].x + p[3].y));  // reduce8
@@ -1345,7 +1341,7 @@ __device__ __noinline__ void produce_estep_rows(const EmShared &S, const EStepSh
     float *row = G + s;
 #pragma unroll
     for (int i = 0; i < Kp / 2; ++i) {
-      const float2 a = __fmul2_rn(term[i], make_float2(inv, inv));
+      const float2 a = mul2(term[i], make_float2(inv, inv));
       row[2 * i * RS] = valid ? a.x : 0.0f;
       row[(2 * i + 1) * RS] = valid ? a.y : 0.0f;
     }
@@ -1447,11 +1443,6 @@ __device__ void produce_for(EmShared &S, Board &b, float *ring, const EStepShape
 // (each component rounded as its own multiply).  The last turn's loads run up
 // to 16 floats past the row; their values are not used.  The loop is inlined
 // into the consumer's chunk loop and works on 32-bit shared-memory addresses.
-__device__ __forceinline__ float4 lds4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-  return v;
-}
 __device__ __forceinline__ void add4(float &acc, float4 v) {
   acc += v.x;
   acc += v.y;
@@ -1459,8 +1450,8 @@ __device__ __forceinline__ void add4(float &acc, float4 v) {
   acc += v.w;
 }
 __device__ __forceinline__ float4 chain_terms(float4 a, float4 d, float4 w) {
-  const float2 p0 = __fmul2_rn(__fmul2_rn(make_float2(d.x, d.y), make_float2(a.x, a.y)), make_float2(w.x, w.y));
-  const float2 p1 = __fmul2_rn(__fmul2_rn(make_float2(d.z, d.w), make_float2(a.z, a.w)), make_float2(w.z, w.w));
+  const float2 p0 = mul2(mul2(make_float2(d.x, d.y), make_float2(a.x, a.y)), make_float2(w.x, w.y));
+  const float2 p1 = mul2(mul2(make_float2(d.z, d.w), make_float2(a.z, a.w)), make_float2(w.z, w.w));
   return make_float4(p0.x, p0.y, p1.x, p1.y);
 }
 // Rows start at 32-bit shared addresses A0 (A1: the second lobe's), D, W
@@ -1783,7 +1774,7 @@ __device__ void pass_estep(EmShared &S, const LeafSamples &L) {
     const uint32_t gen = S.gen % kGrabGenMask + 1u;
     S.gen = gen;
     BoardParams &bp = b.params[gen & 1u];
-    for (int i = 0; i < 3 * Kp / 2; ++i) bp.lobeP[i] = S.lobeP[i];
+    for (int i = 0; i < pair_at(Kp); ++i) bp.lobeP[i] = S.lobeP[i];
     bp.dirw = L.dirw;
     bp.count = L.count;
     bp.seqBase = seqBase;
@@ -1927,7 +1918,7 @@ __device__ void help_others(EmShared &S, Board *boards, float *rings, const uint
         if (tid == 0) __threadfence();
         __syncthreads();
         const BoardParams &src = b.params[gen & 1u];
-        for (int i = tid; i < 3 * kMaxK / 2; i += kEmThreads) S.lobeP[i] = __ldcg(&src.lobeP[i]);
+        for (int i = tid; i < kPairEntries; i += kEmThreads) S.lobeP[i] = __ldcg(&src.lobeP[i]);
         if (tid == 0) {
           S.hp.dirw = reinterpret_cast<const float4 *>(__ldcg(reinterpret_cast<const unsigned long long *>(&src.dirw)));
           S.hp.count = __ldcg(&src.count);
@@ -1952,16 +1943,19 @@ __device__ void pass_distances(EmShared &S, const LeafSamples &L, bool init) {
   const int tid = threadIdx.x;
   const int cnt = vec_count(int(S.vmm.K));
   const int Kp = cnt * kLanes;
-  const PassShape sh = pass_shape<kPassDistance>(Kp);
-  pack_lobes(S, Kp);
+  pack_pairs(S, Kp);
+  if (tid < Kp) {
+    const float w = uint32_t(tid) < S.vmm.K ? S.vmm.w[tid] : 1.0f;  // the sums of lobes past the last are not used
+    S.lobeW[tid] = make_float2(w, (w >= 1e-8f && w <= 1e8f) ? rcp_newton(w) : 0.0f);
+  }
   __syncthreads();
-  float acc = 0.0f, accN = 0.0f;
-  float unused = 0.0f;
-  run_pass<kPassDistance>(S, L, sh, cnt, acc, unused, accN);
-  // exchange: bd in xch[0][k], bw in xch[1][k]
-  const int c = tid - sh.P;
-  if (c >= 0 && c < 2 * Kp) S.xch[c / Kp][c % Kp] = acc;
-  __syncthreads();
+  switch (cnt) {
+    case 1: run_distance<1>(S, L); break;
+    case 2: run_distance<2>(S, L); break;
+    case 3: run_distance<3>(S, L); break;
+    default: run_distance<4>(S, L); break;
+  }
+  // sums over rcp(distance) in xch[0], over 1 in xch[1]
   if (tid == 0) {
     VMMState &v = S.vmm;
     SuffState &s = S.suff;
@@ -1989,45 +1983,23 @@ __device__ void pass_split_stats(EmShared &S, const LeafSamples &L, SplitState &
   const int tid = threadIdx.x;
   const int cnt = vec_count(int(sp.K));
   const int Kp = cnt * kLanes;
-  const PassShape sh = pass_shape<kPassSplit>(Kp);
-  if (tid < Kp) {
-    S.invFrame[tid] = inverse_of(frame_of(mk(S.vmm.mx[tid], S.vmm.my[tid], S.vmm.mz[tid]), true));
-    S.splitN0[tid] = sp.n[tid];
+  if (2 * tid < Kp) {
+    const int k = 2 * tid;
+    const Frame f0 = inverse_of(frame_of(mk(S.vmm.mx[k], S.vmm.my[k], S.vmm.mz[k]), true));
+    const Frame f1 = inverse_of(frame_of(mk(S.vmm.mx[k + 1], S.vmm.my[k + 1], S.vmm.mz[k + 1]), true));
+    float4 *o = S.frameP + pair_at(k);
+    o[0] = make_float4(f0.vx.x, f1.vx.x, f0.vy.x, f1.vy.x);
+    o[1] = make_float4(f0.vz.x, f1.vz.x, f0.vx.y, f1.vx.y);
+    o[2] = make_float4(f0.vy.y, f1.vy.y, f0.vz.y, f1.vz.y);
   }
-  pack_lobes(S, Kp);
+  pack_pairs(S, Kp);
   __syncthreads();
-  const int c = tid - sh.P;
-  const int chiBase = split_chi_base(Kp);
-  // row q < 5 Kp: r = q / Kp selects sa, sw, cx, cy, cz of lobe k = q % Kp
-  auto row_value = [&](int q) {
-    const int r = q / Kp, k = q % Kp;
-    return r == 0 ? sp.sa[k] : r == 1 ? sp.sw[k] : r == 2 ? sp.cx[k] : r == 3 ? sp.cy[k] : sp.cz[k];
-  };
-  auto row_store = [&](int q, float v) {
-    const int r = q / Kp, k = q % Kp;
-    if (r == 0) sp.sa[k] = v;
-    else if (r == 1) sp.sw[k] = v;
-    else if (r == 2) sp.cx[k] = v;
-    else if (r == 3) sp.cy[k] = v;
-    else sp.cz[k] = v;
-  };
-  float acc = 0.0f, acc2 = 0.0f, accN = 0.0f;
-  if (c >= 0 && c < chiBase) {
-    if (c < 5 * Kp) acc = row_value(c);
-    if (c + chiBase < 5 * Kp) acc2 = row_value(c + chiBase);
-  } else if (c >= chiBase && c < chiBase + Kp) {
-    acc = sp.chi2[c - chiBase];
-    accN = sp.n[c - chiBase];
+  switch (cnt) {
+    case 1: run_split<1>(S, L, sp); break;
+    case 2: run_split<2>(S, L, sp); break;
+    case 3: run_split<3>(S, L, sp); break;
+    default: run_split<4>(S, L, sp); break;
   }
-  run_pass<kPassSplit>(S, L, sh, cnt, acc, acc2, accN);
-  if (c >= 0 && c < chiBase) {
-    if (c < 5 * Kp) row_store(c, acc);
-    if (c + chiBase < 5 * Kp) row_store(c + chiBase, acc2);
-  } else if (c >= chiBase && c < chiBase + Kp) {
-    sp.chi2[c - chiBase] = acc;
-    sp.n[c - chiBase] = accN;
-  }
-  __syncthreads();
 }
 
 // updateMixture / partialUpdateMixture (WEMFactory.h:751-844).  prev is the
