@@ -159,15 +159,36 @@ PGL_HD float fd_atan2f(float y, float x) {
   }
 }
 
+// phi / 2 pi + 1/2, the division and the sum in double and rounded once to
+// float, phi in [-pi, pi].  On the device in double-float arithmetic where its
+// rounding test decides (2 pi as the two floats of the double constant), the
+// double form as a function of its own for the rest: a double division holds a
+// scheduler for hundreds of cycles on this part.
+PGL_HD bool dqt_turn_df(float phi, float *out) {
+  const DFloat twoPi = {0x1.921fb6p+2f, -0x1.777a5cp-23f};
+  const DFloat q = df_quotient({phi, 0.0f}, twoPi, 0x1.45f306p-3f);
+  const DFloat s = df_two_sum(0.5f, q.h);
+  return df_round_checked(df_fast_two_sum(s.h, s.l + q.l), out);
+}
+#ifdef __CUDACC__
+static __device__ __noinline__ float dqt_turn_fp64(float phi) { return float(double(phi) / (2.0 * kPiD) + 0.5); }
+#endif
+PGL_HD float dqt_turn(float phi) {
+#ifdef __CUDA_ARCH__
+  float r;
+  return fabsf(phi) >= 1e-20f && dqt_turn_df(phi, &r) ? r : dqt_turn_fp64(phi);
+#else
+  return float(double(phi) / (2.0 * kPiD) + 0.5);
+#endif
+}
 // SphereToSquareCylindrical (SphereToSquare.h:34-61): x = (cos theta + 1) / 2,
 // y = phi / 2pi + 1/2, phi = atan2(d.y, d.x), the division in double.
 PGL_HD void dqt_dir_to_point(float dx, float dy, float dz, float &px, float &py) {
   dx = dqt_clamp(dx, -1.f, 1.f);
   dy = dqt_clamp(dy, -1.f, 1.f);
   dz = dqt_clamp(dz, -1.f, 1.f);
-  const float phi = fd_atan2f(dy, dx);
   px = dqt_clamp((dz + 1.0f) / 2.0f, 0.f, 1.f);
-  py = dqt_clamp(float(double(phi) / (2.0 * kPiD) + 0.5), 0.f, 1.f);
+  py = dqt_clamp(dqt_turn(fd_atan2f(dy, dx)), 0.f, 1.f);
 }
 // SphereToSquareCylindrical::area (SphereToSquare.h:57-59)
 PGL_HD float dqt_area(const Box2 &r) { return 4.0f * 3.14159274101257324f * (r.x1 - r.x0) * (r.y1 - r.y0); }

@@ -897,7 +897,7 @@ void SubField::dqtReserve(uint32_t R) {
   dDqtNodes.reserve(size_t(R) * stride, true);
 }
 DqtSide SubField::dqtSide() {
-  return DqtSide{dDqtHeads.p, dDqtStats.p, dDqtNodes.p, dqtStride, sD_.p, sPdf_.p, cfg.dqtArgs, cfg.decayOnSpatialSplit};
+  return DqtSide{dDqtHeads.p, dDqtStats.p, dDqtNodes.p, dqtStride, sD_.p, sPdf_.p, sP_.p, cfg.dqtArgs, cfg.decayOnSpatialSplit};
 }
 
 std::vector<RegionDir> SubField::downloadRegions() const {
@@ -1034,9 +1034,9 @@ void GpuField::runDqt(SubField *const *sides, int count) {
   if (T > 0) {
     tasks_.reserve(T);
     queue_.reserve(2);
-    dqtRects_.reserve(size_t(blocks) * stride);
+    dqtRects_.reserve(2 * size_t(blocks) * stride + 32);
     dqtBuild_.reserve(size_t(blocks) * stride);
-    dqtLeaves_.reserve(size_t(blocks) * stride);
+    dqtLeaves_.reserve(4 * size_t(blocks) * stride);
     check(cudaMemcpyAsync(tasks_.p, all.data(), T * sizeof(LeafTask), cudaMemcpyHostToDevice, s), "tasks");
     check(cudaMemsetAsync(queue_.p, 0, 2 * sizeof(unsigned int), s), "queue");
   }

@@ -46,6 +46,7 @@ struct DqtSide {
   uint32_t stride;
   const float4 *dirw;
   const float *pdf;
+  float4 *points;  // per sorted sample: its point on the square and moments (scratch)
   DqtArgs args;
   float decay;  // on a spatial split
 };
@@ -53,7 +54,8 @@ struct DqtSides {
   DqtSide side[2];
 };
 // Fit or update of every task's region (persistent blocks on a queue; per
-// block `scratchStride` rectangles, build nodes and leaf indices of scratch);
+// block twice `scratchStride` rectangles (and 32 at the end), as many build nodes
+// and four times as many words of scratch);
 // *err becomes non-zero when a tree outgrows its node slots.
 cudaError_t launch_dqt_update(const LeafTask *tasks, uint32_t numTasks, unsigned int *queue, const DqtSides &sides,
                               Box2 *rects, DqtStatsNode *builds, uint32_t *leaves, uint32_t scratchStride, int blocks,
