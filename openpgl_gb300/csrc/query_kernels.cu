@@ -106,10 +106,8 @@ __device__ __forceinline__ Lobe load_shifted(const VMMState &v, int lane, float 
   V3 mu = mk(v.mx[lane], v.my[lane], v.mz[lane]);
   V3 s = mk(v.pivot[0] - p0, v.pivot[1] - p1, v.pivot[2] - p2);
   V3 p = mu * dist + s;
-  float len = length(p);
-  p = p / len;
   bool cond = (dist > 0.0f) && (dist >= -FLT_MAX) && (dist <= FLT_MAX);
-  if (cond && parallax) mu = p;
+  if (cond && parallax) mu = div3(p, length(p));
   L.mx = mu.x; L.my = mu.y; L.mz = mu.z;
   return L;
 }
@@ -127,7 +125,7 @@ __device__ __forceinline__ Lobe product_terms(const Lobe &L, V3 n, float kappa, 
   float nk = sqrtf(dot(nm, nm));
   bool chk = nk > 1e-3f;
   nk = chk ? nk : 0.0f;
-  nm = chk ? nm / nk : mu;
+  nm = chk ? div3(nm, nk) : mu;
   float ne = fexp(-2.0f * nk);
   float nn = nk / (kTwoPiF * (1.0f - ne));
   nn = chk ? nn : kInv4Pi;
@@ -201,13 +199,13 @@ __device__ V3 lobe_direction(float k, float e2k, V3 mu, float ux, float u1) {
     float z = 1.0f - 2.0f * u1;
     float r = sqrtf(smax(0.f, (1.0f - z * z)));
     float sp, cp;
-    lib_sincosf(float(2.0 * kPiD * double(ux)), &sp, &cp);
+    lib_sincosf(two_pi_times(ux), &sp, &cp);
     d = mk(r * cp, r * sp, z);
   } else {
     float ct = 1.f + (flog(1.0f + ((e2k - 1.f) * ux))) / k;
     ct = smin(1.0f, smax(ct, -1.f));
     float st = sqrtf(1.f - ct * ct);
-    float phi = float(2.0 * kPiD * double(u1));
+    float phi = two_pi_times(u1);
     float sp, cp;
     lib_sincosf(phi, &sp, &cp);
     d = mk(st * cp, st * sp, ct);
@@ -332,101 +330,152 @@ __device__ void dqt_query_out(const FieldView &f, uint32_t reg, uint32_t leaf, f
   o.pdfLi = dqt_pdf(N, d);
 }
 
-// ---------------------------------------------------------------- four queries per warp
-// A group of eight lanes per query: lane j of a group holds lobes j, j + 8,
-// j + 16 and j + 24 (the vfloat8 lane j of each lobe vector), so the sums over
-// the mixture keep the warp-per-query order (per lane over the vectors, then
-// the 8-lane tree) and mixtures of up to eight lobes keep every lane busy.
-// Shuffles stay inside the group (width 8, the group's lane mask): groups of
-// one warp may take different paths.
-struct LobeSet {
-  Lobe l[4];
+// ---------------------------------------------------------------- several queries per warp
+// A group of 8 * kH lanes per query.  With kH = 1 (four queries per warp) lane j
+// holds lobes j, j + 8, j + 16 and j + 24, with kH = 2 (two per warp) lobes j
+// and j + 16: lane j of every lobe vector (vfloat8) sits in a lane whose low
+// three bits are j.  So the sums over the mixture keep the warp-per-query order
+// (per vector lane over the vectors, then the 8-lane tree).
+// Shuffles stay inside the group (its width, its lane mask): groups of one warp
+// may take different paths.
+template <int kH>
+constexpr int kSlots = 4 / kH;  // lobes per lane
+template <int kH>
+struct Group {
+  int j;        // lane of the group
+  unsigned gm;  // its lane mask
+  __device__ __forceinline__ explicit Group(int lane)
+      : j(lane & (8 * kH - 1)), gm((kH == 1 ? 0xFFu : 0xFFFFu) << (lane & (32 - 8 * kH))) {}
+  template <typename T>
+  __device__ __forceinline__ T from(T v, int src) const {
+    return __shfl_sync(gm, v, src, 8 * kH);
+  }
+  // the 8-lane tree: all eight lanes end with the same bits (each step adds the
+  // same two numbers on both sides)
+  __device__ __forceinline__ float tree(float v) const {
+    v += __shfl_xor_sync(gm, v, 1, 8);
+    v += __shfl_xor_sync(gm, v, 2, 8);
+    v += __shfl_xor_sync(gm, v, 4, 8);
+    return v;
+  }
+  // the sum over the mixture; lobes past its last vector count +0, which changes
+  // no bit of a sum that started at +0
+  __device__ __forceinline__ float sum(const float v[kSlots<kH>]) const {
+    float acc = 0.0f;
+    if constexpr (kH == 1) {
+#pragma unroll
+      for (int q = 0; q < kSlots<kH>; ++q) acc += v[q];
+    } else {
+      // vectors 0 and 1 sit in the two halves and add in either order, vectors 2 and 3 in theirs
+      acc = (acc + v[0]) + __shfl_xor_sync(gm, v[0], 8, 16);
+      const float o = __shfl_xor_sync(gm, v[1], 8, 16);
+      acc = j < 8 ? (acc + v[1]) + o : (acc + o) + v[1];
+    }
+    return tree(acc);
+  }
 };
-__device__ __forceinline__ float group_sum(const float v[4], int cnt, unsigned gm) {
-  float acc = 0.0f;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    if (q < cnt) acc += v[q];
-  acc += __shfl_xor_sync(gm, acc, 1, 8);
-  acc += __shfl_xor_sync(gm, acc, 2, 8);
-  acc += __shfl_xor_sync(gm, acc, 4, 8);
-  return __shfl_sync(gm, acc, 0, 8);
+template <int kH>
+struct LobeSet {
+  Lobe l[kSlots<kH>];
+};
+// is slot q of this lane in one of the mixture's cnt lobe vectors?
+template <int kH>
+__device__ __forceinline__ bool holds(const Group<kH> &G, int q, int cnt) {
+  return q * kH + (kH == 1 ? 0 : G.j >> 3) < cnt;
 }
-__device__ __forceinline__ Lobe pick(const LobeSet &L, uint32_t q) {  // q uniform in the group
-  Lobe r = L.l[0];
-  if (q == 1) r = L.l[1];
-  if (q == 2) r = L.l[2];
-  if (q == 3) r = L.l[3];
-  return r;
-}
-// the lobe vectors q < cnt of the mixture (the others are never read)
-__device__ __forceinline__ LobeSet load_shifted_g(const VMMState &v, int j, float p0, float p1, float p2,
-                                                  bool parallax, int cnt) {
-  LobeSet L;
+// the lobe vectors of the mixture (the other slots hold zeros)
+template <int kH>
+__device__ __forceinline__ LobeSet<kH> load_shifted_g(const Group<kH> &G, const VMMState &v, float p0, float p1, float p2,
+                                                      bool parallax, int cnt) {
+  LobeSet<kH> L;
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-    if (q < cnt) L.l[q] = load_shifted(v, q * kLanes + j, p0, p1, p2, parallax);
+  for (int q = 0; q < kSlots<kH>; ++q) {
+    L.l[q] = Lobe{};
+    if (holds(G, q, cnt)) L.l[q] = load_shifted(v, q * 8 * kH + G.j, p0, p1, p2, parallax);
+  }
   return L;
 }
-__device__ __forceinline__ LobeSet product_lobe_g(const LobeSet &L, V3 n, float kappa, float normalization,
-                                                  float weight, int cnt, unsigned gm) {
-  LobeSet R;
-  float w[4];
+template <int kH>
+__device__ __forceinline__ LobeSet<kH> product_lobe_g(const Group<kH> &G, const LobeSet<kH> &L, V3 n, float kappa,
+                                                      float normalization, float weight, int cnt, float &integral) {
+  LobeSet<kH> R;
+  float w[kSlots<kH>];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    if (q < cnt) R.l[q] = product_terms(L.l[q], n, kappa, normalization, weight);
-    w[q] = q < cnt ? R.l[q].w : 0.0f;
+  for (int q = 0; q < kSlots<kH>; ++q) {
+    R.l[q] = Lobe{};
+    if (holds(G, q, cnt)) R.l[q] = product_terms(L.l[q], n, kappa, normalization, weight);
+    w[q] = R.l[q].w;
   }
-  const float integral = group_sum(w, cnt, gm);
+  integral = G.sum(w);
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-    if (q < cnt) R.l[q].w /= integral;
+  for (int q = 0; q < kSlots<kH>; ++q)
+    if (holds(G, q, cnt)) R.l[q].w /= integral;
   return R;
 }
-__device__ __forceinline__ float mixture_pdf_g(const LobeSet &L, V3 d, int cnt, unsigned gm) {
-  float t[4];
+template <int kH>
+__device__ __forceinline__ float mixture_pdf_g(const Group<kH> &G, const LobeSet<kH> &L, V3 d, int cnt) {
+  float t[kSlots<kH>];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) t[q] = q < cnt ? mixture_term(L.l[q], d) : 0.0f;
-  return group_sum(t, cnt, gm);
+  for (int q = 0; q < kSlots<kH>; ++q) t[q] = holds(G, q, cnt) ? mixture_term(L.l[q], d) : 0.0f;
+  return G.sum(t);
 }
-// PAVMM::sample (PAVMM.h:737-806) by a group
-__device__ V3 mixture_sample_g(const LobeSet &L, int K, float ux, float uy, unsigned gm) {
-  // per-vector sums of the weights (vectors past the mixture's last are never searched)
+// PAVMM::sample (PAVMM.h:737-806) by a group: the lobe that uy picks and uy
+// rescaled into it; the direction in the lobe is lobe_direction's.  Both
+// searches run without branches, so the groups of a warp stay together.
+struct PickedLobe {
+  float kappa, e2k, u1;
+  V3 mu;
+};
+template <int kH>
+__device__ __forceinline__ PickedLobe mixture_pick_g(const Group<kH> &G, const LobeSet<kH> &L, int K, float uy) {
   const int cnt = vec_count(K);
-  float vecSum[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    float g = q < cnt ? L.l[q].w : 0.0f;
-    if (q < cnt) {
-      g += __shfl_xor_sync(gm, g, 1, 8);
-      g += __shfl_xor_sync(gm, g, 2, 8);
-      g += __shfl_xor_sync(gm, g, 4, 8);
-      g = __shfl_sync(gm, g, 0, 8);
-    }
-    vecSum[q] = g;
-  }
+  const uint32_t quot = uint32_t((K - 1) / kLanes), rem = uint32_t((K - 1) % kLanes);
+  // per-vector sums of the weights (vectors past the mixture's last are never searched)
   uint32_t sv = 0, sc = 0;
-  float searched = uy, sumW = 0.0f, cdf = 0.0f;
-  uint32_t quot = uint32_t((K - 1) / kLanes), rem = uint32_t((K - 1) % kLanes);
-  for (;;) {
-    cdf = sv == 0 ? vecSum[0] : sv == 1 ? vecSum[1] : sv == 2 ? vecSum[2] : vecSum[3];
-    if (sumW + cdf >= searched || sv + 1 >= quot + 1) break;
-    sumW += cdf;
-    sv++;
+  float sumW = 0.0f, cdf = 0.0f;
+  bool done = false;
+#pragma unroll
+  for (int q = 0; q < kSlots<kH>; ++q) {
+    if (q * kH >= cnt) continue;
+    const float t = G.tree(L.l[q].w);
+#pragma unroll
+    for (int h = 0; h < kH; ++h) {
+      const float g = kH == 1 ? t : G.from(t, 8 * h);
+      const uint32_t vec = uint32_t(q * kH + h);
+      const bool stop = sumW + g >= uy || vec >= quot;
+      sv = done ? sv : vec;
+      sumW = done || stop ? sumW : sumW + g;
+      done = done || stop;
+    }
   }
-  const Lobe V = pick(L, sv);
-  uint32_t maxSel = (sv == quot) ? rem + 1 : kLanes;
-  for (;;) {
-    cdf = __shfl_sync(gm, V.w, int(sc), 8);
-    if (sumW + cdf >= searched || sc + 1 >= maxSel) break;
-    sumW += cdf;
-    sc++;
+  // the picked vector: the slot that its lanes hold it in, and the first of those lanes
+  const uint32_t slot = sv / kH;
+  const int first = kH == 1 ? 0 : int(sv % kH) * 8;
+  const auto held = [&](auto field) {
+    float r = L.l[0].*field;
+#pragma unroll
+    for (int q = 1; q < kSlots<kH>; ++q) r = slot == uint32_t(q) ? L.l[q].*field : r;
+    return r;
+  };
+  const float vw = held(&Lobe::w);
+  const uint32_t maxSel = (sv == quot) ? rem + 1 : kLanes;
+  done = false;
+#pragma unroll
+  for (int c = 0; c < kLanes; ++c) {
+    const float w = G.from(vw, first + c);
+    const bool stop = sumW + w >= uy || uint32_t(c) + 1 >= maxSel;
+    sc = done ? sc : uint32_t(c);
+    cdf = done ? cdf : w;
+    sumW = done || stop ? sumW : sumW + w;
+    done = done || stop;
   }
-  float u1 = smin(1.0f - FLT_EPSILON, (searched - sumW) / cdf);
-  const int s = int(sc);
-  float k = __shfl_sync(gm, V.kappa, s, 8), e2k = __shfl_sync(gm, V.e2k, s, 8);
-  V3 mu = mk(__shfl_sync(gm, V.mx, s, 8), __shfl_sync(gm, V.my, s, 8), __shfl_sync(gm, V.mz, s, 8));
-  return lobe_direction(k, e2k, mu, ux, u1);
+  const int src = first + int(sc);
+  PickedLobe r;
+  r.u1 = smin(1.0f - FLT_EPSILON, (uy - sumW) / cdf);
+  r.kappa = G.from(held(&Lobe::kappa), src);
+  r.e2k = G.from(held(&Lobe::e2k), src);
+  r.mu = mk(G.from(held(&Lobe::mx), src), G.from(held(&Lobe::my), src), G.from(held(&Lobe::mz), src));
+  return r;
 }
 // choose_region by a group: lane j ranks neighbour j
 __device__ uint32_t choose_region_g(const FieldView &f, uint32_t leaf, float p0, float p1, float p2, float &s1d,
@@ -451,127 +500,185 @@ __device__ uint32_t choose_region_g(const FieldView &f, uint32_t leaf, float p0,
   return nb.ids[chosenKey & 7u];
 }
 
-// Batched volume guided queries with the Henyey-Greenstein product, a warp
-// per query: Init + product with the phase function's fit + SamplePDF (+
-// pdfLi).  The three products of a mixture need three times the registers
-// of the cosine product, so a lane keeps one lobe here.
-__global__ void query_hg_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= n) return;
-  const QueryIn q = in[gw];
-  const FieldView &f = P.f;
-  QueryOut o;
-  o.ok = 0; o.id = 0; o.s1d = q.s1d; o.dx = o.dy = o.dz = 0.0f; o.pdf = 0.0f; o.pdfLi = 0.0f;
-  bool inside = f.iteration > 0 && q.px >= f.bounds[0] && q.px <= f.bounds[3] && q.py >= f.bounds[1] &&
-                q.py <= f.bounds[4] && q.pz >= f.bounds[2] && q.pz <= f.bounds[5];
+// Init of a group's query: false when it is outside the field or its region is
+// not valid; else its kd leaf, region and rescaled s1d.
+struct GroupInit {
+  uint32_t leaf, reg;
+  float s1d;
+  bool ok;
+};
+template <typename Q>
+__device__ __forceinline__ GroupInit init_g(const FieldView &f, const Q &q, int lane) {
+  GroupInit r{0, 0, q.s1d, false};
+  const bool inside = f.iteration > 0 && q.px >= f.bounds[0] && q.px <= f.bounds[3] && q.py >= f.bounds[1] &&
+                      q.py <= f.bounds[4] && q.pz >= f.bounds[2] && q.pz <= f.bounds[5];
   if (inside) {
-    uint32_t leaf = kd_leaf(f, q.px, q.py, q.pz);
-    uint32_t reg = leaf;
-    float s1d = q.s1d;
-    if (f.knn && s1d >= 0.f) reg = choose_region(f, leaf, q.px, q.py, q.pz, s1d, lane);
-    o.s1d = s1d;
-    const RegionDir &R = f.regions[reg];
-    if (R.valid) {
-      const int K = int(R.vmm.K), cnt = vec_count(K);
-      Lobe li = load_shifted(R.vmm, lane, q.px, q.py, q.pz, f.parallax != 0);
-      Lobe h[kHgLobes];
-      float w[kHgLobes];
-      hg_products(li, mk(q.nx, q.ny, q.nz), P.hgMeanCosine[gw], cnt, lane, h, w);
-      const V3 d = products_sample(h, w, kHgLobes, K, q.ux, q.uy, lane, o.pdf);
-      o.ok = 1;
-      o.id = leaf;
-      o.dx = d.x; o.dy = d.y; o.dz = d.z;
-      o.pdfLi = mixture_pdf(li, d, cnt, lane);
-    }
+    r.leaf = r.reg = kd_leaf(f, q.px, q.py, q.pz);
+    if (f.knn && r.s1d >= 0.f) r.reg = choose_region_g(f, r.leaf, q.px, q.py, q.pz, r.s1d, lane & 7, lane, 0xFFu << (lane & 24));
+    r.ok = f.regions[r.reg].valid != 0;
   }
-  if (lane == 0) out[gw] = o;
+  return r;
+}
+
+// Batched volume guided queries with the Henyey-Greenstein product, two per
+// warp: Init + product with the phase function's fit + SamplePDF (+ pdfLi).
+// The mixture and its three products are live together, so a lane holds two
+// lobes of each; 72 registers for seven blocks per SM.  262,144 queries:
+// 507 us with a warp per query, 411 us so (450 at 93 registers, 646 four per
+// warp with the large mixtures redone by the whole warp).
+__global__ void __launch_bounds__(128, 7) query_hg_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+  const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  const int lane = threadIdx.x & 31;
+  if (gid >= n) return;
+  const Group<2> G(lane);
+  const FieldView &f = P.f;
+  const QueryIn q = in[gid];
+  const GroupInit init = init_g(f, q, lane);
+  QueryOut o;
+  o.ok = init.ok ? 1u : 0u;
+  o.id = init.ok ? init.leaf : 0u;
+  o.s1d = init.s1d;
+  o.dx = o.dy = o.dz = 0.0f;
+  o.pdf = o.pdfLi = 0.0f;
+  if (init.ok) {
+    const VMMState &v = f.regions[init.reg].vmm;
+    const int K = int(v.K), cnt = vec_count(K);
+    const LobeSet<2> li = load_shifted_g<2>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
+    const float meanCosine = P.hgMeanCosine[gid];
+    const float step = (kHgMaxMeanCosine - kHgMinMeanCosine) / float(kHgFits);
+    int idx = int(floorf((fabsf(meanCosine) - kHgMinMeanCosine) / step));
+    idx = idx < kHgFits - 1 ? idx : kHgFits - 1;
+    const V3 dir = mk(q.nx, q.ny, q.nz);
+    LobeSet<2> h[kHgLobes];
+    float w[kHgLobes], sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kHgLobes; ++i) {  // hg_products
+      const HgLobeFit fit = c_hg[idx][i];
+      const V3 to = meanCosine * fit.meanCosine > 0.f ? dir : mk(-dir.x, -dir.y, -dir.z);
+      h[i] = product_lobe_g<2>(G, li, to, fit.kappa, fit.normalization, fit.weight, cnt, w[i]);
+      sum += w[i];
+    }
+#pragma unroll
+    for (int i = 0; i < kHgLobes; ++i) w[i] /= sum;
+    // products_sample
+    float acc = 0.0f;
+    int i = 0;
+    for (; i < kHgLobes - 1; ++i) {
+      const float next = acc + w[i];
+      if (next > q.ux) break;
+      acc = next;
+    }
+    const LobeSet<2> g = i == 0 ? h[0] : (i == 1 ? h[1] : h[2]);
+    const float wi = i == 0 ? w[0] : (i == 1 ? w[1] : w[2]);
+    const PickedLobe p = mixture_pick_g<2>(G, g, K, q.uy);
+    const V3 d = lobe_direction(p.kappa, p.e2k, p.mu, (q.ux - acc) / wi, p.u1);
+#pragma unroll
+    for (int k = 0; k < kHgLobes; ++k) o.pdf += w[k] * mixture_pdf_g<2>(G, h[k], d, cnt);
+    o.dx = d.x;
+    o.dy = d.y;
+    o.dz = d.z;
+    o.pdfLi = mixture_pdf_g<2>(G, li, d, cnt);
+  }
+  if (G.j == 0) out[gid] = o;
 }
 
 // Batched guided queries, four per warp: Init + optional cosine product
-// (surface) + SamplePDF (+ pdfLi).
-__global__ void query_g_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+// (surface) + SamplePDF (+ pdfLi).  Issue bound at about three quarters of the
+// issue rate; 64 registers for four blocks per SM.  1,048,576 queries: 818 us
+// with searches by branches, FP64 in lobe_direction, divisions one by one and
+// the rsqrt table in constant memory (its lookups went one by one), 706 us so
+// (957 without the bound, 726 at 80 registers, 703 at 48).
+__global__ void __launch_bounds__(256, 4) query_g_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-  const int lane = threadIdx.x & 31, j = lane & 7;
-  const unsigned gm = 0xFFu << (lane & 24);
+  const int lane = threadIdx.x & 31;
   if (gid >= n) return;
+  const Group<1> G(lane);
   const QueryIn q = in[gid];
   const FieldView &f = P.f;
+  const GroupInit init = init_g(f, q, lane);
   QueryOut o;
-  o.ok = 0; o.id = 0; o.s1d = q.s1d; o.dx = o.dy = o.dz = 0.0f; o.pdf = 0.0f; o.pdfLi = 0.0f;
-  bool inside = f.iteration > 0 && q.px >= f.bounds[0] && q.px <= f.bounds[3] && q.py >= f.bounds[1] &&
-                q.py <= f.bounds[4] && q.pz >= f.bounds[2] && q.pz <= f.bounds[5];
-  if (inside) {
-    uint32_t leaf = kd_leaf(f, q.px, q.py, q.pz);
-    uint32_t reg = leaf;
-    float s1d = q.s1d;
-    if (f.knn && s1d >= 0.f) reg = choose_region_g(f, leaf, q.px, q.py, q.pz, s1d, j, lane, gm);
-    o.s1d = s1d;
-    const RegionDir &R = f.regions[reg];
-    if (R.valid) {
-      const int K = int(R.vmm.K), cnt = vec_count(K);
-      const LobeSet li = load_shifted_g(R.vmm, j, q.px, q.py, q.pz, f.parallax != 0, cnt);
-      V3 d;
-      if (P.cosine) {
-        const LobeSet g = product_lobe_g(li, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, gm);
-        d = mixture_sample_g(g, K, (q.ux - 0.0f) / 1.0f, q.uy, gm);
-        o.pdf = 0.0f + 1.0f * mixture_pdf_g(g, d, cnt, gm);
-      } else {
-        d = mixture_sample_g(li, K, (q.ux - 0.0f) / 1.0f, q.uy, gm);
-        o.pdf = 0.0f + 1.0f * mixture_pdf_g(li, d, cnt, gm);
-      }
-      o.ok = 1;
-      o.id = leaf;
-      o.dx = d.x; o.dy = d.y; o.dz = d.z;
-      o.pdfLi = mixture_pdf_g(li, d, cnt, gm);
+  o.ok = 0; o.id = 0; o.s1d = init.s1d; o.dx = o.dy = o.dz = 0.0f; o.pdf = 0.0f; o.pdfLi = 0.0f;
+  if (init.ok) {
+    const VMMState &v = f.regions[init.reg].vmm;
+    const int K = int(v.K), cnt = vec_count(K);
+    const LobeSet<1> li = load_shifted_g<1>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
+    V3 d;
+    if (P.cosine) {
+      float integral;
+      const LobeSet<1> g =
+          product_lobe_g<1>(G, li, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, integral);
+      const PickedLobe p = mixture_pick_g<1>(G, g, K, q.uy);
+      d = lobe_direction(p.kappa, p.e2k, p.mu, (q.ux - 0.0f) / 1.0f, p.u1);
+      o.pdf = 0.0f + 1.0f * mixture_pdf_g<1>(G, g, d, cnt);
+    } else {
+      const PickedLobe p = mixture_pick_g<1>(G, li, K, q.uy);
+      d = lobe_direction(p.kappa, p.e2k, p.mu, (q.ux - 0.0f) / 1.0f, p.u1);
+      o.pdf = 0.0f + 1.0f * mixture_pdf_g<1>(G, li, d, cnt);
     }
+    o.ok = 1;
+    o.id = init.leaf;
+    o.dx = d.x; o.dy = d.y; o.dz = d.z;
+    o.pdfLi = mixture_pdf_g<1>(G, li, d, cnt);
   }
-  if (j == 0) out[gid] = o;
+  if (G.j == 0) out[gid] = o;
 }
 // Batched path-vertex query, four per warp: Init + cosine product once, then
 // one SamplePDF per 2D random number on the same distribution (the sampled
 // distribution is not changed by sampling: VMMSurfaceSamplingDistribution.h:67-103),
 // as a renderer does per vertex and openpgl_bench's lookup loop does per
-// initialised distribution (openpgl_bench.cpp:343-362).
-__global__ void query_s4_g_kernel(QueryParams P, const QueryInS4 *in, QueryOutS4 *out, uint32_t n) {
+// initialised distribution (openpgl_bench.cpp:343-362).  The group picks the
+// four lobes one after the other, then lane k (and k + 4) finds the direction of
+// sample k: one run through lobe_direction per vertex in place of four.
+// 1,048,576 vertices: 1,838 us with four runs, 911 us so.
+__global__ void __launch_bounds__(256, 4)
+query_s4_g_kernel(QueryParams P, const QueryInS4 *in, QueryOutS4 *out, uint32_t n) {
+  static_assert(kVertexSamples == 4, "two lanes of a group per sample");
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-  const int lane = threadIdx.x & 31, j = lane & 7;
-  const unsigned gm = 0xFFu << (lane & 24);
+  const int lane = threadIdx.x & 31;
   if (gid >= n) return;
-  const QueryInS4 q = in[gid];
+  const Group<1> G(lane);
+  const QueryInS4 &q = in[gid];
   const FieldView &f = P.f;
-  QueryOutS4 o;
-  o.ok = 0;
-  o.id = 0;
-  o.s1d = q.s1d;
-#pragma unroll
-  for (int k = 0; k < kVertexSamples; ++k) o.s[k][0] = o.s[k][1] = o.s[k][2] = o.s[k][3] = 0.0f;
-  bool inside = f.iteration > 0 && q.px >= f.bounds[0] && q.px <= f.bounds[3] && q.py >= f.bounds[1] &&
-                q.py <= f.bounds[4] && q.pz >= f.bounds[2] && q.pz <= f.bounds[5];
-  if (inside) {
-    uint32_t leaf = kd_leaf(f, q.px, q.py, q.pz);
-    uint32_t reg = leaf;
-    float s1d = q.s1d;
-    if (f.knn && s1d >= 0.f) reg = choose_region_g(f, leaf, q.px, q.py, q.pz, s1d, j, lane, gm);
-    o.s1d = s1d;
-    const RegionDir &R = f.regions[reg];
-    if (R.valid) {
-      const int K = int(R.vmm.K), cnt = vec_count(K);
-      LobeSet g = load_shifted_g(R.vmm, j, q.px, q.py, q.pz, f.parallax != 0, cnt);
-      if (P.cosine) g = product_lobe_g(g, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, gm);
-#pragma unroll
-      for (int k = 0; k < kVertexSamples; ++k) {
-        const V3 d = mixture_sample_g(g, K, (q.u[k][0] - 0.0f) / 1.0f, q.u[k][1], gm);
-        o.s[k][0] = d.x;
-        o.s[k][1] = d.y;
-        o.s[k][2] = d.z;
-        o.s[k][3] = 0.0f + 1.0f * mixture_pdf_g(g, d, cnt, gm);
-      }
-      o.ok = 1;
-      o.id = leaf;
+  struct {
+    float px, py, pz, s1d;
+  } at = {q.px, q.py, q.pz, q.s1d};
+  const GroupInit init = init_g(f, at, lane);
+  const int mine = G.j & 3;
+  const float ux = q.u[mine][0], uyMine = q.u[mine][1];
+  V3 d = mk(0.0f, 0.0f, 0.0f);
+  float pdf = 0.0f;  // of sample `mine`
+  if (init.ok) {
+    const VMMState &v = f.regions[init.reg].vmm;
+    const int K = int(v.K), cnt = vec_count(K);
+    LobeSet<1> g = load_shifted_g<1>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
+    float integral;
+    if (P.cosine) g = product_lobe_g<1>(G, g, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, integral);
+    PickedLobe p{};
+#pragma unroll 1
+    for (int k = 0; k < kVertexSamples; ++k) {
+      const PickedLobe t = mixture_pick_g<1>(G, g, K, G.from(uyMine, k));
+      if (k == mine) p = t;
+    }
+    d = lobe_direction(p.kappa, p.e2k, p.mu, (ux - 0.0f) / 1.0f, p.u1);
+#pragma unroll 1
+    for (int k = 0; k < kVertexSamples; ++k) {
+      const V3 dk = mk(G.from(d.x, k), G.from(d.y, k), G.from(d.z, k));
+      const float t = 0.0f + 1.0f * mixture_pdf_g<1>(G, g, dk, cnt);
+      if (k == mine) pdf = t;
     }
   }
-  if (j == 0) out[gid] = o;
+  QueryOutS4 &o = out[gid];
+  if (G.j == 0) {
+    o.ok = init.ok ? 1u : 0u;
+    o.id = init.ok ? init.leaf : 0u;
+    o.s1d = init.s1d;
+  }
+  if (G.j < kVertexSamples) {
+    o.s[mine][0] = d.x;
+    o.s[mine][1] = d.y;
+    o.s[mine][2] = d.z;
+    o.s[mine][3] = pdf;
+  }
 }
 
 
@@ -760,7 +867,7 @@ cudaError_t launch_query(const QueryParams &p, const QueryIn *in, QueryOut *out,
     return cudaGetLastError();
   }
   if (p.hgMeanCosine) {
-    query_hg_kernel<<<unsigned((uint64_t(n) * 32 + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
+    query_hg_kernel<<<unsigned((uint64_t(n) * 16 + 127) / 128), 128, 0, s>>>(p, in, out, n);
     return cudaGetLastError();
   }
   query_g_kernel<<<unsigned((uint64_t(n) * 8 + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
