@@ -3,10 +3,11 @@
 // pdf evaluation (Field.h:109-145, KNN.h:22-28,134-148,
 // VMMSurfaceSamplingDistribution.h:37-108, PAVMM.h:609-831).
 //
-// One warp per query, lane k owning mixture lobe k, which mirrors the
-// reference's 8-wide SIMD lanes: per-lane arithmetic is the reference's, and
-// horizontal sums use shuffles in the vfloat8 reduce order (lanes j, j+8, j+16,
-// j+24 summed in vector order, then the 8-lane tree).
+// The arithmetic mirrors the reference's 8-wide SIMD lanes: per-lobe arithmetic
+// is the reference's, and horizontal sums use shuffles in the vfloat8 reduce
+// order (lobes j, j+8, j+16, j+24 summed in vector order, then the 8-lane tree).
+// Per-object calls take a warp with lane k owning lobe k, batches several
+// queries per warp with two or four lobes per lane.
 #include <cuda_runtime.h>
 
 #include "dqt.cuh"
@@ -477,6 +478,38 @@ __device__ __forceinline__ PickedLobe mixture_pick_g(const Group<kH> &G, const L
   r.mu = mk(G.from(held(&Lobe::mx), src), G.from(held(&Lobe::my), src), G.from(held(&Lobe::mz), src));
   return r;
 }
+// The directions of a block's kN picked lobes, a thread per lobe (groups would
+// run lobe_direction on one lobe with all their lanes: its logarithm, sine and
+// cosine, and frame cost a sixth of a surface query).  Every thread of the block
+// calls it; `writer` threads hand in the lobe of slot `i`, every thread gets the
+// direction of slot `i`.  1,048,576 surface queries 706 -> 635 us, 262,147 with
+// the phase function 411 -> 377 us, 1,000,003 vertices 911 -> 877 us.
+template <int kN>
+struct DirectionSlots {
+  float kappa[kN], e2k[kN], u1[kN], ux[kN], x[kN], y[kN], z[kN];
+};
+template <int kN>
+__device__ __forceinline__ V3 block_direction(DirectionSlots<kN> &S, int i, bool writer, const PickedLobe &p, float ux) {
+  if (writer) {
+    S.kappa[i] = p.kappa;
+    S.e2k[i] = p.e2k;
+    S.u1[i] = p.u1;
+    S.ux[i] = ux;
+    S.x[i] = p.mu.x;
+    S.y[i] = p.mu.y;
+    S.z[i] = p.mu.z;
+  }
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t < kN) {
+    const V3 d = lobe_direction(S.kappa[t], S.e2k[t], mk(S.x[t], S.y[t], S.z[t]), S.ux[t], S.u1[t]);
+    S.x[t] = d.x;
+    S.y[t] = d.y;
+    S.z[t] = d.z;
+  }
+  __syncthreads();
+  return mk(S.x[i], S.y[i], S.z[i]);
+}
 // choose_region by a group: lane j ranks neighbour j
 __device__ uint32_t choose_region_g(const FieldView &f, uint32_t leaf, float p0, float p1, float p2, float &s1d,
                                     int j, int lane, unsigned gm) {
@@ -520,37 +553,37 @@ __device__ __forceinline__ GroupInit init_g(const FieldView &f, const Q &q, int 
   return r;
 }
 
+constexpr int kQueryThreads = 256, kHgThreads = 256, kHgBlocks = 4;
 // Batched volume guided queries with the Henyey-Greenstein product, two per
 // warp: Init + product with the phase function's fit + SamplePDF (+ pdfLi).
 // The mixture and its three products are live together, so a lane holds two
-// lobes of each; 72 registers for seven blocks per SM.  262,144 queries:
-// 507 us with a warp per query, 411 us so (450 at 93 registers, 646 four per
-// warp with the large mixtures redone by the whole warp).
-__global__ void __launch_bounds__(128, 7) query_hg_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+// lobes of each; 64 registers for four blocks per SM.  262,147 queries: 507 us
+// with a warp per query, 377 us so (383 at 80 registers, 387 in blocks of 128
+// threads, 490 in blocks of 512).
+__global__ void __launch_bounds__(kHgThreads, kHgBlocks)
+query_hg_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+  __shared__ DirectionSlots<kHgThreads / 16> slots;
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
   const int lane = threadIdx.x & 31;
-  if (gid >= n) return;
   const Group<2> G(lane);
   const FieldView &f = P.f;
-  const QueryIn q = in[gid];
+  const QueryIn q = in[min(gid, n - 1)];
   const GroupInit init = init_g(f, q, lane);
-  QueryOut o;
-  o.ok = init.ok ? 1u : 0u;
-  o.id = init.ok ? init.leaf : 0u;
-  o.s1d = init.s1d;
-  o.dx = o.dy = o.dz = 0.0f;
-  o.pdf = o.pdfLi = 0.0f;
-  if (init.ok) {
+  LobeSet<2> li, h[kHgLobes];
+  float w[kHgLobes], ux = 0.0f;
+  PickedLobe p{};
+  int cnt = 0;
+  if (init.ok) {  // an untrained field has no regions to read
     const VMMState &v = f.regions[init.reg].vmm;
-    const int K = int(v.K), cnt = vec_count(K);
-    const LobeSet<2> li = load_shifted_g<2>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
-    const float meanCosine = P.hgMeanCosine[gid];
+    const int K = int(v.K);
+    cnt = vec_count(K);
+    li = load_shifted_g<2>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
+    const float meanCosine = P.hgMeanCosine[gid < n ? gid : n - 1];
     const float step = (kHgMaxMeanCosine - kHgMinMeanCosine) / float(kHgFits);
     int idx = int(floorf((fabsf(meanCosine) - kHgMinMeanCosine) / step));
     idx = idx < kHgFits - 1 ? idx : kHgFits - 1;
     const V3 dir = mk(q.nx, q.ny, q.nz);
-    LobeSet<2> h[kHgLobes];
-    float w[kHgLobes], sum = 0.0f;
+    float sum = 0.0f;
 #pragma unroll
     for (int i = 0; i < kHgLobes; ++i) {  // hg_products
       const HgLobeFit fit = c_hg[idx][i];
@@ -570,8 +603,17 @@ __global__ void __launch_bounds__(128, 7) query_hg_kernel(QueryParams P, const Q
     }
     const LobeSet<2> g = i == 0 ? h[0] : (i == 1 ? h[1] : h[2]);
     const float wi = i == 0 ? w[0] : (i == 1 ? w[1] : w[2]);
-    const PickedLobe p = mixture_pick_g<2>(G, g, K, q.uy);
-    const V3 d = lobe_direction(p.kappa, p.e2k, p.mu, (q.ux - acc) / wi, p.u1);
+    p = mixture_pick_g<2>(G, g, K, q.uy);
+    ux = (q.ux - acc) / wi;
+  }
+  const V3 d = block_direction(slots, threadIdx.x >> 4, G.j == 0, p, ux);
+  QueryOut o;
+  o.ok = init.ok ? 1u : 0u;
+  o.id = init.ok ? init.leaf : 0u;
+  o.s1d = init.s1d;
+  o.dx = o.dy = o.dz = 0.0f;
+  o.pdf = o.pdfLi = 0.0f;
+  if (init.ok) {
 #pragma unroll
     for (int k = 0; k < kHgLobes; ++k) o.pdf += w[k] * mixture_pdf_g<2>(G, h[k], d, cnt);
     o.dx = d.x;
@@ -579,65 +621,65 @@ __global__ void __launch_bounds__(128, 7) query_hg_kernel(QueryParams P, const Q
     o.dz = d.z;
     o.pdfLi = mixture_pdf_g<2>(G, li, d, cnt);
   }
-  if (G.j == 0) out[gid] = o;
+  if (gid < n && G.j == 0) out[gid] = o;
 }
 
 // Batched guided queries, four per warp: Init + optional cosine product
 // (surface) + SamplePDF (+ pdfLi).  Issue bound at about three quarters of the
 // issue rate; 64 registers for four blocks per SM.  1,048,576 queries: 818 us
 // with searches by branches, FP64 in lobe_direction, divisions one by one and
-// the rsqrt table in constant memory (its lookups went one by one), 706 us so
-// (957 without the bound, 726 at 80 registers, 703 at 48).
-__global__ void __launch_bounds__(256, 4) query_g_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+// the rsqrt table in constant memory (its lookups went one by one), 635 us so
+// (687 at 80 registers, 660 at 48, 669 in blocks of 128 threads).
+__global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
+query_g_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+  __shared__ DirectionSlots<kQueryThreads / 8> slots;
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   const int lane = threadIdx.x & 31;
-  if (gid >= n) return;
   const Group<1> G(lane);
-  const QueryIn q = in[gid];
+  const QueryIn q = in[min(gid, n - 1)];
   const FieldView &f = P.f;
   const GroupInit init = init_g(f, q, lane);
+  LobeSet<1> li, g;
+  PickedLobe p{};
+  int cnt = 0;
+  if (init.ok) {  // an untrained field has no regions to read
+    const VMMState &v = f.regions[init.reg].vmm;
+    const int K = int(v.K);
+    cnt = vec_count(K);
+    li = load_shifted_g<1>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
+    float integral;
+    g = li;
+    if (P.cosine) g = product_lobe_g<1>(G, li, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, integral);
+    p = mixture_pick_g<1>(G, g, K, q.uy);
+  }
+  const V3 d = block_direction(slots, threadIdx.x >> 3, G.j == 0, p, (q.ux - 0.0f) / 1.0f);
   QueryOut o;
   o.ok = 0; o.id = 0; o.s1d = init.s1d; o.dx = o.dy = o.dz = 0.0f; o.pdf = 0.0f; o.pdfLi = 0.0f;
   if (init.ok) {
-    const VMMState &v = f.regions[init.reg].vmm;
-    const int K = int(v.K), cnt = vec_count(K);
-    const LobeSet<1> li = load_shifted_g<1>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
-    V3 d;
-    if (P.cosine) {
-      float integral;
-      const LobeSet<1> g =
-          product_lobe_g<1>(G, li, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, integral);
-      const PickedLobe p = mixture_pick_g<1>(G, g, K, q.uy);
-      d = lobe_direction(p.kappa, p.e2k, p.mu, (q.ux - 0.0f) / 1.0f, p.u1);
-      o.pdf = 0.0f + 1.0f * mixture_pdf_g<1>(G, g, d, cnt);
-    } else {
-      const PickedLobe p = mixture_pick_g<1>(G, li, K, q.uy);
-      d = lobe_direction(p.kappa, p.e2k, p.mu, (q.ux - 0.0f) / 1.0f, p.u1);
-      o.pdf = 0.0f + 1.0f * mixture_pdf_g<1>(G, li, d, cnt);
-    }
     o.ok = 1;
     o.id = init.leaf;
     o.dx = d.x; o.dy = d.y; o.dz = d.z;
+    o.pdf = 0.0f + 1.0f * mixture_pdf_g<1>(G, g, d, cnt);
     o.pdfLi = mixture_pdf_g<1>(G, li, d, cnt);
   }
-  if (G.j == 0) out[gid] = o;
+  if (gid < n && G.j == 0) out[gid] = o;
 }
 // Batched path-vertex query, four per warp: Init + cosine product once, then
 // one SamplePDF per 2D random number on the same distribution (the sampled
 // distribution is not changed by sampling: VMMSurfaceSamplingDistribution.h:67-103),
 // as a renderer does per vertex and openpgl_bench's lookup loop does per
 // initialised distribution (openpgl_bench.cpp:343-362).  The group picks the
-// four lobes one after the other, then lane k (and k + 4) finds the direction of
-// sample k: one run through lobe_direction per vertex in place of four.
-// 1,048,576 vertices: 1,838 us with four runs, 911 us so.
-__global__ void __launch_bounds__(256, 4)
+// four lobes one after the other, and the block finds all their directions at
+// once.  1,000,003 vertices: 1,838 us with four runs through lobe_direction per
+// vertex, 877 us so.
+__global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
 query_s4_g_kernel(QueryParams P, const QueryInS4 *in, QueryOutS4 *out, uint32_t n) {
   static_assert(kVertexSamples == 4, "two lanes of a group per sample");
+  __shared__ DirectionSlots<kQueryThreads / 2> slots;
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   const int lane = threadIdx.x & 31;
-  if (gid >= n) return;
   const Group<1> G(lane);
-  const QueryInS4 &q = in[gid];
+  const QueryInS4 &q = in[min(gid, n - 1)];
   const FieldView &f = P.f;
   struct {
     float px, py, pz, s1d;
@@ -645,28 +687,35 @@ query_s4_g_kernel(QueryParams P, const QueryInS4 *in, QueryOutS4 *out, uint32_t 
   const GroupInit init = init_g(f, at, lane);
   const int mine = G.j & 3;
   const float ux = q.u[mine][0], uyMine = q.u[mine][1];
-  V3 d = mk(0.0f, 0.0f, 0.0f);
-  float pdf = 0.0f;  // of sample `mine`
-  if (init.ok) {
+  LobeSet<1> g;
+  PickedLobe p{};
+  int cnt = 0;
+  if (init.ok) {  // an untrained field has no regions to read
     const VMMState &v = f.regions[init.reg].vmm;
-    const int K = int(v.K), cnt = vec_count(K);
-    LobeSet<1> g = load_shifted_g<1>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
+    const int K = int(v.K);
+    cnt = vec_count(K);
+    g = load_shifted_g<1>(G, v, q.px, q.py, q.pz, f.parallax != 0, cnt);
     float integral;
     if (P.cosine) g = product_lobe_g<1>(G, g, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, integral);
-    PickedLobe p{};
 #pragma unroll 1
     for (int k = 0; k < kVertexSamples; ++k) {
       const PickedLobe t = mixture_pick_g<1>(G, g, K, G.from(uyMine, k));
       if (k == mine) p = t;
     }
-    d = lobe_direction(p.kappa, p.e2k, p.mu, (ux - 0.0f) / 1.0f, p.u1);
+  }
+  V3 d = block_direction(slots, (threadIdx.x >> 3) * 4 + mine, G.j < kVertexSamples, p, (ux - 0.0f) / 1.0f);
+  float pdf = 0.0f;  // of sample `mine`
+  if (init.ok) {
 #pragma unroll 1
     for (int k = 0; k < kVertexSamples; ++k) {
       const V3 dk = mk(G.from(d.x, k), G.from(d.y, k), G.from(d.z, k));
       const float t = 0.0f + 1.0f * mixture_pdf_g<1>(G, g, dk, cnt);
       if (k == mine) pdf = t;
     }
+  } else {
+    d = mk(0.0f, 0.0f, 0.0f);
   }
+  if (gid >= n) return;
   QueryOutS4 &o = out[gid];
   if (G.j == 0) {
     o.ok = init.ok ? 1u : 0u;
@@ -867,10 +916,10 @@ cudaError_t launch_query(const QueryParams &p, const QueryIn *in, QueryOut *out,
     return cudaGetLastError();
   }
   if (p.hgMeanCosine) {
-    query_hg_kernel<<<unsigned((uint64_t(n) * 16 + 127) / 128), 128, 0, s>>>(p, in, out, n);
+    query_hg_kernel<<<unsigned((uint64_t(n) * 16 + kHgThreads - 1) / kHgThreads), kHgThreads, 0, s>>>(p, in, out, n);
     return cudaGetLastError();
   }
-  query_g_kernel<<<unsigned((uint64_t(n) * 8 + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
+  query_g_kernel<<<unsigned((uint64_t(n) * 8 + kQueryThreads - 1) / kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
   return cudaGetLastError();
 }
 cudaError_t launch_query_s4(const QueryParams &p, const QueryInS4 *in, QueryOutS4 *out, uint32_t n,
@@ -882,7 +931,7 @@ cudaError_t launch_query_s4(const QueryParams &p, const QueryInS4 *in, QueryOutS
     query_s4_dqt_kernel<<<unsigned((uint64_t(n) + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
     return cudaGetLastError();
   }
-  query_s4_g_kernel<<<unsigned((uint64_t(n) * 8 + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
+  query_s4_g_kernel<<<unsigned((uint64_t(n) * 8 + kQueryThreads - 1) / kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
   return cudaGetLastError();
 }
 cudaError_t launch_ssd_init(const FieldView &f, float px, float py, float pz, float s1d, SSDState *st, SSDResult *res,

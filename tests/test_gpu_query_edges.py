@@ -96,3 +96,25 @@ def test_ends_of_the_random_numbers(field):
             assert np.array(d, np.float32).tobytes() == out["dir"][i].tobytes(), i
             assert np.float32(pdf).tobytes() == out["pdf"][i].tobytes(), i
         sd.release()
+
+
+def test_untrained_side():
+    """Queries on a side of the field without regions, and on a field before its
+    first Update: all refused, nothing read."""
+    import openpgl_gb300 as pgl
+    from openpgl_gb300 import synthetic as syn
+
+    dev = pgl.Device()
+    f = pgl.Field(dev, pgl.FieldConfig(True, 4000))
+    q, v = syn.queries(100, 304), syn.vertices(100, 305)
+    g = np.full(100, 0.5, np.float32)
+    st = pgl.SampleStorage()
+    st.add_samples(syn.cube_face_samples(20000, 306))
+    for trained in (False, True):
+        if trained:
+            f.update(st)
+        assert not f.sample_batch_hg(q, g)["ok"].any()
+        assert not f.sample_batch(q, volume=True, cosine=False)["ok"].any()
+        assert f.sample_batch(q)["ok"].any() == trained
+        assert f.sample_vertices(v)["ok"].any() == trained
+    f.release()
