@@ -164,7 +164,7 @@ struct PathSegmentRecord;
 struct PathFlags;
 cudaError_t launch_path_samples(const PathSegmentRecord *seg, const uint32_t *begin, uint32_t numPaths,
                                 float maxDistance, PathFlags fl, PGLSampleRecord *out, uint32_t *offsets,
-                                Scratch &scratch, cudaStream_t s);
+                                Scratch &scratch, int numSMs, cudaStream_t s);
 cudaError_t launch_ssd_init(const FieldView &f, float px, float py, float pz, float s1d, SSDState *st, SSDResult *res,
                             cudaStream_t s);
 cudaError_t launch_ssd_cosine(SSDState *st, float nx, float ny, float nz, float ck, float cn, cudaStream_t s);

@@ -234,7 +234,7 @@ OPENPGL_CORE_INTERFACE bool pglPathSegmentsPrepareSamplesDevice(const PGLPathSeg
   static thread_local Scratch scratch;
   check(launch_path_samples(reinterpret_cast<const PathSegmentRecord *>(dSegments), dPathBegin, uint32_t(numPaths),
                             maxDistance, PathFlags{useNEEMiWeights, guideDirectLight, rrAffectsDirectContribution},
-                            reinterpret_cast<PGLSampleRecord *>(dSamples), dSampleBegin, scratch, st),
+                            reinterpret_cast<PGLSampleRecord *>(dSamples), dSampleBegin, scratch, c.numSMs, st),
         "path samples");
   return true;
   PGL_PS_CATCH(false)
@@ -262,6 +262,7 @@ OPENPGL_CORE_INTERFACE size_t pglPathSegmentsPropagateSamplesDevice(const PGLPat
   uint32_t total = 0;
   check(cudaMemcpyAsync(&total, offsets.p + numPaths, 4, cudaMemcpyDeviceToHost, c.stream), "sample count");
   check(cudaStreamSynchronize(c.stream), "path samples");
+  if (total == ~0u) throw std::runtime_error("path samples: a block gave up waiting for the ones before it");
   reinterpret_cast<Storage *>(sampleStorage)->ingestDevice(out.p, total);
   return total;
   PGL_PS_CATCH(0)
