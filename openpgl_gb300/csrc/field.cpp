@@ -704,8 +704,8 @@ bool SubField::prepare(SampleSide &in) {
     iteration = 0;
     totalSPP = 0;
   }
-  for (DevArray<float4> *a : {&posA_, &posB_, &sP_, &sD_, &tmpP_, &tmpD_}) a->reserve(n);
-  for (DevArray<float> *a : {&sPdf_, &tmpPdf_, &dist_}) a->reserve(n);
+  for (DevArray<float4> *a : {&posA_, &posB_, &sP_, &sD_}) a->reserve(n);
+  for (DevArray<float> *a : {&sPdf_, &dist_}) a->reserve(n);
   for (DevArray<uint32_t> *a : {&node_, &nodeB_, &jobOf_, &isLeft_, &scanLeft_}) a->reserve(n);
   keys_.reserve(2 * size_t(n));
   vals_.reserve(2 * size_t(n));
@@ -804,7 +804,7 @@ bool SubField::prepare(SampleSide &in) {
   leafSeg_.reserve(seg.size());
   check(cudaMemcpyAsync(leafSeg_.p, seg.data(), seg.size() * 4, cudaMemcpyHostToDevice, stream()), "segments");
   check(gather_and_order(posA_.p, n, in.P.p, in.D.p, in.pdf.p, leafSeg_.p, leafSeg_.p + 2 * L, L, cfg.deterministic,
-                         tmpP_.p, tmpD_.p, tmpPdf_.p, keys_.p, vals_.p, keys64_.p, sP_.p, sD_.p, sPdf_.p, scratch_,
+                         vals_.p, keys64_.p, sP_.p, sD_.p, sPdf_.p, scratch_,
                          stream()),
         "gather");
 
@@ -1289,8 +1289,8 @@ void GpuField::runEm(SubField *const *sides, int count) {
 }
 
 size_t SubField::workBytes() const {
-  return posA_.bytes() + posB_.bytes() + sP_.bytes() + sD_.bytes() + tmpP_.bytes() + tmpD_.bytes() + sPdf_.bytes() +
-         tmpPdf_.bytes() + dist_.bytes() + node_.bytes() + nodeB_.bytes() + jobOf_.bytes() + isLeft_.bytes() +
+  return posA_.bytes() + posB_.bytes() + sP_.bytes() + sD_.bytes() + sPdf_.bytes() +
+         dist_.bytes() + node_.bytes() + nodeB_.bytes() + jobOf_.bytes() + isLeft_.bytes() +
          scanLeft_.bytes() + keys_.bytes() + vals_.bytes() + nodeToJob_.bytes() + leafSeg_.bytes() + copyIdx_.bytes() +
          keysB_.bytes() + valsB_.bytes() + routeNodes_.bytes() + keys64_.bytes() + jobs_.bytes() + acc_.bytes() +
          means_.bytes() + bounds6_.bytes() + scratch_.bytes;

@@ -106,8 +106,7 @@ cudaError_t kd_level(const float4 *pos, const uint32_t *jobOf, uint32_t n, const
 // order (SampleDataLess) when `sorted`; leafBegin/leafCount are device arrays.
 cudaError_t gather_and_order(const float4 *posIdx, uint32_t n, const float4 *P, const float4 *D, const float *pdf,
                              const uint32_t *leafBegin, const uint32_t *leafCount, uint32_t numLeaves, bool sorted,
-                             float4 *tmpP, float4 *tmpD, float *tmpPdf, uint32_t *keys, uint32_t *vals,
-                             unsigned long long *keys64, float4 *oP, float4 *oD, float *oPdf, Scratch &scratch,
+                             uint32_t *vals, unsigned long long *keys64, float4 *oP, float4 *oD, float *oPdf, Scratch &scratch,
                              cudaStream_t s);
 cudaError_t copy_regions(RegionDir *regions, const uint32_t *dst, const uint32_t *src, uint32_t n, cudaStream_t s);
 cudaError_t build_knn(const float4 *means, uint32_t R, Neighbours *out, cudaStream_t s);

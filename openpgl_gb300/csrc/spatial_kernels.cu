@@ -77,8 +77,15 @@ __device__ __forceinline__ uint32_t ford(float f) {
   uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-__global__ void bounds_kernel(const float4 *P, uint64_t n, uint32_t *out6) {
+__device__ __forceinline__ float unford(uint32_t o) {
+  return __uint_as_float((o & 0x80000000u) ? o & 0x7FFFFFFFu : ~o);
+}
+// Bounds of the positions as ordered integers.  Bytes bound (1.5M positions in
+// 7 us) with six atomics per block; with six per warp they took 130 us.
+__global__ void __launch_bounds__(256) bounds_kernel(const float4 *P, uint64_t n, uint32_t *out6) {
+  __shared__ uint32_t part[8][6];
   uint32_t lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0, 0, 0};
+#pragma unroll 4
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
     float4 p = P[i];
     float c[3] = {p.x, p.y, p.z};
@@ -89,34 +96,57 @@ __global__ void bounds_kernel(const float4 *P, uint64_t n, uint32_t *out6) {
     }
   }
   for (int d = 0; d < 3; ++d) {
-    for (int off = 16; off > 0; off >>= 1) {
-      lo[d] = min(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], off));
-      hi[d] = max(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], off));
-    }
+    lo[d] = __reduce_min_sync(0xFFFFFFFFu, lo[d]);
+    hi[d] = __reduce_max_sync(0xFFFFFFFFu, hi[d]);
   }
   if ((threadIdx.x & 31) == 0)
     for (int d = 0; d < 3; ++d) {
-      atomicMin(&out6[d], lo[d]);
-      atomicMax(&out6[3 + d], hi[d]);
+      part[threadIdx.x >> 5][d] = lo[d];
+      part[threadIdx.x >> 5][3 + d] = hi[d];
     }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    uint32_t v = part[0][threadIdx.x];
+    for (int w = 1; w < 8; ++w) {
+      const uint32_t o = part[w][threadIdx.x];
+      v = threadIdx.x < 3 ? min(v, o) : max(v, o);
+    }
+    if (threadIdx.x < 3) atomicMin(&out6[threadIdx.x], v);
+    else atomicMax(&out6[threadIdx.x], v);
+  }
 }
 
 // ------------------------------------------------------------------ kd levels
 // One job per inner node visited at the current level.
 
 constexpr int kKdThreads = 256;
-constexpr int kKdItems = 16;                      // samples per thread
+constexpr int kKdItems = 8;                       // samples per thread
 constexpr int kKdTile = kKdThreads * kKdItems;    // samples per block
-constexpr int kKdLocal = 16;                      // distinct jobs aggregated per block
 
-__device__ __forceinline__ void quantize(const KdJob &j, float4 p, long long q[3], long long qv[3]) {
-  float c[3] = {p.x, p.y, p.z};
+// A sample's place in its node's frame in units of 1 / 4096, before and after
+// the conversion to integers (in 32 bits where that holds them: the 64-bit
+// conversion runs at a fraction of the rate: with it the root's statistics took
+// 22 us of 1.5M samples in place of 12, 62 us with an atomic per warp).
+__device__ __noinline__ long long to_int64(float t) { return (long long)t; }
+__device__ __forceinline__ void quantize(const KdJob &j, float4 p, float t[3], long long q[3], long long qv[3]) {
+  float c[3] = {p.x, p.y, p.z}, tv[3];
+  bool small = true;
   for (int d = 0; d < 3; ++d) {
-    float t = (c[d] - j.c[d]) * j.inv[d];
-    float tv = (t * t) * 4096.f;
-    t *= 4096.f;
-    q[d] = (long long)t;
-    qv[d] = (long long)tv;
+    t[d] = (c[d] - j.c[d]) * j.inv[d];
+    tv[d] = (t[d] * t[d]) * 4096.f;
+    t[d] *= 4096.f;
+    small = small && fabsf(t[d]) < 0x1p31f && tv[d] < 0x1p31f;
+  }
+  if (small) {
+    for (int d = 0; d < 3; ++d) {
+      q[d] = __float2int_rz(t[d]);
+      qv[d] = __float2int_rz(tv[d]);
+    }
+  } else {
+    for (int d = 0; d < 3; ++d) {
+      q[d] = to_int64(t[d]);
+      qv[d] = to_int64(tv[d]);
+    }
   }
 }
 
@@ -133,56 +163,110 @@ __device__ __forceinline__ void acc_add(IStatsAcc *a, const long long m[3], cons
   atomicAdd(&a->n, n);
 }
 
-// A warp's running integer statistics of one job's two children, per lane.
+// Smallest and largest integers of some samples by their unconverted floats (the
+// conversion keeps the order; a NaN converts to the smallest integer, infinities
+// to the ends, which are also what no samples leave).
+struct FloatRange {
+  float lo, hi;
+  __device__ __forceinline__ void clear() {
+    lo = INFINITY;
+    hi = -INFINITY;
+  }
+  __device__ __forceinline__ void add(float t, bool on) {
+    lo = fminf(lo, on ? (t == t ? t : -INFINITY) : INFINITY);
+    hi = fmaxf(hi, on ? t : -INFINITY);
+  }
+  __device__ __forceinline__ void warp(long long &l, long long &h) const {
+    l = (long long)unford(__reduce_min_sync(0xFFFFFFFFu, ford(lo)));
+    h = (long long)unford(__reduce_max_sync(0xFFFFFFFFu, ford(hi)));
+  }
+};
+// A warp's running integer statistics of one job: sums over all samples and
+// over the left ones per lane, ranges of both sides per lane, counts per warp.
 struct WarpSideAcc {
-  long long m[2][3], v[2][3], lo[2][3], hi[2][3];
-  unsigned long long n[2];
+  long long m[3], v[3], ml[3], vl[3];
+  FloatRange range[2][3];
+  uint32_t n, nl;
   __device__ __forceinline__ void clear() {
 #pragma unroll
-    for (int sd = 0; sd < 2; ++sd) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) { m[sd][d] = 0; v[sd][d] = 0; lo[sd][d] = LLONG_MAX; hi[sd][d] = LLONG_MIN; }
-      n[sd] = 0;
+    for (int d = 0; d < 3; ++d) {
+      m[d] = v[d] = ml[d] = vl[d] = 0;
+      range[0][d].clear();
+      range[1][d].clear();
     }
+    n = nl = 0;
   }
 };
 __device__ __forceinline__ long long warp_sum64(long long x) {
   for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, off);
   return x;
 }
-__device__ __forceinline__ long long warp_min64(long long x) {
-  for (int off = 16; off > 0; off >>= 1) x = min(x, __shfl_xor_sync(0xFFFFFFFFu, x, off));
-  return x;
-}
-__device__ __forceinline__ long long warp_max64(long long x) {
-  for (int off = 16; off > 0; off >>= 1) x = max(x, __shfl_xor_sync(0xFFFFFFFFu, x, off));
-  return x;
-}
-// Adds a warp's running statistics of job `job` to acc[2 job + side] (or to
-// the block's shared copy) and clears them.
-__device__ __forceinline__ void warp_flush(WarpSideAcc &w, uint32_t job, bool stats, IStatsAcc *acc,
-                                           IStatsAcc *local, bool useLocal, uint32_t firstJob) {
+// A warp's reduced statistics of a job: both sides' IStatsAcc as 26 words.
+constexpr int kAccWords = sizeof(IStatsAcc) / 8;
+static_assert(kAccWords == 13 && offsetof(IStatsAcc, v) == 24 && offsetof(IStatsAcc, lo) == 48 &&
+                  offsetof(IStatsAcc, hi) == 72 && offsetof(IStatsAcc, n) == 96,
+              "words of m, v, lo, hi, n");
+struct WarpWords {
+  IStatsAcc side[2];
+  uint32_t job;  // ~0: none
+  bool stats;
+};
+// Reduces a warp's running statistics into `out` and clears them.
+__device__ __forceinline__ void warp_words(WarpSideAcc &w, uint32_t job, bool stats, WarpWords &out) {
   const int lane = threadIdx.x & 31;
+  if (stats) {
 #pragma unroll
-  for (int sd = 0; sd < 2; ++sd) {
-    unsigned long long cnt = (unsigned long long)warp_sum64((long long)w.n[sd]);
-    if (cnt == 0) continue;
-    const uint32_t slot = 2 * job + uint32_t(sd);
-    if (stats) {
-      long long sm[3], sv[3], lo[3], hi[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        sm[d] = warp_sum64(w.m[sd][d]);
-        sv[d] = warp_sum64(w.v[sd][d]);
-        lo[d] = warp_min64(w.lo[sd][d]);
-        hi[d] = warp_max64(w.hi[sd][d]);
+    for (int d = 0; d < 3; ++d) {
+      const long long m = warp_sum64(w.m[d]), ml = warp_sum64(w.ml[d]);
+      const long long v = warp_sum64(w.v[d]), vl = warp_sum64(w.vl[d]);
+      long long lo[2], hi[2];
+      w.range[0][d].warp(lo[0], hi[0]);
+      w.range[1][d].warp(lo[1], hi[1]);
+      if (lane == 0) {
+        out.side[0].m[d] = ml;
+        out.side[0].v[d] = vl;
+        out.side[1].m[d] = m - ml;
+        out.side[1].v[d] = v - vl;
+        for (int sd = 0; sd < 2; ++sd) {
+          out.side[sd].lo[d] = lo[sd];
+          out.side[sd].hi[d] = hi[sd];
+        }
       }
-      if (lane == 0) acc_add(useLocal ? &local[slot - 2 * firstJob] : &acc[slot], sm, sv, lo, hi, cnt);
-    } else if (lane == 0) {
-      atomicAdd(&acc[slot].n, cnt);
     }
   }
+  if (lane == 0) {
+    out.side[0].n = w.nl;
+    out.side[1].n = w.n - w.nl;
+    out.job = job;
+    out.stats = stats;
+  }
   w.clear();
+  __syncwarp();
+}
+// Word k of the job's two accumulators takes the warps' words: atomics in
+// global memory, which are single operations there (64-bit ones in shared memory
+// are loops).  The warps [w, end) of `words` that hold w's job.
+__device__ __forceinline__ void add_words(const WarpWords *words, int w, int end, int k, IStatsAcc *acc) {
+  const uint32_t job = words[w].job;
+  const int side = k / kAccWords, f = k % kAccWords;
+  if (!words[w].stats && f != kAccWords - 1) return;
+  unsigned long long n = 0;
+  long long x = 0;
+  for (int o = w; o < end; ++o) {
+    const WarpWords &W = words[o];
+    if (W.job != job || W.side[side].n == 0) continue;
+    const long long y = reinterpret_cast<const long long *>(&W.side[side])[f];
+    if (n == 0) x = y;
+    else if (f >= 9 && f < 12) x = max(x, y);
+    else if (f >= 6 && f < 9) x = min(x, y);
+    else x += y;
+    n += W.side[side].n;
+  }
+  if (n == 0) return;
+  long long *to = reinterpret_cast<long long *>(&acc[2 * job + uint32_t(side)]) + f;
+  if (f >= 9 && f < 12) atomicMax(to, x);
+  else if (f >= 6 && f < 9) atomicMin(to, x);
+  else atomicAdd(reinterpret_cast<unsigned long long *>(to), (unsigned long long)x);
 }
 
 // Classifies the samples of every job at this level: side flag (1 = left),
@@ -190,107 +274,106 @@ __device__ __forceinline__ void warp_flush(WarpSideAcc &w, uint32_t job, bool st
 // (or ~0 when the sample already sits in a finished leaf).  Samples of a job
 // are contiguous, so a warp mostly meets one job: each lane keeps running
 // statistics of the warp's current job in registers, and the warp reduces
-// and adds them only when its job changes and at the end; a group of 32
-// samples that mixes jobs adds per sample.
-__global__ void __launch_bounds__(kKdThreads)
+// and adds them only when its job changes and, together with the other warps of
+// the block, at the end.  Samples past the fourth job of 32 add one by one.
+// Latency bound.  1.5M samples: 48 us with 64-bit shared-memory atomics (loops)
+// per warp, 64-bit conversions and the ranges in integers, 27 us so.
+__global__ void __launch_bounds__(kKdThreads, 3)
 kd_classify_kernel(const float4 *pos, const uint32_t *jobOf, uint32_t n, const KdJob *jobs, uint32_t *isLeft,
                    IStatsAcc *acc) {
-  __shared__ IStatsAcc local[2 * kKdLocal];
-  __shared__ uint32_t firstJob, lastJob;
+  __shared__ WarpWords words[kKdThreads / 32];
   const uint32_t tileBegin = blockIdx.x * kKdTile;
   if (tileBegin >= n) return;
   const uint32_t tileEnd = min(n, tileBegin + kKdTile);
-  if (threadIdx.x == 0) {
-    firstJob = ~0u;
-    lastJob = 0;
-  }
-  for (int s = threadIdx.x; s < 2 * kKdLocal; s += blockDim.x) {
-    IStatsAcc &a = local[s];
-    for (int d = 0; d < 3; ++d) { a.m[d] = 0; a.v[d] = 0; a.lo[d] = LLONG_MAX; a.hi[d] = LLONG_MIN; }
-    a.n = 0;
-  }
-  __syncthreads();
-  // jobs are sorted by segment and samples of a job are contiguous, so the
-  // tile's jobs form the range [min, max] of its job ids (~0: finished sample)
-  {
-    uint32_t f = ~0u, l = 0;
-    for (uint32_t i = tileBegin + threadIdx.x; i < tileEnd; i += blockDim.x) {
-      const uint32_t j = jobOf[i];
-      if (j != ~0u) {
-        f = min(f, j);
-        l = max(l, j);
-      }
-    }
-    if (f != ~0u) {
-      atomicMin(&firstJob, f);
-      atomicMax(&lastJob, l);
-    }
-  }
-  __syncthreads();
-  const bool useLocal = firstJob != ~0u && (lastJob - firstJob) < uint32_t(kKdLocal);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned full = 0xFFFFFFFFu;
   WarpSideAcc w;
   w.clear();
   uint32_t cur = ~0u;  // the warp's current job
   bool curStats = false;
-  for (uint32_t base = tileBegin; base < tileEnd; base += blockDim.x) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t jid = i < tileEnd ? jobOf[i] : ~0u;
-    KdJob j;
+  KdJob j;
+  uint32_t jAt = ~0u;  // the job in j
+  // two samples ahead
+  uint32_t i = tileBegin + threadIdx.x, jidA = ~0u, jidB = ~0u;
+  float4 pA = make_float4(0.0f, 0.0f, 0.0f, 0.0f), pB = pA;
+  if (i < tileEnd) {
+    jidA = jobOf[i];
+    pA = pos[i];
+  }
+  if (i + kKdThreads < tileEnd) {
+    jidB = jobOf[i + kKdThreads];
+    pB = pos[i + kKdThreads];
+  }
+#pragma unroll 1
+  for (uint32_t base = tileBegin; base < tileEnd; base += kKdThreads, i += kKdThreads) {
+    const uint32_t jid = jidA;
+    const float4 p = pA;
+    jidA = jidB;
+    pA = pB;
+    jidB = ~0u;
+    if (i + 2 * kKdThreads < tileEnd) {
+      jidB = jobOf[i + 2 * kKdThreads];
+      pB = pos[i + 2 * kKdThreads];
+    }
     uint32_t left = 0;
+    float t[3] = {0.0f, 0.0f, 0.0f};
     long long q[3] = {0, 0, 0}, qv[3] = {0, 0, 0};
     bool stats = false;
     if (jid != ~0u) {
-      j = jobs[jid];
-      const float4 p = pos[i];
+      if (jid != jAt) {
+        j = jobs[jid];
+        jAt = jid;
+      }
       const float coord = j.dim == 0 ? p.x : (j.dim == 1 ? p.y : p.z);
       left = coord < j.pos ? 1u : 0u;
       stats = j.needStats != 0;
-      if (stats) quantize(j, p, q, qv);
+      if (stats) quantize(j, p, t, q, qv);
     }
     if (i < tileEnd) isLeft[i] = left;
-    const unsigned act = __ballot_sync(full, jid != ~0u);
-    if (act == 0) continue;
-    const uint32_t j0 = __shfl_sync(full, jid, __ffs(act) - 1);
-    if (__all_sync(full, jid == ~0u || jid == j0)) {
+    unsigned rest = __ballot_sync(full, jid != ~0u);
+#pragma unroll 1
+    for (int g = 0; g < 4 && rest != 0; ++g) {
+      const int src = __ffs(rest) - 1;
+      const uint32_t j0 = __shfl_sync(full, jid, src);
       if (j0 != cur) {
-        if (cur != ~0u) warp_flush(w, cur, curStats, acc, local, useLocal, firstJob);
+        if (cur != ~0u) {
+          warp_words(w, cur, curStats, words[warp]);
+          if (lane < 2 * kAccWords) add_words(words, warp, warp + 1, lane, acc);
+          __syncwarp();
+        }
         cur = j0;
-        curStats = __shfl_sync(full, stats ? 1 : 0, __ffs(act) - 1) != 0;
+        curStats = __shfl_sync(full, stats ? 1 : 0, src) != 0;
       }
-      // both sides with selects (fixed register indices)
+      const bool on = jid == j0, onLeft = on && left != 0u;
+      const unsigned members = __ballot_sync(full, on);
+      w.n += __popc(members);
+      w.nl += __popc(__ballot_sync(full, onLeft));
+      rest &= ~members;
+      if (curStats) {
 #pragma unroll
-      for (int sd = 0; sd < 2; ++sd) {
-        const bool on = jid != ~0u && (left != 0u) == (sd == 0);
-        w.n[sd] += on ? 1ull : 0ull;
-        if (curStats) {
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            w.m[sd][d] += on ? q[d] : 0ll;
-            w.v[sd][d] += on ? qv[d] : 0ll;
-            w.lo[sd][d] = min(w.lo[sd][d], on ? q[d] : LLONG_MAX);
-            w.hi[sd][d] = max(w.hi[sd][d], on ? q[d] : LLONG_MIN);
-          }
+        for (int d = 0; d < 3; ++d) {
+          w.m[d] += on ? q[d] : 0ll;
+          w.v[d] += on ? qv[d] : 0ll;
+          w.ml[d] += onLeft ? q[d] : 0ll;
+          w.vl[d] += onLeft ? qv[d] : 0ll;
+          w.range[0][d].add(t[d], onLeft);
+          w.range[1][d].add(t[d], on && !onLeft);
         }
       }
-    } else if (jid != ~0u) {
-      const uint32_t side = left ? 0u : 1u;
-      if (stats) {
-        IStatsAcc *a = useLocal ? &local[2 * (jid - firstJob) + side] : &acc[2 * jid + side];
-        acc_add(a, q, qv, q, q, 1ull);
-      } else {
-        atomicAdd(&acc[2 * jid + side].n, 1ull);
-      }
+    }
+    if (rest >> lane & 1u) {
+      IStatsAcc *a = &acc[2 * jid + (left ? 0u : 1u)];
+      if (stats) acc_add(a, q, qv, q, q, 1ull);
+      else atomicAdd(&a->n, 1ull);
     }
   }
-  if (cur != ~0u) warp_flush(w, cur, curStats, acc, local, useLocal, firstJob);
+  warp_words(w, cur, curStats, words[warp]);
   __syncthreads();
-  if (useLocal) {
-    for (int s = threadIdx.x; s < 2 * kKdLocal; s += blockDim.x) {
-      const IStatsAcc &a = local[s];
-      if (a.n == 0) continue;
-      acc_add(&acc[2 * firstJob + s], a.m, a.v, a.lo, a.hi, a.n);
-    }
+  // the first warp of each job adds for all that hold it
+  if (cur != ~0u) {
+    for (int o = 0; o < warp; ++o)
+      if (words[o].job == cur) return;
+    if (lane < 2 * kAccWords) add_words(words, warp, kKdThreads / 32, lane, acc);
   }
 }
 
@@ -298,25 +381,43 @@ kd_classify_kernel(const float4 *pos, const uint32_t *jobOf, uint32_t n, const K
 // a leaf: KDTreeBuilder.h:94-115).
 __global__ void __launch_bounds__(kKdThreads)
 kd_root_stats_kernel(const float4 *pos, uint32_t n, KdJob job, IStatsAcc *acc) {
-  long long m[3] = {0, 0, 0}, v[3] = {0, 0, 0}, lo[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX},
-            hi[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
-  unsigned long long cnt = 0;
+  __shared__ WarpWords words[kKdThreads / 32];
+  long long m[3] = {0, 0, 0}, v[3] = {0, 0, 0}, lo[3], hi[3];
+  FloatRange range[3];
+  for (int d = 0; d < 3; ++d) range[d].clear();
+  uint32_t cnt = 0;
+#pragma unroll 4
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float t[3];
     long long q[3], qv[3];
-    quantize(job, pos[i], q, qv);
-    for (int d = 0; d < 3; ++d) { m[d] += q[d]; v[d] += qv[d]; lo[d] = min(lo[d], q[d]); hi[d] = max(hi[d], q[d]); }
+    quantize(job, pos[i], t, q, qv);
+    for (int d = 0; d < 3; ++d) {
+      m[d] += q[d];
+      v[d] += qv[d];
+      range[d].add(t[d], true);
+    }
     cnt++;
   }
-  for (int off = 16; off > 0; off >>= 1) {
-    for (int d = 0; d < 3; ++d) {
-      m[d] += __shfl_xor_sync(0xFFFFFFFFu, m[d], off);
-      v[d] += __shfl_xor_sync(0xFFFFFFFFu, v[d], off);
-      lo[d] = min(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], off));
-      hi[d] = max(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], off));
-    }
-    cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, off);
+  for (int d = 0; d < 3; ++d) {
+    m[d] = warp_sum64(m[d]);
+    v[d] = warp_sum64(v[d]);
+    range[d].warp(lo[d], hi[d]);
   }
-  if ((threadIdx.x & 31) == 0 && cnt > 0) acc_add(acc, m, v, lo, hi, cnt);
+  cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+  if ((threadIdx.x & 31) == 0) {
+    WarpWords &W = words[threadIdx.x >> 5];
+    for (int d = 0; d < 3; ++d) {
+      W.side[0].m[d] = m[d];
+      W.side[0].v[d] = v[d];
+      W.side[0].lo[d] = lo[d];
+      W.side[0].hi[d] = hi[d];
+    }
+    W.side[0].n = cnt;
+    W.job = 0;
+    W.stats = true;
+  }
+  __syncthreads();
+  if (threadIdx.x < kAccWords) add_words(words, 0, kKdThreads / 32, threadIdx.x, acc);
 }
 
 // One pass down an existing tree: the leaf every sample reaches, by the
@@ -395,21 +496,33 @@ __global__ void kd_job_of_kernel(const uint32_t *node, uint32_t n, const uint32_
 }
 
 // ------------------------------------------------------------------ gather + ordering
-// Gathers full samples into leaf order and builds the sort keys.  The key is
-// the weight's bits mapped to an order-preserving integer (-0 as +0), the
-// first field of SampleDataLess (SampleData.h:82-93).
+// Gathers full samples into leaf order.
 __global__ void gather_kernel(const float4 *posIdx, uint32_t n, const float4 *P, const float4 *D, const float *pdf,
-                              float4 *oP, float4 *oD, float *oPdf, uint32_t *key, uint32_t *val) {
+                              float4 *oP, float4 *oD, float *oPdf) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t src = __float_as_uint(posIdx[i].w);
-  float4 d = D[src];
   oP[i] = P[src];
-  oD[i] = d;
+  oD[i] = D[src];
   oPdf[i] = pdf[src];
-  float w = d.w == 0.0f ? 0.0f : d.w;
-  key[i] = ford(w);
-  val[i] = i;
+}
+// 64-bit sort keys of the samples in leaf order, beside the samples' indices:
+// the leaf's ordinal, then the weight's bits mapped to an order-preserving
+// integer (-0 as +0), the first field of SampleDataLess (SampleData.h:82-93).
+// blockIdx.x: leaf, blockIdx.y: its part.  Bound by the scattered reads: 1.5M
+// samples 15 us, the permutation below 34 us; with the full samples gathered
+// first and a block per leaf the three kernels took 35 + 31 + 29 us (56 for the
+// second with large leaves).
+__global__ void leaf_key_kernel(const float4 *posIdx, const uint32_t *leafBegin, const uint32_t *leafEnd,
+                                const float4 *D, unsigned long long *key64, uint32_t *val) {
+  const uint32_t leaf = blockIdx.x, end = leafEnd[leaf];
+  const unsigned long long hi = (unsigned long long)leaf << 32;
+  for (uint32_t i = leafBegin[leaf] + blockIdx.y * blockDim.x + threadIdx.x; i < end; i += gridDim.y * blockDim.x) {
+    const uint32_t src = __float_as_uint(posIdx[i].w);
+    const float w = D[src].w;
+    key64[i] = hi | ford(w == 0.0f ? 0.0f : w);
+    val[i] = src;
+  }
 }
 __device__ __forceinline__ bool sample_less(float4 pa, float4 da, float fa, float4 pb, float4 db, float fb) {
   if (da.w != db.w) return da.w < db.w;   // weight
@@ -471,20 +584,20 @@ __global__ void copy_region_kernel(RegionDir *regions, const uint32_t *dst, cons
 
 // 8 nearest region means per region (KNN.h:212-266); nanoflann's squared
 // distance ((dx*dx + dy*dy) + dz*dz), ties by region index.
-__global__ void knn_kernel(const float4 *means, uint32_t R, Neighbours *out) {
-  uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  float4 q = means[r];
+__device__ __forceinline__ float mean_distance(float4 q, float4 p) {
+  float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+  float d = 0.0f;
+  d += dx * dx;
+  d += dy * dy;
+  d += dz * dz;
+  return d;
+}
+// by one thread, any distances
+__device__ __noinline__ int nearest_in_order(const float4 *means, uint32_t R, float4 q, uint32_t bi[8]) {
   float bd[8];
-  uint32_t bi[8];
   int cnt = 0;
   for (uint32_t j = 0; j < R; ++j) {
-    float4 p = means[j];
-    float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-    float d = 0.0f;
-    d += dx * dx;
-    d += dy * dy;
-    d += dz * dz;
+    const float d = mean_distance(q, means[j]);
     if (cnt < 8 || d < bd[cnt - 1]) {
       int k = cnt < 8 ? cnt : 7;
       while (k > 0 && bd[k - 1] > d) {
@@ -496,19 +609,76 @@ __global__ void knn_kernel(const float4 *means, uint32_t R, Neighbours *out) {
       if (cnt < 8) cnt++;
     }
   }
-  Neighbours nb;
-  nb.size = uint32_t(cnt);
-  for (int i = 0; i < 8; ++i) {
-    if (i < cnt) {
-      nb.ids[i] = bi[i];
-      float4 p = means[bi[i]];
-      nb.px[i] = p.x; nb.py[i] = p.y; nb.pz[i] = p.z;
-    } else {
-      nb.ids[i] = ~0u;
-      nb.px[i] = nb.py[i] = nb.pz[i] = 0.0f;
+  return cnt;
+}
+// A warp per region: each lane keeps the nearest 8 of every 32nd mean, then the
+// warp takes the least of the lanes' heads 8 times.  With distances that have no
+// order (infinite or NaN means) lane 0 goes through the means alone.  128
+// regions: 68 us with a thread per region, 5 us so.
+__global__ void __launch_bounds__(128) knn_kernel(const float4 *means, uint32_t R, Neighbours *out) {
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xFFFFFFFFu;
+  if (r >= R) return;
+  const float4 q = means[r];
+  float bd[8];
+  uint32_t bi[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    bd[k] = INFINITY;
+    bi[k] = ~0u;
+  }
+  bool odd = false;
+  for (uint32_t j = lane; j < R; j += 32) {
+    const float d = mean_distance(q, means[j]);
+    odd = odd || !(d <= FLT_MAX);
+    if (!(d < bd[7])) continue;
+#pragma unroll
+    for (int k = 7; k > 0; --k) {
+      const bool down = d < bd[k - 1], here = d < bd[k];
+      bi[k] = down ? bi[k - 1] : (here ? j : bi[k]);
+      bd[k] = down ? bd[k - 1] : (here ? d : bd[k]);
+    }
+    if (d < bd[0]) {
+      bd[0] = d;
+      bi[0] = j;
     }
   }
-  out[r] = nb;
+  uint32_t mine = ~0u;  // lane k < 8: neighbour k
+  int cnt = int(min(R, 8u));
+  if (__any_sync(full, odd)) {
+    uint32_t in[8];
+    for (int k = 0; k < 8; ++k) in[k] = ~0u;
+    if (lane == 0) cnt = nearest_in_order(means, R, q, in);
+    cnt = __shfl_sync(full, cnt, 0);
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t id = __shfl_sync(full, in[k], 0);
+      if (lane == k) mine = id;
+    }
+  } else {
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t d = __reduce_min_sync(full, __float_as_uint(bd[0]));  // not negative
+      const uint32_t id = __reduce_min_sync(full, __float_as_uint(bd[0]) == d ? bi[0] : ~0u);
+      if (lane == k) mine = id;
+      if (bi[0] == id && id != ~0u) {
+#pragma unroll
+        for (int m = 0; m < 7; ++m) {
+          bd[m] = bd[m + 1];
+          bi[m] = bi[m + 1];
+        }
+        bd[7] = INFINITY;
+        bi[7] = ~0u;
+      }
+    }
+  }
+  if (lane == 0) out[r].size = uint32_t(cnt);
+  if (lane < 8) {
+    const float4 p = lane < cnt ? means[mine] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    out[r].ids[lane] = lane < cnt ? mine : ~0u;
+    out[r].px[lane] = p.x;
+    out[r].py[lane] = p.y;
+    out[r].pz[lane] = p.z;
+  }
 }
 
 // ------------------------------------------------------------------ launchers
@@ -576,8 +746,8 @@ cudaError_t scene_bounds(const float4 *P, uint64_t n, uint32_t *d6, cudaStream_t
   uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
   cudaError_t e = cudaMemcpyAsync(d6, init, sizeof(init), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess || n == 0) return e;
-  unsigned b = blocks_for(n, 256);
-  if (b > 4096) b = 4096;
+  unsigned b = blocks_for(n, 1024);
+  if (b > 1024) b = 1024;
   count_launch();
   bounds_kernel<<<b, 256, 0, s>>>(P, n, d6);
   return cudaGetLastError();
@@ -614,7 +784,7 @@ cudaError_t init_acc(IStatsAcc *acc, uint32_t count, cudaStream_t s) {
 cudaError_t kd_root_stats(const float4 *pos, uint32_t n, const KdJob &job, IStatsAcc *acc, cudaStream_t s) {
   unsigned b = blocks_for(n, kKdThreads * 8);
   if (b < 1) b = 1;
-  if (b > 2048) b = 2048;
+  if (b > 608) b = 608;
   count_launch();
   kd_root_stats_kernel<<<b, kKdThreads, 0, s>>>(pos, n, job, acc);
   return cudaGetLastError();
@@ -676,35 +846,26 @@ cudaError_t kd_classify(const float4 *pos, const uint32_t *jobOf, uint32_t n, co
   return cudaGetLastError();
 }
 
-// 64-bit sort keys: the leaf's ordinal above the 32-bit weight key.
-__global__ void leaf_key_kernel(const uint32_t *leafBegin, const uint32_t *leafEnd, uint32_t numLeaves,
-                                const uint32_t *key, unsigned long long *key64) {
-  const uint32_t leaf = blockIdx.x;
-  if (leaf >= numLeaves) return;
-  const unsigned long long hi = (unsigned long long)leaf << 32;
-  for (uint32_t i = leafBegin[leaf] + threadIdx.x; i < leafEnd[leaf]; i += blockDim.x) key64[i] = hi | key[i];
-}
-
 cudaError_t gather_and_order(const float4 *posIdx, uint32_t n, const float4 *P, const float4 *D, const float *pdf,
                              const uint32_t *leafBegin, const uint32_t *leafCount, uint32_t numLeaves, bool sorted,
-                             float4 *tmpP, float4 *tmpD, float *tmpPdf, uint32_t *keys, uint32_t *vals,
-                             unsigned long long *keys64, float4 *oP, float4 *oD, float *oPdf, Scratch &scratch,
+                             uint32_t *vals, unsigned long long *keys64, float4 *oP, float4 *oD, float *oPdf, Scratch &scratch,
                              cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (!sorted) {
     count_launch();
-    gather_kernel<<<blocks_for(n, 256), 256, 0, s>>>(posIdx, n, P, D, pdf, oP, oD, oPdf, keys, vals);
+    gather_kernel<<<blocks_for(n, 256), 256, 0, s>>>(posIdx, n, P, D, pdf, oP, oD, oPdf);
     return cudaGetLastError();
   }
-  count_launch();
-  gather_kernel<<<blocks_for(n, 256), 256, 0, s>>>(posIdx, n, P, D, pdf, tmpP, tmpD, tmpPdf, keys, vals);
   // stable order by (leaf, weight key): one LSD radix sort over the bits in
   // use (the leaves' sample ranges are disjoint and cover [0, n))
   uint32_t *valsOut = vals + n;
   unsigned long long *keys64Out = keys64 + n;
   const uint32_t *ends = leafBegin + numLeaves;  // caller stores ends after begins
+  // blocks for about eight samples per thread whatever the number of leaves
+  uint32_t parts = n / 2048 / numLeaves;
+  parts = parts < 1 ? 1 : (parts > 4096 ? 4096 : parts);
   count_launch();
-  leaf_key_kernel<<<numLeaves, 256, 0, s>>>(leafBegin, ends, numLeaves, keys, keys64);
+  leaf_key_kernel<<<dim3(numLeaves, parts), 256, 0, s>>>(posIdx, leafBegin, ends, D, keys64, vals);
   int leafBits = 1;
   while (leafBits < 32 && (1u << leafBits) < numLeaves) ++leafBits;
   size_t tempBytes = 0;
@@ -714,7 +875,7 @@ cudaError_t gather_and_order(const float4 *posIdx, uint32_t n, const float4 *P, 
   cub::DeviceRadixSort::SortPairs(scratch.ptr, tempBytes, keys64, keys64Out, vals, valsOut, int(n), 0, 32 + leafBits,
                                   s);
   count_launch();
-  permute_kernel<<<blocks_for(n, 256), 256, 0, s>>>(valsOut, n, tmpP, tmpD, tmpPdf, oP, oD, oPdf);
+  permute_kernel<<<blocks_for(n, 256), 256, 0, s>>>(valsOut, n, P, D, pdf, oP, oD, oPdf);
   count_launch();
   fix_ties_kernel<<<blocks_for(n, 256), 256, 0, s>>>(keys64Out, n, oP, oD, oPdf);
   (void)leafCount;
@@ -731,7 +892,7 @@ cudaError_t copy_regions(RegionDir *regions, const uint32_t *dst, const uint32_t
 cudaError_t build_knn(const float4 *means, uint32_t R, Neighbours *out, cudaStream_t s) {
   if (R == 0) return cudaSuccess;
   count_launch();
-  knn_kernel<<<blocks_for(R, 128), 128, 0, s>>>(means, R, out);
+  knn_kernel<<<blocks_for(uint64_t(R) * 32, 128), 128, 0, s>>>(means, R, out);
   return cudaGetLastError();
 }
 
