@@ -75,6 +75,16 @@ struct Unassigned {
   float sw, dx, dy, dz;
 };
 
+constexpr int kMergePairs = 256;  // merge costs computed at once
+struct MergeParts {               // see merge_costs
+  float mx[kMergePairs], my[kMergePairs], mz[kMergePairs], kappa[kMergePairs], norm[kMergePairs], e2k[kMergePairs];
+  // products of pairs, then of the components with themselves
+  float px[kMergePairs + kMaxK], py[kMergePairs + kMaxK], pz[kMergePairs + kMaxK], pkappa[kMergePairs + kMaxK],
+      pnorm[kMergePairs + kMaxK], pscale[kMergePairs + kMaxK];
+  float part[3][kMergePairs];
+  uint8_t i[kMergePairs], j[kMergePairs];
+};
+
 struct EmShared {
   VMMState vmm;
   SuffState suff;     // training statistics ("previous" statistics of EM)
@@ -90,6 +100,7 @@ struct EmShared {
   float xch[2][kMaxK];
   uint32_t rcpTab[2048];
   float cost[kMaxK][kMaxK];  // merge cost of components i < j (cost[i][j])
+  MergeParts merge;
   float ll;
   Unassigned un;
   int mask[kMaxK];
@@ -591,13 +602,15 @@ __device__ float integrated_division(V3 m0, float k0, float n0, V3 m1, float k1,
   scale *= lib_expf((k0 * (c0 - 1.0f) + k1 * (c1 - 1.0f)) + (2.0f * k1));
   return scale;
 }
-__device__ float merge_cost(const VMMState &v, int i0, int i1) {  // Merger.h:92-177
-  float w0 = v.w[i0], k0 = v.kappa[i0], mc0 = v.mc[i0], n0 = v.norm[i0];
-  float w1 = v.w[i1], k1 = v.kappa[i1], mc1 = v.mc[i1], n1 = v.norm[i1];
-  V3 m0 = mk(v.mx[i0], v.my[i0], v.mz[i0]), m1 = mk(v.mx[i1], v.my[i1], v.mz[i1]);
-  if (i0 == i1) { w0 /= 2.0f; w1 /= 2.0f; }
-  float w = w0 + w1, kappa = 0.0f, nrm = kInv4Pi, e2k = 1.0f;
-  V3 m = m0 * (w0 * mc0) + m1 * (w1 * mc1);
+// The merged lobe of components i0 and i1 (Merger.h:92-133).
+__device__ void merged_lobe(const VMMState &v, int i0, int i1, V3 &m, float &kappa, float &nrm, float &e2k) {
+  const float w0 = v.w[i0], mc0 = v.mc[i0], w1 = v.w[i1], mc1 = v.mc[i1];
+  const V3 m0 = mk(v.mx[i0], v.my[i0], v.mz[i0]), m1 = mk(v.mx[i1], v.my[i1], v.mz[i1]);
+  const float w = w0 + w1;
+  kappa = 0.0f;
+  nrm = kInv4Pi;
+  e2k = 1.0f;
+  m = m0 * (w0 * mc0) + m1 * (w1 * mc1);
   m = m / w;
   float mc = m.x * m.x + m.y * m.y + m.z * m.z;
   if (mc > 0.f) {
@@ -610,19 +623,66 @@ __device__ float merge_cost(const VMMState &v, int i0, int i1) {  // Merger.h:92
   } else {
     m = m0;
   }
-  V3 nm = mk(-m.x, -m.y, -m.z);
-  V3 m00, m11, m01;
-  float k00, k11, k01, n00, n11, n01;
-  float s00 = product_scale(m0, k0, n0, m0, k0, n0, m00, k00, n00);
-  float s11 = product_scale(m1, k1, n1, m1, k1, n1, m11, k11, n11);
-  float s01 = product_scale(m0, k0, n0, m1, k1, n1, m01, k01, n01);
-  float w00 = w0 * w0, w11 = w1 * w1, w01 = w0 * w1;
-  float chi = 0.0f;
-  chi += (w00 / w) * (s00 * integrated_division(m00, k00, n00, nm, kappa, nrm, e2k));
-  chi += (w11 / w) * (s11 * integrated_division(m11, k11, n11, nm, kappa, nrm, e2k));
-  chi += 2.0f * (w01 / w) * (s01 * integrated_division(m01, k01, n01, nm, kappa, nrm, e2k));
-  chi -= w;
-  return chi;
+}
+// Merge costs (Merger.h:92-177) of the first nP pairs of M.i, M.j (255: none)
+// into S.cost, by the whole block.  A cost is the merged lobe, the products of
+// the two components with themselves and with each other, and the integral of
+// each product over the merged lobe; computed by one thread it was one chain of
+// 20,000 cycles, twenty times per region.  Here a thread takes one part of one
+// cost: merged lobes and products first (warps of either), then the three
+// integrals of each pair, then their sum.  A component's product with itself
+// serves all its pairs: it is made anew for the components with `selves` set.
+__device__ void merge_costs(EmShared &S, int nP, uint32_t selves) {
+  MergeParts &M = S.merge;
+  const VMMState &v = S.vmm;
+  const int nPad = (nP + 31) & ~31;
+  for (int x = threadIdx.x; x < 2 * nPad + kMaxK; x += kEmThreads) {
+    if (x < nPad) {
+      if (x >= nP || M.i[x] == 255) continue;
+      V3 m;
+      merged_lobe(v, M.i[x], M.j[x], m, M.kappa[x], M.norm[x], M.e2k[x]);
+      M.mx[x] = m.x;
+      M.my[x] = m.y;
+      M.mz[x] = m.z;
+      continue;
+    }
+    const bool self = x >= 2 * nPad;
+    const int q = x - nPad, c = x - 2 * nPad;
+    if (self ? !(selves >> c & 1u) : q >= nP || M.i[q] == 255) continue;
+    const int i = self ? c : M.i[q], j = self ? c : M.j[q];
+    V3 pm;
+    float pk, pn;
+    const float scale = product_scale(mk(v.mx[i], v.my[i], v.mz[i]), v.kappa[i], v.norm[i],
+                                      mk(v.mx[j], v.my[j], v.mz[j]), v.kappa[j], v.norm[j], pm, pk, pn);
+    const int o = self ? kMergePairs + c : q;
+    M.px[o] = pm.x;
+    M.py[o] = pm.y;
+    M.pz[o] = pm.z;
+    M.pkappa[o] = pk;
+    M.pnorm[o] = pn;
+    M.pscale[o] = scale;
+  }
+  __syncthreads();
+  for (int x = threadIdx.x; x < 3 * nPad; x += kEmThreads) {
+    const int t = x / nPad, q = x - t * nPad;
+    if (q >= nP || M.i[q] == 255) continue;
+    const int o = t == 0 ? kMergePairs + M.i[q] : (t == 1 ? kMergePairs + M.j[q] : q);
+    M.part[t][q] = M.pscale[o] * integrated_division(mk(M.px[o], M.py[o], M.pz[o]), M.pkappa[o], M.pnorm[o],
+                                                     mk(-M.mx[q], -M.my[q], -M.mz[q]), M.kappa[q], M.norm[q], M.e2k[q]);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < nP; q += kEmThreads) {
+    const int i = M.i[q], j = M.j[q];
+    if (i == 255) continue;
+    const float w0 = v.w[i], w1 = v.w[j], w = w0 + w1;
+    const float w00 = w0 * w0, w11 = w1 * w1, w01 = w0 * w1;
+    float chi = 0.0f;
+    chi += (w00 / w) * M.part[0][q];
+    chi += (w11 / w) * M.part[1][q];
+    chi += 2.0f * (w01 / w) * M.part[2][q];
+    chi -= w;
+    S.cost[i][j] = chi;
+  }
 }
 // ComponentSplitStatistics::mergeComponentStats, zero-mean form (Splitter.h:994-1100)
 __device__ void split_merge_stats(SplitState &s, int I, int J, float wI, V3 muI, float wJ, V3 muJ, float wK, V3 muK) {
@@ -2078,8 +2138,10 @@ __device__ void sort_candidates(EmShared &S, const SplitState &sp) {
 // the first minimum in (i, j) scan order below the threshold, as the smallest
 // (cost, i, j) over the block's threads.  A region's merging was bound by the
 // costs' double-precision functions and their table searches and by one
-// thread's scan of the pairs: 1.3 M cycles per region with 23 to 30 lobes, now
-// 0.3 M (fourth frame of 2,097,152 samples, whose EM launch 4.3 -> 3.1 ms).
+// thread's scan of the pairs: 1.3 M cycles per region with 23 to 30 lobes, 0.3 M
+// without those, 0.19 M with the parts of a cost spread over threads (fourth
+// frame of 2,097,152 samples, whose EM launch took 4.3, 3.1 and 2.0 ms with the
+// other steps of the time).
 __device__ int perform_merging(EmShared &S, const FieldConfig &cfg) {
   const int tid = threadIdx.x;
   __shared__ int mergeAgain, total, lastI, lastJ;
@@ -2090,12 +2152,18 @@ __device__ int perform_merging(EmShared &S, const FieldConfig &cfg) {
     const int K = int(S.vmm.K);
     if (lastI < 0) {  // every pair
       const int pairs = K * (K - 1) / 2;
-      for (int p = tid; p < pairs; p += kEmThreads) {
-        // p -> (i, j), i < j
-        int i = 0, rem = p;
-        while (rem >= K - 1 - i) { rem -= K - 1 - i; ++i; }
-        const int j = i + 1 + rem;
-        S.cost[i][j] = merge_cost(S.vmm, i, j);
+      for (int first = 0; first < pairs; first += kMergePairs) {
+        const int nP = min(pairs - first, kMergePairs);
+        for (int q = tid; q < nP; q += kEmThreads) {
+          // the pair's (i, j), i < j
+          int i = 0, rem = first + q;
+          while (rem >= K - 1 - i) { rem -= K - 1 - i; ++i; }
+          S.merge.i[q] = uint8_t(i);
+          S.merge.j[q] = uint8_t(i + 1 + rem);
+        }
+        __syncthreads();
+        merge_costs(S, nP, first == 0 ? 0xFFFFFFFFu >> (kMaxK - K) : 0u);
+        __syncthreads();
       }
     } else {
       // after merging lastJ into lastI (and moving the last component into
@@ -2105,12 +2173,14 @@ __device__ int perform_merging(EmShared &S, const FieldConfig &cfg) {
       const int moved = lastJ < K ? 1 : 0;  // lastJ was not the last slot
       for (int t = tid; t < (1 + moved) * K; t += kEmThreads) {
         const int a = t < K ? lastI : lastJ, b = t < K ? t : t - K;
-        if (b == a || (a == lastJ && b == lastI)) continue;  // (lastI, lastJ) is in the first row
-        const int i = a < b ? a : b, j = a < b ? b : a;
-        S.cost[i][j] = merge_cost(S.vmm, i, j);
+        const bool none = b == a || (a == lastJ && b == lastI);  // (lastI, lastJ) is in the first row
+        S.merge.i[t] = none ? uint8_t(255) : uint8_t(min(a, b));
+        S.merge.j[t] = uint8_t(max(a, b));
       }
+      __syncthreads();
+      merge_costs(S, (1 + moved) * K, 1u << lastI | (moved ? 1u << lastJ : 0u));
+      __syncthreads();
     }
-    __syncthreads();
     // the reference's row-major double loop (Merger.h:67-90) keeps the first of equal
     // costs; both zeros are equal
     unsigned long long best = ~0ull;
@@ -2130,23 +2200,24 @@ __device__ int perform_merging(EmShared &S, const FieldConfig &cfg) {
     }
     if ((tid & 31) == 0) warpBest[tid >> 5] = best;
     __syncthreads();
-    if (tid == 0) {
+    if (tid == 0 || tid == 32) {
+      best = warpBest[0];
       for (int w = 1; w < kEmThreads / 32; ++w) best = warpBest[w] < best ? warpBest[w] : best;
       const bool found = best != ~0ull;
       const int ci = int(uint32_t(best)) / kMaxK, cj = int(uint32_t(best)) % kMaxK;
-      if (found) {
+      if (found && tid == 32) suff_merge(S.suff, ci, cj);
+      if (found && tid == 0) {
         VMMState &v = S.vmm;
         V3 muI = mk(v.mx[ci], v.my[ci], v.mz[ci]), muJ = mk(v.mx[cj], v.my[cj], v.mz[cj]);
         float wI = v.w[ci], wJ = v.w[cj];
         vmm_merge(v, ci, cj);
         V3 muK = mk(v.mx[ci], v.my[ci], v.mz[ci]);
         split_merge_stats(S.split, ci, cj, wI, muI, wJ, muJ, v.w[ci], muK);
-        suff_merge(S.suff, ci, cj);
         total++;
         lastI = ci;
         lastJ = cj;
       }
-      mergeAgain = (found && S.vmm.K > cfg.laneWidth) ? 1 : 0;
+      if (tid == 0) mergeAgain = (found && S.vmm.K > cfg.laneWidth) ? 1 : 0;
     }
     __syncthreads();
   }
