@@ -181,6 +181,26 @@ PGL_HD float dqt_turn(float phi) {
   return float(double(phi) / (2.0 * kPiD) + 0.5);
 #endif
 }
+// phi of a point's y, float((y - 0.5) 2 pi) with the difference and products in
+// double; on the device in double-float arithmetic where its rounding test decides.
+PGL_HD bool dqt_phi_df(float y, float *out) {
+  const DFloat v = df_two_sum(y, -0.5f);  // exact
+  const float p = v.h * 0x1.921fb6p+2f;
+  float e = fmaf_(v.h, 0x1.921fb6p+2f, -p);
+  e = fmaf_(v.l, 0x1.921fb6p+2f, fmaf_(v.h, -0x1.777a5cp-23f, e));
+  return df_round_checked(df_fast_two_sum(p, e), out);
+}
+#ifdef __CUDACC__
+static __device__ __noinline__ float dqt_phi_fp64(float y) { return float((double(y) - 0.5) * 2.0 * kPiD); }
+#endif
+PGL_HD float dqt_phi(float y) {
+#ifdef __CUDA_ARCH__
+  float r;
+  return y >= 0.0f && y <= 1.0f && fabsf(y - 0.5f) >= 1e-7f && dqt_phi_df(y, &r) ? r : dqt_phi_fp64(y);
+#else
+  return float((double(y) - 0.5) * 2.0 * kPiD);
+#endif
+}
 // SphereToSquareCylindrical (SphereToSquare.h:34-61): x = (cos theta + 1) / 2,
 // y = phi / 2pi + 1/2, phi = atan2(d.y, d.x), the division in double.
 PGL_HD void dqt_dir_to_point(float dx, float dy, float dz, float &px, float &py) {

@@ -63,6 +63,7 @@ static LibmTables load_libm_tables() {
   LibmTables t{};
   t.expMargin = libm_margin(v.data(), n[0], [](double x) { return std::exp(x); });
   t.cosMargin = libm_margin(v.data() + n[0], n[1], [](double x) { return std::cos(x); });
+  t.sinMargin = libm_margin(v.data() + n[0] + n[1], n[2], [](double x) { return std::sin(x); });
   if (n[0] > 0) {
     // about one expf entry per bucket of the float order
     const uint32_t first = float_key(v[0].x), span = float_key(v[n[0] - 1].x) - first;

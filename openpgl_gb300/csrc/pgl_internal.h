@@ -72,7 +72,7 @@ struct KDNode {  // 8 bytes, as KDTree.h:21-170: top 2 bits dim (3 = leaf), low 
   uint32_t bits;
 };
 
-struct Neighbours {  // RegionNeighbours<8> (KNN.h:116-149)
+struct alignas(16) Neighbours {  // RegionNeighbours<8> (KNN.h:116-149); aligned for 128-bit loads
   uint32_t ids[8];
   float px[8], py[8], pz[8];
   uint32_t size;

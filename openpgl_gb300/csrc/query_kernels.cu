@@ -69,21 +69,39 @@ __device__ uint32_t choose_region_1(const FieldView &f, uint32_t leaf, float p0,
   uint32_t sel = uint32_t(s1d * float(size));
   s1d = (s1d - float(sel) / float(size)) * float(size);
   sel = min(sel, size - 1);
-  uint32_t key[8];
+  // 128-bit loads: 32 threads read 32 lines with each one
+  uint32_t key[8], ids[8];
+  const uint4 *pid = reinterpret_cast<const uint4 *>(nb.ids);
+  const float4 *px = reinterpret_cast<const float4 *>(nb.px), *py = reinterpret_cast<const float4 *>(nb.py),
+               *pz = reinterpret_cast<const float4 *>(nb.pz);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    V3 d = mk(nb.px[j] - p0, nb.py[j] - p1, nb.pz[j] - p2);
-    float dd = dot(d, d);
-    key[j] = (f2u(dd) & ~7u) | uint32_t(j);
-    if (nb.ids[j] == ~0u) key[j] = f2u(INFINITY);
+  for (int h = 0; h < 2; ++h) {
+    const uint4 id = pid[h];
+    const float4 x = px[h], y = py[h], z = pz[h];
+    const uint32_t idv[4] = {id.x, id.y, id.z, id.w};
+    const float xv[4] = {x.x, x.y, x.z, x.w}, yv[4] = {y.x, y.y, y.z, y.w}, zv[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      V3 d = mk(xv[j] - p0, yv[j] - p1, zv[j] - p2);
+      float dd = dot(d, d);
+      ids[4 * h + j] = idv[j];
+      key[4 * h + j] = (f2u(dd) & ~7u) | uint32_t(4 * h + j);
+      if (idv[j] == ~0u) key[4 * h + j] = f2u(INFINITY);
+    }
   }
+  uint32_t chosen = ids[0];
+  bool found = false;
+#pragma unroll
   for (int j = 0; j < 8; ++j) {
     uint32_t rank = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) rank += (u2f(key[k]) < u2f(key[j])) ? 1u : 0u;
-    if (rank == sel && key[j] != f2u(INFINITY)) return nb.ids[key[j] & 7u];
+    if (!found && rank == sel && key[j] != f2u(INFINITY)) {
+      found = true;
+      chosen = ids[j];  // a finite key's low bits are its slot
+    }
   }
-  return nb.ids[key[0] & 7u];
+  return chosen;
 }
 
 // vfloat8 horizontal sum of lane values over the mixture: per group lane j
@@ -265,8 +283,9 @@ __device__ V3 dqt_point_to_dir(float px, float py) {
   py = dqt_clamp(py, 0.f, 1.f);
   const float cosTheta = 2.0f * px - 1.0f;
   const float sinTheta = sqrtf(1.0f - cosTheta * cosTheta);
-  const float phi = float((double(py) - 0.5) * 2.0 * kPiD);
-  return mk(dqt_clamp(sinTheta * lib_cosf_any(phi), -1.f, 1.f), dqt_clamp(sinTheta * lib_sinf(phi), -1.f, 1.f),
+  float sinPhi, cosPhi;
+  lib_sincosf_any(dqt_phi(py), &sinPhi, &cosPhi);
+  return mk(dqt_clamp(sinTheta * cosPhi, -1.f, 1.f), dqt_clamp(sinTheta * sinPhi, -1.f, 1.f),
             dqt_clamp(cosTheta, -1.f, 1.f));
 }
 // samplePdf (DQT.h:62-72, :115-153): a stochastic descent that picks the
@@ -275,33 +294,31 @@ __device__ V3 dqt_point_to_dir(float px, float py) {
 // area) / 4 pi
 __device__ float dqt_sample_pdf(const DqtNode *N, float ux, float uy, V3 &dir) {
   float span = 1.0f, x = 0.0f, y = 0.0f;
+  // one division either way
   auto rescale = [](float t, float &u) {
-    if (u < t) {
-      u /= t;
-      return true;
-    }
-    u -= t;
-    u /= 1.0f - t;
-    return false;
+    const bool first = u < t;
+    u = (first ? u : u - t) / (first ? t : 1.0f - t);
+    return first;
   };
-  uint32_t idx = 0;
-  while (N[idx].child > 0) {
+  // a node's four children are one load each, and the chosen one's own child comes with it
+  const auto node = [&](uint32_t i) {
+    const uint2 v = *reinterpret_cast<const uint2 *>(&N[i]);
+    return DqtNode{v.x, u2f(v.y)};
+  };
+  const DqtNode root = node(0);
+  DqtNode at = root;
+  while (at.child > 0) {
     span /= 2.0f;
-    uint32_t off = 0;
-    const DqtNode *c = &N[N[idx].child];
-    const float wl = c[0].weight + c[2].weight, wr = c[1].weight + c[3].weight;
-    if (!rescale(wl / (wl + wr), ux)) {
-      off += 1;
-      x += span;
-    }
-    const float wt = c[off].weight, wb = c[off + 2].weight;
-    if (!rescale(wt / (wt + wb), uy)) {
-      off += 2;
-      y += span;
-    }
-    idx = N[idx].child + off;
+    const DqtNode c0 = node(at.child), c1 = node(at.child + 1), c2 = node(at.child + 2), c3 = node(at.child + 3);
+    const float wl = c0.weight + c2.weight, wr = c1.weight + c3.weight;
+    const bool left = rescale(wl / (wl + wr), ux);
+    if (!left) x += span;
+    const DqtNode t = left ? c0 : c1, b = left ? c2 : c3;
+    const bool top = rescale(t.weight / (t.weight + b.weight), uy);
+    if (!top) y += span;
+    at = top ? t : b;
   }
-  float pdf = N[idx].weight / (N[0].weight * span * span);
+  float pdf = at.weight / (root.weight * span * span);
   const float px = x + ux * span, py = y + uy * span;
   pdf /= kDqtJacobian;
   dir = dqt_point_to_dir(px, py);
@@ -732,8 +749,12 @@ query_s4_g_kernel(QueryParams P, const QueryInS4 *in, QueryOutS4 *out, uint32_t 
 
 
 // Batched guided queries on a quadtree field: a thread per query (a
-// quadtree's descent has no lobes to spread over a warp).
-__global__ void query_dqt_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+// quadtree's descent has no lobes to spread over a warp).  Latency bound, so as
+// many threads as fit.  1,048,576 queries: 206 us with the angle, its sine and the
+// direction's turn in double, the neighbours in 33 loads and two loads one after
+// the other per level, 160 us without those, 135 us at 32 registers; vertices of
+// four samples 643, 461 and (at 40) 404 us.
+__global__ void __launch_bounds__(256, 8) query_dqt_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const QueryIn q = in[i];

@@ -1,10 +1,11 @@
-// two_pi_times and div3 (pgl_math.cuh) against what they stand for; each
+// two_pi_times, div3, lib_sincosf_any (pgl_math.cuh) and dqt_phi (dqt.cuh) against
+// what they stand for (the tables of the C library's exceptions empty); each
 // returns the number of differences, or -1.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
-#include "pgl_math.cuh"
+#include "dqt.cuh"
 
 // every float of [0, 2.5) against the double product rounded once
 __global__ void two_pi_kernel(unsigned *bad) {
@@ -13,6 +14,27 @@ __global__ void two_pi_kernel(unsigned *bad) {
     if (__float_as_uint(pgl::two_pi_times(u)) != __float_as_uint(float(2.0 * 3.14159265358979323846 * double(u))))
       atomicAdd(bad, 1u);
   }
+}
+// every float of [0, 1.5) as a point's y; every float of (-8.5, 8.5) as an angle
+__global__ void phi_kernel(unsigned *bad) {
+  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < 0x3fc00000u; b += gridDim.x * blockDim.x) {
+    const float y = __uint_as_float(b);
+    if (__float_as_uint(pgl::dqt_phi(y)) !=
+        __float_as_uint(float((double(y) - 0.5) * 2.0 * 3.14159265358979323846)))
+      atomicAdd(bad, 1u);
+  }
+}
+__global__ void sincos_kernel(unsigned *bad) {
+  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < 0x41080000u; b += gridDim.x * blockDim.x)
+    for (int sign = 0; sign < 2; ++sign) {
+      const float x = sign ? -__uint_as_float(b) : __uint_as_float(b);
+      float s, c;
+      pgl::lib_sincosf_any(x, &s, &c);
+      float want = float(sin(double(fabsf(x))));
+      want = x < 0.0f ? -want : want;
+      if (__float_as_uint(s) != __float_as_uint(want) || __float_as_uint(c) != __float_as_uint(float(cos(double(x)))))
+        atomicAdd(bad, 1u);
+    }
 }
 __device__ uint32_t hash(uint32_t x) {
   x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu;
@@ -54,6 +76,20 @@ extern "C" int two_pi_check() {
   if (cudaMalloc(&d, sizeof(unsigned)) != cudaSuccess) return -1;
   cudaMemset(d, 0, sizeof(unsigned));
   two_pi_kernel<<<1216, 256>>>(d);
+  return count(cudaGetLastError(), d);
+}
+extern "C" int phi_check() {
+  unsigned *d = nullptr;
+  if (cudaMalloc(&d, sizeof(unsigned)) != cudaSuccess) return -1;
+  cudaMemset(d, 0, sizeof(unsigned));
+  phi_kernel<<<1216, 256>>>(d);
+  return count(cudaGetLastError(), d);
+}
+extern "C" int sincos_check() {
+  unsigned *d = nullptr;
+  if (cudaMalloc(&d, sizeof(unsigned)) != cudaSuccess) return -1;
+  cudaMemset(d, 0, sizeof(unsigned));
+  sincos_kernel<<<1216, 256>>>(d);
   return count(cudaGetLastError(), d);
 }
 extern "C" int div3_check(unsigned n, int mode) {

@@ -28,6 +28,11 @@ def test_two_pi_times(math):
     assert math.two_pi_check() == 0
 
 
+def test_phi_and_its_sine_and_cosine(math):
+    assert math.phi_check() == 0
+    assert math.sincos_check() == 0
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 def test_div3(math, mode):
     assert math.div3_check(1 << 26, mode) == 0
