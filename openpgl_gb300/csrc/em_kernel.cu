@@ -218,31 +218,28 @@ __device__ void vmm_merge(VMMState &v, int i0, int i1) {  // PAVMM.h:259-343
   vmm_clear(v, int(v.K) - 1);
   v.K -= 1;
 }
+// The two lobes of a split (PAVMM.h:225-255); the caller sets K and the norms.
 __device__ void vmm_split(VMMState &v, int i0, int i1, float w0, float w1, V3 m0, V3 m1, float mc0, float mc1) {
-  v.dist[i1] = v.dist[i0];  // PAVMM.h:225-255
+  v.dist[i1] = v.dist[i0];
   v.w[i0] = w0; v.mc[i0] = mc0; v.kappa[i0] = mean_cosine_to_kappa(mc0);
   v.mx[i0] = m0.x; v.my[i0] = m0.y; v.mz[i0] = m0.z;
   v.w[i1] = w1; v.mc[i1] = mc1; v.kappa[i1] = mean_cosine_to_kappa(mc1);
   v.mx[i1] = m1.x; v.my[i1] = m1.y; v.mz[i1] = m1.z;
-  if (uint32_t(i1) == v.K) v.K++;
-  vmm_calc_norm(v);
 }
-__device__ void vmm_parallax_shift(VMMState &v, V3 s) {  // PAVMM.h:809-831
-  int c = vec_count(int(v.K));
-  for (int k = 0; k < c * kLanes; ++k) {
-    V3 p = mk(v.mx[k], v.my[k], v.mz[k]) * v.dist[k] + s;
-    float len = length(p);
-    p = p / len;
-    bool cond = (v.dist[k] > 0.0f) && (v.dist[k] >= -FLT_MAX) && (v.dist[k] <= FLT_MAX);
-    if (cond) { v.mx[k] = p.x; v.my[k] = p.y; v.mz[k] = p.z; }
-    v.dist[k] = v.dist[k] > 0.0f ? len : 0.0f;
-  }
-  v.pivot[0] -= s.x; v.pivot[1] -= s.y; v.pivot[2] -= s.z;
+__device__ void vmm_parallax_shift(VMMState &v, V3 s, int k) {  // PAVMM.h:809-831, lobe k; the caller moves the pivot
+  V3 p = mk(v.mx[k], v.my[k], v.mz[k]) * v.dist[k] + s;
+  float len = length(p);
+  p = p / len;
+  bool cond = (v.dist[k] > 0.0f) && (v.dist[k] >= -FLT_MAX) && (v.dist[k] <= FLT_MAX);
+  if (cond) { v.mx[k] = p.x; v.my[k] = p.y; v.mz[k] = p.z; }
+  v.dist[k] = v.dist[k] > 0.0f ? len : 0.0f;
 }
+// Validity of a region's state: one warp, a lane per lobe.
 __device__ bool vmm_is_valid(const VMMState &v) {  // PAVMM.h:422-513
-  bool ok = true;
-  for (uint32_t k = 0; k < v.K && k < kMaxK; ++k) {
-    ok = ok && isvalidf(v.w[k]) && v.w[k] >= 0.0f && v.w[k] <= 1.0f + 1e-6f;
+  const uint32_t k = threadIdx.x & 31;
+  bool ok;
+  if (k < v.K) {
+    ok = isvalidf(v.w[k]) && v.w[k] >= 0.0f && v.w[k] <= 1.0f + 1e-6f;
     ok = ok && isvalidf(v.kappa[k]) && v.kappa[k] >= 0.0f;
     ok = ok && isvalidf(v.mc[k]) && v.mc[k] >= 0.0f && v.mc[k] <= 1.0f;
     ok = ok && isvalidf(v.mx[k]) && v.mx[k] >= -1.0f && v.mx[k] <= 1.0f;
@@ -250,12 +247,11 @@ __device__ bool vmm_is_valid(const VMMState &v) {  // PAVMM.h:422-513
     ok = ok && isvalidf(v.mz[k]) && v.mz[k] >= -1.0f && v.mz[k] <= 1.0f;
     ok = ok && isvalidf(v.norm[k]) && v.norm[k] >= 0.0f && isvalidf(v.e2k[k]);
     ok = ok && isvalidf(v.dist[k]) && v.dist[k] >= 0.0f;
-  }
-  for (uint32_t k = v.K; k < kMaxK; ++k) {
-    ok = ok && v.w[k] == 0.0f && v.kappa[k] == 0.0f && v.mx[k] == 0.0f && v.my[k] == 0.0f && v.mz[k] == 1.0f;
+  } else {
+    ok = v.w[k] == 0.0f && v.kappa[k] == 0.0f && v.mx[k] == 0.0f && v.my[k] == 0.0f && v.mz[k] == 1.0f;
     ok = ok && v.mc[k] == 0.0f && fabsf(v.norm[k] - kInv4Pi) < 1e-6f && v.e2k[k] == 1.0f && v.dist[k] == 0.0f;
   }
-  return ok;
+  return __all_sync(0xFFFFFFFFu, ok);
 }
 
 __device__ void suff_clear(SuffState &s, uint32_t K) {
@@ -295,19 +291,16 @@ __device__ void suff_decay(SuffState &s, float a) {
   for (int k = 0; k < kMaxK; ++k) { s.dx[k] *= a; s.dy[k] *= a; s.dz[k] *= a; s.w[k] *= a; s.dw[k] *= a; }
   s.numSamples *= a; s.sumWeights *= a;
 }
-__device__ void suff_parallax_shift(SuffState &s, const VMMState &v, V3 shift) {  // WEMFactory.h:265-283
-  int c = vec_count(int(v.K));
-  for (int k = 0; k < c * kLanes; ++k) {
-    V3 d0 = mk(s.dx[k], s.dy[k], s.dz[k]);
-    float smc = length(d0);
-    V3 d = d0 / smc;
-    d = d * v.dist[k];
-    d = d + shift;
-    d = d / length(d);
-    d = d * smc;
-    d = smc > 0.0f ? d : d0;
-    if (v.dist[k] > 0.0f) { s.dx[k] = d.x; s.dy[k] = d.y; s.dz[k] = d.z; }
-  }
+__device__ void suff_parallax_shift(SuffState &s, const VMMState &v, V3 shift, int k) {  // WEMFactory.h:265-283, lobe k
+  V3 d0 = mk(s.dx[k], s.dy[k], s.dz[k]);
+  float smc = length(d0);
+  V3 d = d0 / smc;
+  d = d * v.dist[k];
+  d = d + shift;
+  d = d / length(d);
+  d = d * smc;
+  d = smc > 0.0f ? d : d0;
+  if (v.dist[k] > 0.0f) { s.dx[k] = d.x; s.dy[k] = d.y; s.dz[k] = d.z; }
 }
 __device__ void suff_split(SuffState &s, int i, int j, V3 m0, V3 m1, float mc0, float mc1) {  // WEMFactory.h:516-550
   float sw = s.w[i];
@@ -316,7 +309,6 @@ __device__ void suff_split(SuffState &s, int i, int j, V3 m0, V3 m1, float mc0, 
   s.w[j] = sw; s.dx[j] = (m1.x * mc1) * sw; s.dy[j] = (m1.y * mc1) * sw; s.dz[j] = (m1.z * mc1) * sw;
   float t = s.dw[i] * 0.5f;
   s.dw[i] = t; s.dw[j] = t;
-  s.K += 1;
 }
 __device__ void suff_merge(SuffState &s, int i0, int i1) {  // WEMFactory.h:485-513
   int L = int(s.K) - 1;
@@ -326,13 +318,12 @@ __device__ void suff_merge(SuffState &s, int i0, int i1) {  // WEMFactory.h:485-
   s.K--;
 }
 __device__ bool suff_is_valid(const SuffState &s) {
-  bool ok = true;
-  for (uint32_t k = 0; k < s.K && k < kMaxK; ++k)
-    ok = ok && isvalidf(s.dx[k]) && isvalidf(s.dy[k]) && isvalidf(s.dz[k]) && isvalidf(s.w[k]) && s.w[k] >= 0.0f &&
-         isvalidf(s.dw[k]) && s.dw[k] >= 0.0f;
-  for (uint32_t k = s.K; k < kMaxK; ++k)
-    ok = ok && s.dx[k] == 0.0f && s.dy[k] == 0.0f && s.dz[k] == 0.0f && s.w[k] == 0.0f && s.dw[k] == 0.0f;
-  return ok && isvalidf(s.numSamples) && s.numSamples >= 0.0f && isvalidf(s.sumWeights) && s.sumWeights >= 0.0f;
+  const uint32_t k = threadIdx.x & 31;
+  const bool ok = k < s.K ? isvalidf(s.dx[k]) && isvalidf(s.dy[k]) && isvalidf(s.dz[k]) && isvalidf(s.w[k]) &&
+                                s.w[k] >= 0.0f && isvalidf(s.dw[k]) && s.dw[k] >= 0.0f
+                          : s.dx[k] == 0.0f && s.dy[k] == 0.0f && s.dz[k] == 0.0f && s.w[k] == 0.0f && s.dw[k] == 0.0f;
+  return __all_sync(0xFFFFFFFFu, ok) && isvalidf(s.numSamples) && s.numSamples >= 0.0f && isvalidf(s.sumWeights) &&
+         s.sumWeights >= 0.0f;
 }
 __device__ void split_clear(SplitState &s, uint32_t K) {
   s.K = K;
@@ -348,17 +339,13 @@ __device__ void split_decay(SplitState &s, float a) {
   for (int k = 0; k < c * kLanes; ++k) { s.cx[k] *= a; s.cy[k] *= a; s.cz[k] *= a; s.n[k] *= a; s.sw[k] *= a; s.sa[k] *= a; }
 }
 __device__ bool split_is_valid(const SplitState &s) {
-  bool lane[kLanes];
-  for (int j = 0; j < kLanes; ++j) lane[j] = true;
-  for (int k = 0; k < kMaxK; ++k) {
-    bool ok = isvalidf(s.mx[k]) && isvalidf(s.my[k]) && isvalidf(s.cx[k]) && isvalidf(s.cy[k]) && isvalidf(s.cz[k]) &&
-              isvalidf(s.chi2[k]) && s.chi2[k] >= 0.0f && isvalidf(s.sw[k]) && s.sw[k] >= 0.0f && isvalidf(s.sa[k]) &&
-              s.sa[k] >= 0.0f && isvalidf(s.n[k]) && s.n[k] >= 0.0f;
-    lane[k % kLanes] = lane[k % kLanes] && ok;
-  }
-  bool any = false;
-  for (int j = 0; j < kLanes; ++j) any = any || lane[j];
-  return any && s.K > 0 && s.K <= kMaxK;
+  const int k = threadIdx.x & 31;
+  const bool ok = isvalidf(s.mx[k]) && isvalidf(s.my[k]) && isvalidf(s.cx[k]) && isvalidf(s.cy[k]) &&
+                  isvalidf(s.cz[k]) && isvalidf(s.chi2[k]) && s.chi2[k] >= 0.0f && isvalidf(s.sw[k]) &&
+                  s.sw[k] >= 0.0f && isvalidf(s.sa[k]) && s.sa[k] >= 0.0f && isvalidf(s.n[k]) && s.n[k] >= 0.0f;
+  // a vector lane is good when it is in all four lobe vectors; one good lane is enough
+  const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
+  return (m & m >> 8 & m >> 16 & m >> 24 & 0xFFu) != 0 && s.K > 0 && s.K <= kMaxK;
 }
 
 // MAP M-step (WEMFactory.h:895-1148); mask == nullptr is the full step.
@@ -528,8 +515,14 @@ __device__ V3 map2d_to_3d(float x, float y) {  // Splitter.h:174-186
   return r;
 }
 
-// SplitComponent (Splitter.h:527-665)
-__device__ bool split_component(VMMState &v, SplitState &sp, SuffState &suff, int idx, const FieldConfig &cfg) {
+// SplitComponent (Splitter.h:527-665): what becomes of component idx, false
+// when it is not split.
+struct SplitLobes {
+  float w;  // of either
+  V3 m0, m1;
+  float mc0, mc1;
+};
+__device__ bool split_component(const VMMState &v, const SplitState &sp, int idx, const FieldConfig &cfg, SplitLobes &o) {
   float numAssigned = sp.sa[idx];
   float invSW = rcp_avx2(sp.sw[idx]);
   float meanx = sp.mx[idx], meany = sp.my[idx];
@@ -544,26 +537,21 @@ __device__ bool split_component(VMMState &v, SplitState &sp, SuffState &suff, in
   float w = v.w[idx], mc = v.mc[idx], kappa = v.kappa[idx];
   if (double(kappa) >= double(cfg.maxKappaSplit) * 0.9) return false;
   V3 mu = mk(v.mx[idx], v.my[idx], v.mz[idx]);
-  float nw0 = w * 0.5f, nw1 = nw0;
-  V3 m0 = mu, m1 = mu;
-  float nmc0 = mc, nmc1 = mc * mc;
+  o.w = w * 0.5f;
+  o.m0 = o.m1 = mu;
+  o.mc0 = mc;
+  o.mc1 = mc * mc;
   if (D > 1e-8f) {
     float ax = (e0x * ev0) * 0.5f, ay = (e0y * ev0) * 0.5f;
     Frame fr = frame_of(mu, false);
-    m0 = xfm(fr, map2d_to_3d(meanx + ax, meany + ay));
-    nmc0 = mc / fabsf(dot(mu, m0));
-    nmc0 = smin(nmc0, cfg.maxMeanCosineSplit);
-    nmc1 = nmc0;
-    m1 = xfm(fr, map2d_to_3d(meanx - ax, meany - ay));
+    o.m0 = xfm(fr, map2d_to_3d(meanx + ax, meany + ay));
+    o.mc0 = mc / fabsf(dot(mu, o.m0));
+    o.mc0 = smin(o.mc0, cfg.maxMeanCosineSplit);
+    o.mc1 = o.mc0;
+    o.m1 = xfm(fr, map2d_to_3d(meanx - ax, meany - ay));
   } else {
     if (numAssigned < 2.0f) return false;
   }
-  int K = int(v.K);
-  vmm_split(v, idx, K, nw0, nw1, m0, m1, nmc0, nmc1);
-  suff_split(suff, idx, K, m0, m1, nmc0, nmc1);
-  split_zero_lane(sp, idx);
-  split_zero_lane(sp, K);
-  sp.K = uint32_t(K + 1);
   return true;
 }
 
@@ -2118,20 +2106,83 @@ __device__ int em_loop(EmShared &S, const LeafSamples &L, SuffState &prev, bool 
   return S.iterations;
 }
 
+// getSplitCandidates (Splitter.h:1103-1117) by one warp: descending chi-square,
+// equal values keep index order (values without an order, NaN, as the
+// insertion sort of one thread leaves them).
 __device__ void sort_candidates(EmShared &S, const SplitState &sp) {
-  // getSplitCandidates (Splitter.h:1103-1117): descending chi-square, equal
-  // values keep index order
-  int n = int(sp.K);
-  for (int i = 0; i < n; ++i) { S.candIdx[i] = i; S.candChi[i] = sp.chi2[i]; }
-  for (int i = 1; i < n; ++i) {
-    int ci = S.candIdx[i];
-    float cv = S.candChi[i];
-    int j = i - 1;
-    while (j >= 0 && cv > S.candChi[j]) { S.candIdx[j + 1] = S.candIdx[j]; S.candChi[j + 1] = S.candChi[j]; --j; }
-    S.candIdx[j + 1] = ci;
-    S.candChi[j + 1] = cv;
+  const int n = int(sp.K), lane = threadIdx.x & 31;
+  const unsigned full = 0xFFFFFFFFu;
+  const float c = lane < n ? sp.chi2[lane] : 0.0f;
+  if (__any_sync(full, c != c)) {
+    if (lane == 0) {
+      for (int i = 0; i < n; ++i) { S.candIdx[i] = i; S.candChi[i] = sp.chi2[i]; }
+      for (int i = 1; i < n; ++i) {
+        int ci = S.candIdx[i];
+        float cv = S.candChi[i];
+        int j = i - 1;
+        while (j >= 0 && cv > S.candChi[j]) { S.candIdx[j + 1] = S.candIdx[j]; S.candChi[j + 1] = S.candChi[j]; --j; }
+        S.candIdx[j + 1] = ci;
+        S.candChi[j + 1] = cv;
+      }
+    }
+  } else {
+    int rank = 0;
+    for (int j = 0; j < n; ++j) {
+      const float o = __shfl_sync(full, c, j);
+      rank += (o > c || (o == c && j < lane)) ? 1 : 0;
+    }
+    if (lane < n) {
+      S.candIdx[rank] = lane;
+      S.candChi[rank] = c;
+    }
   }
-  S.numCands = n;
+  if (lane == 0) S.numCands = n;
+  __syncwarp();
+}
+// Splits the candidates above the threshold in order while there are slots
+// (Splitter.h:293-356, 364-420), by one warp, a lane per candidate: a split reads
+// its own component only and takes the slot behind the splits before it.  One
+// thread took 60,000 to 190,000 cycles per region and Update, a twentieth of a
+// small region's time.  Returns the splits made; tried: the candidates
+// considered.
+__device__ int split_candidates(EmShared &S, SplitState &sp, SuffState &suff, int n, const FieldConfig &cfg, int &tried) {
+  VMMState &v = S.vmm;
+  const int lane = threadIdx.x & 31, K = int(v.K);
+  const unsigned full = 0xFFFFFFFFu;
+  const bool wanted = lane < n && S.candChi[lane] > cfg.splitThreshold;
+  const int idx = wanted ? S.candIdx[lane] : 0;
+  SplitLobes o;
+  bool ok = wanted && split_component(v, sp, idx, cfg, o);
+  const int slot = K + __popc(__ballot_sync(full, ok) & ((1u << lane) - 1u));  // K when its turn comes
+  const bool considered = wanted && slot < int(kMaxK);
+  ok = ok && considered;
+  if (ok) {
+    vmm_split(v, idx, slot, o.w, o.w, o.m0, o.m1, o.mc0, o.mc1);
+    suff_split(suff, idx, slot, o.m0, o.m1, o.mc0, o.mc1);
+    split_zero_lane(sp, idx);
+    split_zero_lane(sp, slot);
+  }
+  if (considered) {
+    S.mask[idx] = 1;
+    S.mask[ok ? slot : slot - 1] = 1;  // the last component after its turn
+  }
+  const int made = __popc(__ballot_sync(full, ok));
+  tried = __popc(__ballot_sync(full, considered));
+  __syncwarp();
+  if (made > 0) {
+    if (lane == 0) {
+      v.K = uint32_t(K + made);
+      sp.K = uint32_t(K + made);
+      suff.K += uint32_t(made);
+    }
+    if (lane < vec_count(K + made) * kLanes) {  // vmm_calc_norm
+      v.e2k[lane] = fexp(-2.0f * v.kappa[lane]);
+      const float nrm = v.kappa[lane] / (kTwoPiF * (1.0f - v.e2k[lane]));
+      v.norm[lane] = v.kappa[lane] > 0.0f ? nrm : kInv4Pi;
+    }
+  }
+  __syncwarp();
+  return made;
 }
 
 // PerformMerging (Merger.h:67-89, 218-279): all pair costs in parallel, then
@@ -2245,19 +2296,16 @@ __device__ void recursive_splitting(EmShared &S, const LeafSamples &L, const Fie
       pass_split_stats(S, L, S.lsplit);
       PGL_PROF_END(tp0, cycSplit)
     }
-    if (tid == 0) {
+    if (tid < 32) {
       sort_candidates(S, S.lsplit);
-      for (int k = 0; k < kMaxK; ++k) S.mask[k] = 0;
-      int numComp = int(S.vmm.K);
-      for (int k = 0; k < numComp; ++k) {
-        if (S.candChi[k] > cfg.splitThreshold && S.vmm.K < kMaxK) {
-          bool ok = split_component(S.vmm, S.lsplit, S.temp, S.candIdx[k], cfg);
-          S.mask[S.candIdx[k]] = 1;
-          S.mask[S.vmm.K - 1] = 1;
-          if (ok) S.splitCount++;
-        }
+      S.mask[tid] = 0;
+      __syncwarp();
+      int tried;
+      const int made = split_candidates(S, S.lsplit, S.temp, int(S.vmm.K), cfg, tried);
+      if (tid == 0) {
+        S.splitCount += made;
+        if (S.splitCount > 0) suff_clear(S.temp, S.vmm.K);
       }
-      if (S.splitCount > 0) suff_clear(S.temp, S.vmm.K);
     }
     __syncthreads();
     if (S.splitCount > 0) {
@@ -2339,23 +2387,18 @@ __device__ void asm_update(EmShared &S, const LeafSamples &L, const FieldConfig 
       PGL_PROF_END(tp2, cycSplit)
     }
     if (afterSplit >= uint64_t(int64_t(cfg.minSplit))) {
-      if (tid == 0) {
-        for (int k = 0; k < kMaxK; ++k) S.mask[k] = 0;
+      if (tid < 32) {
+        S.mask[tid] = 0;
         sort_candidates(S, S.split);
-        int total = 0;
-        for (int k = 0; k < S.numCands; ++k) {
-          if (S.candChi[k] > cfg.splitThreshold && S.vmm.K < kMaxK) {
-            split_component(S.vmm, S.split, S.suff, S.candIdx[k], cfg);
-            S.mask[S.candIdx[k]] = 1;
-            S.mask[S.vmm.K - 1] = 1;
-            total++;
+        int total;
+        split_candidates(S, S.split, S.suff, S.numCands, cfg, total);
+        if (tid == 0) {
+          S.report.splits += uint32_t(total);
+          doRefit = (total > 0 && cfg.partialReFit && uint64_t(L.count) >= uint64_t(int64_t(cfg.minRefit))) ? 1 : 0;
+          if (doRefit) {
+            S.temp = S.suff;
+            suff_clear(S.temp, S.vmm.K);
           }
-        }
-        S.report.splits += uint32_t(total);
-        doRefit = (total > 0 && cfg.partialReFit && uint64_t(L.count) >= uint64_t(int64_t(cfg.minRefit))) ? 1 : 0;
-        if (doRefit) {
-          S.temp = S.suff;
-          suff_clear(S.temp, S.vmm.K);
         }
       }
       __syncthreads();
@@ -2485,21 +2528,30 @@ em_leaf_kernel(const LeafTask *tasks, uint32_t numTasks, unsigned int *queue, Em
       LeafSamples L{E.dirw + t.begin, E.pdf + t.begin, E.dist + t.begin, t.count};
       if (fit) {
         asm_fit(S, L, cfg, E.uniformDirs);
+        if (threadIdx.x < 32) valid = vmm_is_valid(S.vmm) ? 1u : 0u;
         if (threadIdx.x == 0) {
           S.vmm.pivot[0] = t.mean[0]; S.vmm.pivot[1] = t.mean[1]; S.vmm.pivot[2] = t.mean[2];
-          valid = vmm_is_valid(S.vmm) ? 1u : 0u;
           afterSplit = 0;
           afterMerge = 0;
         }
       } else {
-        if (threadIdx.x == 0 && cfg.parallax) {  // Field.h:476-482
-          V3 shift = mk(S.vmm.pivot[0] - t.mean[0], S.vmm.pivot[1] - t.mean[1], S.vmm.pivot[2] - t.mean[2]);
-          suff_parallax_shift(S.suff, S.vmm, shift);
-          vmm_parallax_shift(S.vmm, shift);
+        if (threadIdx.x < 32 && cfg.parallax) {  // Field.h:476-482, a lane per lobe
+          const V3 shift = mk(S.vmm.pivot[0] - t.mean[0], S.vmm.pivot[1] - t.mean[1], S.vmm.pivot[2] - t.mean[2]);
+          const int k = threadIdx.x;
+          if (k < vec_count(int(S.vmm.K)) * kLanes) {
+            suff_parallax_shift(S.suff, S.vmm, shift, k);
+            vmm_parallax_shift(S.vmm, shift, k);
+          }
+          __syncwarp();
+          if (k == 0) {
+            S.vmm.pivot[0] -= shift.x;
+            S.vmm.pivot[1] -= shift.y;
+            S.vmm.pivot[2] -= shift.z;
+          }
         }
         __syncthreads();
         asm_update(S, L, cfg, afterSplit, afterMerge);
-        if (threadIdx.x == 0)
+        if (threadIdx.x < 32)
           valid = (vmm_is_valid(S.vmm) && suff_is_valid(S.suff) && split_is_valid(S.split)) ? 1u : 0u;
       }
     } else if (fit) {

@@ -34,6 +34,15 @@ def test_out_of_range_quotients(weight, pdf):
     _check(frames)
 
 
+@pytest.mark.parametrize("seed", [740, 741, 742])
+def test_mixtures_that_run_out_of_slots(seed):
+    """Many clusters in one region: more components want to split than there
+    are slots left."""
+    from openpgl_gb300 import synthetic as syn
+
+    _check([syn.cluster_samples(10000, seed + 10 * i) for i in range(3)])
+
+
 def _check(frames):
     import openpgl_gb300 as pgl
     import pyoracle
