@@ -15,8 +15,9 @@
 // (one per accumulator, e.g. the x component of lobe 7's weighted direction
 // sum) add the chunk's terms in sample order.  That keeps the reference's
 // summation order (sequential over samples within each SIMD lane), so every
-// accumulator gets the reference's bits.  Scalar per-leaf logic (M step,
-// split/merge bookkeeping) runs on thread 0 between passes.
+// accumulator gets the reference's bits.  Per-leaf logic between the passes runs
+// on one warp, a lane per lobe (M step, splits, shifts, checks), on the whole block
+// (merge costs) or on thread 0.
 #include <cuda_runtime.h>
 
 #include <cstddef>
