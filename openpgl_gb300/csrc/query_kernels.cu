@@ -570,16 +570,25 @@ __device__ __forceinline__ GroupInit init_g(const FieldView &f, const Q &q, int 
   return r;
 }
 
-constexpr int kQueryThreads = 256, kHgThreads = 256, kHgBlocks = 4;
+// Blocks of a batch that fills the chip, and of one that does not: a small batch
+// takes one query's latency, which is shorter with few warps on an SM, with the
+// registers of few blocks and without the exchange of directions; one with the
+// phase function with a warp per query.  The lines lie where the forms cross
+// (launch by launch, us, large form / few): surface queries 777 10.8 / 10.0, 8,000
+// 12.0 / 11.2, 20,000 22.3 / 20.8 (1,048,576 635 / 706 without the exchange, in
+// blocks of 256); vertices 777 15.0 / 14.3, 8,000 16.2 / 15.6; phase function 300 11.6 / 8.3, 4,000 12.9 / 12.3, 8,000
+// 16.8 / 20.3.
+constexpr int kQueryThreads = 256, kQueryBlocks = 4, kFewThreads = 64, kFewBlocks = 4;
+constexpr uint32_t kFewQueries = 16384, kFewHg = 4096;
 // Batched volume guided queries with the Henyey-Greenstein product, two per
 // warp: Init + product with the phase function's fit + SamplePDF (+ pdfLi).
 // The mixture and its three products are live together, so a lane holds two
 // lobes of each; 64 registers for four blocks per SM.  262,147 queries: 507 us
 // with a warp per query, 377 us so (383 at 80 registers, 387 in blocks of 128
 // threads, 490 in blocks of 512).
-__global__ void __launch_bounds__(kHgThreads, kHgBlocks)
+__global__ void __launch_bounds__(kQueryThreads, kQueryBlocks)
 query_hg_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
-  __shared__ DirectionSlots<kHgThreads / 16> slots;
+  __shared__ DirectionSlots<kQueryThreads / 16> slots;
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
   const int lane = threadIdx.x & 31;
   const Group<2> G(lane);
@@ -641,15 +650,50 @@ query_hg_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
   if (gid < n && G.j == 0) out[gid] = o;
 }
 
+// The same for a batch that does not fill the chip: a warp per query, a lobe per
+// lane, so that a query's chain is one lobe's work.
+__global__ void query_hg_few_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (gw >= n) return;
+  const QueryIn q = in[gw];
+  const FieldView &f = P.f;
+  QueryOut o;
+  o.ok = 0; o.id = 0; o.s1d = q.s1d; o.dx = o.dy = o.dz = 0.0f; o.pdf = 0.0f; o.pdfLi = 0.0f;
+  bool inside = f.iteration > 0 && q.px >= f.bounds[0] && q.px <= f.bounds[3] && q.py >= f.bounds[1] &&
+                q.py <= f.bounds[4] && q.pz >= f.bounds[2] && q.pz <= f.bounds[5];
+  if (inside) {
+    uint32_t leaf = kd_leaf(f, q.px, q.py, q.pz);
+    uint32_t reg = leaf;
+    float s1d = q.s1d;
+    if (f.knn && s1d >= 0.f) reg = choose_region(f, leaf, q.px, q.py, q.pz, s1d, lane);
+    o.s1d = s1d;
+    const RegionDir &R = f.regions[reg];
+    if (R.valid) {
+      const int K = int(R.vmm.K), cnt = vec_count(K);
+      Lobe li = load_shifted(R.vmm, lane, q.px, q.py, q.pz, f.parallax != 0);
+      Lobe h[kHgLobes];
+      float w[kHgLobes];
+      hg_products(li, mk(q.nx, q.ny, q.nz), P.hgMeanCosine[gw], cnt, lane, h, w);
+      const V3 d = products_sample(h, w, kHgLobes, K, q.ux, q.uy, lane, o.pdf);
+      o.ok = 1;
+      o.id = leaf;
+      o.dx = d.x; o.dy = d.y; o.dz = d.z;
+      o.pdfLi = mixture_pdf(li, d, cnt, lane);
+    }
+  }
+  if (lane == 0) out[gw] = o;
+}
+
 // Batched guided queries, four per warp: Init + optional cosine product
 // (surface) + SamplePDF (+ pdfLi).  Issue bound at about three quarters of the
 // issue rate; 64 registers for four blocks per SM.  1,048,576 queries: 818 us
 // with searches by branches, FP64 in lobe_direction, divisions one by one and
 // the rsqrt table in constant memory (its lookups went one by one), 635 us so
 // (687 at 80 registers, 660 at 48, 669 in blocks of 128 threads).
-__global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
+template <int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks)
 query_g_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
-  __shared__ DirectionSlots<kQueryThreads / 8> slots;
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   const int lane = threadIdx.x & 31;
   const Group<1> G(lane);
@@ -669,7 +713,14 @@ query_g_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
     if (P.cosine) g = product_lobe_g<1>(G, li, mk(q.nx, q.ny, q.nz), P.cosKappa, P.cosNorm, 1.0f, cnt, integral);
     p = mixture_pick_g<1>(G, g, K, q.uy);
   }
-  const V3 d = block_direction(slots, threadIdx.x >> 3, G.j == 0, p, (q.ux - 0.0f) / 1.0f);
+  const float ux = (q.ux - 0.0f) / 1.0f;
+  V3 d;
+  if constexpr (kThreads == kFewThreads) {
+    d = lobe_direction(p.kappa, p.e2k, p.mu, ux, p.u1);
+  } else {
+    __shared__ DirectionSlots<kThreads / 8> slots;
+    d = block_direction(slots, threadIdx.x >> 3, G.j == 0, p, ux);
+  }
   QueryOut o;
   o.ok = 0; o.id = 0; o.s1d = init.s1d; o.dx = o.dy = o.dz = 0.0f; o.pdf = 0.0f; o.pdfLi = 0.0f;
   if (init.ok) {
@@ -689,10 +740,10 @@ query_g_kernel(QueryParams P, const QueryIn *in, QueryOut *out, uint32_t n) {
 // four lobes one after the other, and the block finds all their directions at
 // once.  1,000,003 vertices: 1,838 us with four runs through lobe_direction per
 // vertex, 877 us so.
-__global__ void __launch_bounds__(kQueryThreads, 1024 / kQueryThreads)
+template <int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks)
 query_s4_g_kernel(QueryParams P, const QueryInS4 *in, QueryOutS4 *out, uint32_t n) {
   static_assert(kVertexSamples == 4, "two lanes of a group per sample");
-  __shared__ DirectionSlots<kQueryThreads / 2> slots;
   const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   const int lane = threadIdx.x & 31;
   const Group<1> G(lane);
@@ -720,7 +771,13 @@ query_s4_g_kernel(QueryParams P, const QueryInS4 *in, QueryOutS4 *out, uint32_t 
       if (k == mine) p = t;
     }
   }
-  V3 d = block_direction(slots, (threadIdx.x >> 3) * 4 + mine, G.j < kVertexSamples, p, (ux - 0.0f) / 1.0f);
+  V3 d;
+  if constexpr (kThreads == kFewThreads) {
+    d = lobe_direction(p.kappa, p.e2k, p.mu, (ux - 0.0f) / 1.0f, p.u1);
+  } else {
+    __shared__ DirectionSlots<kThreads / 2> slots;
+    d = block_direction(slots, (threadIdx.x >> 3) * 4 + mine, G.j < kVertexSamples, p, (ux - 0.0f) / 1.0f);
+  }
   float pdf = 0.0f;  // of sample `mine`
   if (init.ok) {
 #pragma unroll 1
@@ -931,28 +988,39 @@ cudaError_t query_upload_tables(const LibmTables &libm) {
 cudaError_t launch_query(const QueryParams &p, const QueryIn *in, QueryOut *out, uint32_t n, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const unsigned threads = 256;
+  const auto blocks = [&](unsigned lanes, unsigned per) { return unsigned((uint64_t(n) * lanes + per - 1) / per); };
   count_launch();
   if (p.f.dqt) {
     query_dqt_kernel<<<unsigned((uint64_t(n) + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
     return cudaGetLastError();
   }
   if (p.hgMeanCosine) {
-    query_hg_kernel<<<unsigned((uint64_t(n) * 16 + kHgThreads - 1) / kHgThreads), kHgThreads, 0, s>>>(p, in, out, n);
+    if (n <= kFewHg)
+      query_hg_few_kernel<<<blocks(32, kFewThreads), kFewThreads, 0, s>>>(p, in, out, n);
+    else
+      query_hg_kernel<<<blocks(16, kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
     return cudaGetLastError();
   }
-  query_g_kernel<<<unsigned((uint64_t(n) * 8 + kQueryThreads - 1) / kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
+  if (n <= kFewQueries)
+    query_g_kernel<kFewThreads, kFewBlocks><<<blocks(8, kFewThreads), kFewThreads, 0, s>>>(p, in, out, n);
+  else
+    query_g_kernel<kQueryThreads, kQueryBlocks><<<blocks(8, kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
   return cudaGetLastError();
 }
 cudaError_t launch_query_s4(const QueryParams &p, const QueryInS4 *in, QueryOutS4 *out, uint32_t n,
                             cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const unsigned threads = 256;
+  const auto blocks = [&](unsigned lanes, unsigned per) { return unsigned((uint64_t(n) * lanes + per - 1) / per); };
   count_launch();
   if (p.f.dqt) {
     query_s4_dqt_kernel<<<unsigned((uint64_t(n) + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
     return cudaGetLastError();
   }
-  query_s4_g_kernel<<<unsigned((uint64_t(n) * 8 + kQueryThreads - 1) / kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
+  if (n <= kFewQueries)
+    query_s4_g_kernel<kFewThreads, kFewBlocks><<<blocks(8, kFewThreads), kFewThreads, 0, s>>>(p, in, out, n);
+  else
+    query_s4_g_kernel<kQueryThreads, kQueryBlocks><<<blocks(8, kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
   return cudaGetLastError();
 }
 cudaError_t launch_ssd_init(const FieldView &f, float px, float py, float pz, float s1d, SSDState *st, SSDResult *res,

@@ -77,6 +77,21 @@ def test_batches_of_every_remainder(field):
         assert _rows_equal(f.sample_vertices(v[:n]), vert[:n]), n
 
 
+def test_small_batches_equal_their_rows_in_large_ones(field):
+    """Batches on either side of the sizes that take the kernels for few queries
+    (16,384, with the phase function 4,096)."""
+    from openpgl_gb300 import synthetic as syn
+
+    pgl, f = field
+    q, v = syn.queries(20000, 307), syn.vertices(20000, 308)
+    g = np.linspace(-0.99, 0.99, 20000).astype(np.float32)
+    plain, hg, vert = f.sample_batch(q), f.sample_batch_hg(q, g), f.sample_vertices(v)
+    for n in (4096, 4097, 16384, 16385):
+        assert _rows_equal(f.sample_batch(q[:n]), plain[:n]), n
+        assert _rows_equal(f.sample_batch_hg(q[:n], g[:n]), hg[:n]), n
+        assert _rows_equal(f.sample_vertices(v[:n]), vert[:n]), n
+
+
 def test_ends_of_the_random_numbers(field):
     from openpgl_gb300 import synthetic as syn
 
