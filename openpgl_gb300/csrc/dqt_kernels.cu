@@ -81,7 +81,7 @@ struct DqtScratch {  // per block, `scratchStride` entries each: trees too large
 };
 
 __device__ __noinline__ float dqt_divide(float a, float b) { return a / b; }
-// a leaf's share a / area of a box; y = RN(1 / area), 0 where the division is needed
+// a leaf's share a / area of a box, area not 0; y = RN(1 / area), 0 where the division is needed
 __device__ __forceinline__ float dqt_share(float a, float area, float y) {
   if (y == 0.0f || (a < 1e-25f && a != 0.0f)) return dqt_divide(a, area);
   return markstein_q(a, area, y);
@@ -213,6 +213,7 @@ __device__ void dqt_update(DqtShared &X, DqtHead &h, DqtStatsNode *Sg, DqtNode *
         const float hx = ff * (leaf.x1 - leaf.x0) / 2.0f, hy = ff * (leaf.y1 - leaf.y0) / 2.0f;
         filter = Box2{px - hx, py - hy, px + hx, py + hy}.intersect(Box2{0.f, 0.f, 1.f, 1.f});
         area = filter.area();
+        if (area == 0.0f) area = 1.0f;  // its sides round to the point: it overlaps nothing and gives no shares
       }
       X.box[tid] = make_float4(filter.x0, filter.y0, filter.x1, filter.y1);
       X.area[tid] = area;
@@ -308,16 +309,16 @@ __device__ void dqt_update(DqtShared &X, DqtHead &h, DqtStatsNode *Sg, DqtNode *
       auto put = [&](uint32_t l, uint32_t t, float w) {
         const uint32_t m = mask[l * words + t / 32], e = slotOf[l] + before[l * words + t / 32] +
                                                          uint32_t(__popc(m & ((1u << (t & 31)) - 1u)));
-        slot[e] = w;
-        slot[slots + e] = w * X.first[t];
-        slot[2 * slots + e] = w * X.second[t];
+        slot[e] = w;  // without a share the sample's moments do not count, whatever they are
+        slot[slots + e] = w != 0.0f ? w * X.first[t] : 0.0f;
+        slot[2 * slots + e] = w != 0.0f ? w * X.second[t] : 0.0f;
       };
       for (uint32_t j = 0; j < found; ++j)
         put(mine[j], s, ff > 0.0f ? dqt_share(dqt_overlap(box, leafRect[mine[j]]), area, inv) : 1.0f);
       for (uint32_t q = tid / 32; q < X.numLongs; q += kDqtThreads / 32) {  // a warp for a long list
         const uint32_t t = X.longs[q] % T;
         for (uint32_t k = 32 * (X.longs[q] / T) + (tid & 31); k < L; k += 32 * parts)
-          if (mask[k * words + t / 32] >> (t & 31) & 1u) put(k, t, dqt_overlap(X.box[t], leafRect[k]) / X.area[t]);
+          if (mask[k * words + t / 32] >> (t & 31) & 1u) put(k, t, dqt_share(dqt_overlap(X.box[t], leafRect[k]), X.area[t], 0.0f));
       }
       for (uint32_t k = tid; k < L; k += kDqtThreads) {  // the slots that round a leaf's up to a multiple of four
         const uint32_t q = k * words + words - 1;
