@@ -148,7 +148,10 @@ __device__ void dqt_update(DqtShared &X, DqtHead &h, DqtStatsNode *Sg, DqtNode *
   const uint32_t L = X.numLeaves;
   float4 *leafRect = L <= kDqtRects ? X.leafRect : Y.leafRect;  // padded to a multiple of 32 with nothing
   for (uint32_t l = tid; l < ((L + 31) & ~31u); l += kDqtThreads) {
-    const Box2 r = l < L ? rect[base[l]] : Box2{2.f, 2.f, 1.f, 1.f};
+    // without a footprint a sample counts for the leaf that its point descends to, which may
+    // have no width (its sides round together some 25 levels down): cells by number
+    const Box2 cell{float(l), 0.f, float(l) + 1.f, 1.f};
+    const Box2 r = l >= L ? Box2{2.f, 2.f, 1.f, 1.f} : ff > 0.0f ? rect[base[l]] : cell;
     leafRect[l] = make_float4(r.x0, r.y0, r.x1, r.y1);
   }
   // Samples per chunk: as many as the pool holds a matrix of shares for, or
@@ -207,7 +210,8 @@ __device__ void dqt_update(DqtShared &X, DqtHead &h, DqtStatsNode *Sg, DqtNode *
       }
       Box2 leaf;
       const uint32_t li = dqt_query(S, px, py, leaf);
-      Box2 filter = leaf;  // no footprint: the sample's leaf and nothing else
+      const float cell = float(count[li]);
+      Box2 filter{cell, 0.f, cell + 1.f, 1.f};
       float area = 1.0f;
       if (ff > 0.0f) {
         const float hx = ff * (leaf.x1 - leaf.x0) / 2.0f, hy = ff * (leaf.y1 - leaf.y0) / 2.0f;

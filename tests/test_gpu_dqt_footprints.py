@@ -1,5 +1,6 @@
 """Quadtree updates whose sample boxes have no area (a footprint so small that
-the box's sides round to its point), against the oracle: the same structure,
+the box's sides round to its point) and whose leaves have none (trees so deep
+that a leaf's sides round together), against the oracle: the same structure,
 statistics and validity after every frame."""
 
 import os
@@ -62,3 +63,11 @@ def _check(args, kind, n, frames, seed):
 ])
 def test_boxes_without_area(args, kind, n, frames):
     _check(args, kind, n, frames, 7100)
+
+
+# a leaf 25 levels down the square's far edge has no width; without a footprint the samples
+# count for the leaf that their points descend to all the same
+@pytest.mark.parametrize("threshold,n", [(0.1, 64), (0.02, 700)])
+def test_leaves_without_area(threshold, n):
+    nodes = _check((0, 0, threshold, 0.0, 30), "edge", n, 32, 7300)
+    assert nodes > 4 * 24  # as deep as where the sides round together
