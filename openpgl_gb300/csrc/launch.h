@@ -158,12 +158,15 @@ cudaError_t launch_em(const LeafTask *tasks, uint32_t numTasks, unsigned int *qu
 cudaError_t launch_query(const QueryParams &p, const QueryIn *in, QueryOut *out, uint32_t n, cudaStream_t s);
 // Samples of numPaths paths (path p = seg[begin[p], begin[p + 1])): offsets
 // (numPaths + 1 entries) gets each path's first sample slot and the total;
-// out needs room for the total (at most begin[numPaths]).
+// out needs room for the total (at most begin[numPaths]).  The blocks of a
+// launch talk to each other through `counts`, path_counts_bytes(numPaths) bytes
+// that are this launch's alone until it is done.
 struct PathSegmentRecord;
 struct PathFlags;
+size_t path_counts_bytes(uint32_t numPaths);
 cudaError_t launch_path_samples(const PathSegmentRecord *seg, const uint32_t *begin, uint32_t numPaths,
                                 float maxDistance, PathFlags fl, PGLSampleRecord *out, uint32_t *offsets,
-                                Scratch &scratch, int numSMs, cudaStream_t s);
+                                void *counts, int numSMs, cudaStream_t s);
 cudaError_t launch_ssd_init(const FieldView &f, float px, float py, float pz, float s1d, SSDState *st, SSDResult *res,
                             cudaStream_t s);
 cudaError_t launch_ssd_cosine(SSDState *st, float nx, float ny, float nz, float ck, float cn, cudaStream_t s);

@@ -567,22 +567,21 @@ path_samples_kernel(const PathSegmentRecord *seg, const uint32_t *begin, uint32_
   }
 }
 
+size_t path_counts_bytes(uint32_t numPaths) { return TileCounts::words(most_tiles(numPaths)) * sizeof(unsigned long long); }
 cudaError_t launch_path_samples(const PathSegmentRecord *seg, const uint32_t *begin, uint32_t numPaths,
                                 float maxDistance, PathFlags fl, PGLSampleRecord *out, uint32_t *offsets,
-                                Scratch &scratch, int numSMs, cudaStream_t s) {
+                                void *counts, int numSMs, cudaStream_t s) {
   if (numPaths == 0) return cudaMemsetAsync(offsets, 0, sizeof(uint32_t), s);
   // once per process (thread-safe static initialisation)
   static const cudaError_t attr =
       cudaFuncSetAttribute(path_samples_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(PathShared)));
   if (attr != cudaSuccess) return attr;
   const uint32_t most = most_tiles(numPaths), blocks = uint32_t(kPathBlocksPerSM * numSMs);
-  const size_t bytes = TileCounts::words(most) * sizeof(unsigned long long);
-  cudaError_t e = scratch_reserve(scratch, bytes);
-  if (e == cudaSuccess) e = cudaMemsetAsync(scratch.ptr, 0, bytes, s);
+  const cudaError_t e = cudaMemsetAsync(counts, 0, path_counts_bytes(numPaths), s);
   if (e != cudaSuccess) return e;
   count_launch();
   path_samples_kernel<<<most < blocks ? most : blocks, kPathThreads, sizeof(PathShared), s>>>(
-      seg, begin, numPaths, maxDistance, fl, scratch.ptr, offsets, out);
+      seg, begin, numPaths, maxDistance, fl, counts, offsets, out);
   return cudaGetLastError();
 }
 

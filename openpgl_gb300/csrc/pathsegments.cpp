@@ -27,6 +27,28 @@ static_assert(offsetof(PGLPathSegmentData, volumeScatter) == offsetof(PathSegmen
               "path segment fields");
 static_assert(sizeof(PGLSampleData) == sizeof(PGLSampleRecord), "sample layout");
 
+// What the blocks of one device batch tell each other lives from a point of the
+// caller's stream to a later one, and each call has its own: calls on several
+// streams may run at the same time, from one thread or many, and a captured call
+// whenever its graph does.  The pool keeps up to 64 MB between calls (a call of
+// 131,072 paths takes 139 KB) and never makes one stream wait for another.
+static cudaMemPool_t path_counts_pool(int device) {
+  static const cudaMemPool_t pool = [&] {  // thread-safe one-time set-up
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t p = nullptr;
+    check(cudaMemPoolCreate(&p, &props), "path counts pool");
+    uint64_t keep = 64ull << 20;
+    int no = 0;
+    check(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep), "path counts pool");
+    check(cudaMemPoolSetAttribute(p, cudaMemPoolReuseAllowInternalDependencies, &no), "path counts pool");
+    return p;
+  }();
+  return pool;
+}
+
 // PathSegmentDataStorage with OPENPGL_PATHSEGMENT_STORAGE_USE_ARRAY: fixed
 // arrays of the reserved size.  Where the reference writes one element past
 // them (its bounds test is `index + 1 <= size`), this one stops at the size.
@@ -231,11 +253,16 @@ OPENPGL_CORE_INTERFACE bool pglPathSegmentsPrepareSamplesDevice(const PGLPathSeg
   if (numPaths >= 0xFFFFFFFFull) throw std::runtime_error("too many paths for one call");
   Context &c = Context::get();
   cudaStream_t st = cudaStream ? static_cast<cudaStream_t>(cudaStream) : c.stream;
-  static thread_local Scratch scratch;
-  check(launch_path_samples(reinterpret_cast<const PathSegmentRecord *>(dSegments), dPathBegin, uint32_t(numPaths),
-                            maxDistance, PathFlags{useNEEMiWeights, guideDirectLight, rrAffectsDirectContribution},
-                            reinterpret_cast<PGLSampleRecord *>(dSamples), dSampleBegin, scratch, c.numSMs, st),
-        "path samples");
+  void *counts = nullptr;
+  check(cudaMallocFromPoolAsync(&counts, path_counts_bytes(uint32_t(numPaths)), path_counts_pool(c.device), st),
+        "path counts");
+  const cudaError_t e =
+      launch_path_samples(reinterpret_cast<const PathSegmentRecord *>(dSegments), dPathBegin, uint32_t(numPaths),
+                          maxDistance, PathFlags{useNEEMiWeights, guideDirectLight, rrAffectsDirectContribution},
+                          reinterpret_cast<PGLSampleRecord *>(dSamples), dSampleBegin, counts, c.numSMs, st);
+  const cudaError_t freed = cudaFreeAsync(counts, st);
+  check(e, "path samples");
+  check(freed, "path counts");
   return true;
   PGL_PS_CATCH(false)
 }
