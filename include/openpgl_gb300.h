@@ -166,7 +166,10 @@ OPENPGL_CORE_INTERFACE size_t pglFieldGetEmTuningTrials(PGLField field, int *tun
 // sample count) in path order, each path's in the reference's order, and
 // path p's first slot to dSampleBegin[p] (numPaths + 1 entries, the last is
 // the total).  Enqueued on cudaStream (null: the library's stream); does not
-// synchronise.
+// synchronise.  The blocks of the launch wait for each other's counts with a
+// limit of some seconds without progress, which no input reaches by its size;
+// should a wait run out all the same, the total is 0xFFFFFFFF and the other
+// outputs are undefined.
 OPENPGL_CORE_INTERFACE bool pglPathSegmentsPrepareSamplesDevice(const PGLPathSegmentData *dSegments,
                                                                 const uint32_t *dPathBegin, size_t numPaths,
                                                                 float maxDistance, bool useNEEMiWeights,

@@ -160,13 +160,16 @@ cudaError_t launch_query(const QueryParams &p, const QueryIn *in, QueryOut *out,
 // (numPaths + 1 entries) gets each path's first sample slot and the total;
 // out needs room for the total (at most begin[numPaths]).  The blocks of a
 // launch talk to each other through `counts`, path_counts_bytes(numPaths) bytes
-// that are this launch's alone until it is done.
+// that are this launch's alone until it is done.  A block that looks waitLimit times in
+// vain for the counts of those before it, with no sign of work from them, fails
+// the launch: offsets[numPaths] is then ~0 and the rest of the output undefined.
 struct PathSegmentRecord;
 struct PathFlags;
+constexpr uint32_t kPathWaitLimit = 1u << 23;  // some seconds
 size_t path_counts_bytes(uint32_t numPaths);
 cudaError_t launch_path_samples(const PathSegmentRecord *seg, const uint32_t *begin, uint32_t numPaths,
                                 float maxDistance, PathFlags fl, PGLSampleRecord *out, uint32_t *offsets,
-                                void *counts, int numSMs, cudaStream_t s);
+                                void *counts, int numSMs, cudaStream_t s, uint32_t waitLimit = kPathWaitLimit);
 cudaError_t launch_ssd_init(const FieldView &f, float px, float py, float pz, float s1d, SSDState *st, SSDResult *res,
                             cudaStream_t s);
 cudaError_t launch_ssd_cosine(SSDState *st, float nx, float ny, float nz, float ck, float cn, cudaStream_t s);

@@ -51,7 +51,7 @@ struct PathShared {
   PathTile tiles[2];  // this tile and the next
   uint32_t made[kPathRounds * kPathWarps], before[kPathRounds * kPathWarps + 1];
   uint32_t base, sorted;
-  int failed;
+  bool failed;
   uint32_t depth[kDepths];
   union {
     uint32_t order[kStagedSegments];  // vertices by depth: record, place in the path, the path's segments
@@ -305,11 +305,25 @@ __device__ __forceinline__ void write_staged(const PathShared &S, const PathTile
 }
 
 // A path with more segments than the stage holds: a thread per vertex on the
-// records in memory; out == nullptr counts.
+// records in memory; out == nullptr counts.  Its time grows with the square of the
+// segments, so every thousand steps or so a thread says that it is still at it
+// (any new value will do), and the tiles behind keep waiting.
 __device__ __noinline__ uint32_t long_path(const PathSegmentRecord *seg, int n, float maxDistance,
-                                           PathFlags fl, PGLSampleRecord *out) {
+                                           PathFlags fl, PGLSampleRecord *out, unsigned long long *progress) {
   PathShared &S = path_shared();
-  uint32_t total = 0;
+  uint32_t total = 0, steps = 0;
+  const auto beat = [&] {
+    if ((++steps & 1023u) == 0) *static_cast<volatile unsigned long long *>(progress) = (unsigned long long)clock64();
+  };
+  const auto step = [&](int v) { return vertex_step(seg[v], seg[v + 1]); };
+  const auto factor = [&](int v) {
+    beat();
+    return vertex_factor(seg[v]);
+  };
+  const auto rcp = [&](const PathSegmentRecord &s) {
+    beat();
+    return rr_reciprocal(s.rr);
+  };
   for (int top = n - 2; top >= 0; top -= kPathRounds * kPathThreads) {
     bool made[kPathRounds];
 #pragma unroll 1
@@ -317,11 +331,9 @@ __device__ __noinline__ uint32_t long_path(const PathSegmentRecord *seg, int n, 
       const int i = top - (r * kPathThreads + int(threadIdx.x));
       made[r] = false;
       if (i >= 0 && vertex_eligible(seg[i])) {
-        const float distance =
-            vertex_distance(i, n, maxDistance, [&](int v) { return vertex_step(seg[v], seg[v + 1]); },
-                            [&](int v) { return vertex_factor(seg[v]); });
+        const float distance = vertex_distance(i, n, maxDistance, step, factor);
         float c[3];
-        vertex_contribution(seg + i, n - i, fl, [](const PathSegmentRecord &s) { return rr_reciprocal(s.rr); }, c);
+        vertex_contribution(seg + i, n - i, fl, rcp, c);
         made[r] = made_sample(c, distance);
       }
       const uint32_t mask = __ballot_sync(0xFFFFFFFFu, made[r]);
@@ -335,7 +347,7 @@ __device__ __noinline__ uint32_t long_path(const PathSegmentRecord *seg, int n, 
         if (!made[r]) continue;
         const PathSegmentRecord &cur = seg[i];
         float c[3];
-        vertex_contribution(seg + i, n - i, fl, [](const PathSegmentRecord &s) { return rr_reciprocal(s.rr); }, c);
+        vertex_contribution(seg + i, n - i, fl, rcp, c);
         PGLSampleRecord o;
         o.px = cur.px;
         o.py = cur.py;
@@ -345,8 +357,7 @@ __device__ __noinline__ uint32_t long_path(const PathSegmentRecord *seg, int n, 
         o.dz = cur.diz;
         o.pdf = vertex_pdf(cur);
         o.weight = ((c[0] + c[1] + c[2]) / 3.0f) / o.pdf;
-        o.distance = vertex_distance(i, n, maxDistance, [&](int v) { return vertex_step(seg[v], seg[v + 1]); },
-                                     [&](int v) { return vertex_factor(seg[v]); });
+        o.distance = vertex_distance(i, n, maxDistance, step, factor);
         o.flags = cur.volumeScatter ? 2u : 0u;
         out[total + made_before(S, uint32_t(x))] = o;
       }
@@ -358,7 +369,8 @@ __device__ __noinline__ uint32_t long_path(const PathSegmentRecord *seg, int n, 
 }
 
 // The counts that say where a tile's samples go, in groups of 32 tiles.  All
-// words start at zero: ticket, then per tile its samples (bit 63 set when known),
+// words start at zero: ticket, whether a wait ran out, the last sign of a long path
+// at work, then per tile its samples (bit 63 set when known),
 // per group the sum of its tiles' samples (the tiles added so far above bit 40)
 // and the samples before it (bit 63 set when known).  A tile reads its group's
 // tiles and up to 32 groups per step, so the blocks that wait at the same time
@@ -367,32 +379,51 @@ __device__ __noinline__ uint32_t long_path(const PathSegmentRecord *seg, int n, 
 constexpr unsigned long long kKnown = 1ull << 63;
 constexpr int kGroupShift = 40;  // samples are fewer than 2^32: a group's sum stays below
 struct TileCounts {
-  unsigned long long *ticket, *tile, *group, *before;
+  unsigned long long *ticket, *failed, *progress, *tile, *group, *before;
   __host__ __device__ TileCounts(void *words, uint32_t numTiles) {
     const size_t groups = (size_t(numTiles) + 31) / 32;
     ticket = static_cast<unsigned long long *>(words);
-    tile = ticket + 1;
+    failed = ticket + 1;
+    progress = ticket + 2;
+    tile = ticket + 3;
     group = tile + numTiles;
     before = group + groups;
   }
-  static size_t words(uint32_t numTiles) { return 1 + size_t(numTiles) + 2 * ((size_t(numTiles) + 31) / 32); }
+  static size_t words(uint32_t numTiles) { return 3 + size_t(numTiles) + 2 * ((size_t(numTiles) + 31) / 32); }
 };
 __device__ __forceinline__ unsigned long long poll(const unsigned long long *p) {
   return *static_cast<const volatile unsigned long long *>(p);
 }
+// A wait's limit, in looks in vain (most of a microsecond each) since a long path last
+// showed itself at work.  One wait that runs out fails the whole launch: every
+// other wait ends too, and the total says so.
+struct PathWait {
+  uint32_t looks = 0;
+  unsigned long long seen = 0;
+  __device__ __forceinline__ bool over(const TileCounts &C, uint32_t limit) {
+    if ((++looks & 63u) != 0) return false;  // many wait at once: they read the shared words now and then
+    if (__shfl_sync(0xFFFFFFFFu, poll(C.failed), 0) != 0) return true;
+    const unsigned long long now = __shfl_sync(0xFFFFFFFFu, poll(C.progress), 0);
+    if (now != seen) {
+      seen = now;
+      looks = 0;
+    }
+    return looks >= limit;
+  }
+};
 // Samples before this tile (one warp calls it).  Blocks take their tiles in
 // order, each its next one only when this one's samples are counted, and wait
 // for earlier tiles only, so the earliest tile not yet counted is always being
-// worked on; the wait has a limit of some seconds all the same.
-__device__ __forceinline__ uint32_t samples_before(const TileCounts &C, uint32_t tile, uint32_t total, int *failed) {
+// worked on; the wait has a limit all the same.
+__device__ __forceinline__ uint32_t samples_before(const TileCounts &C, uint32_t tile, uint32_t total, uint32_t limit,
+                                                   bool *failed) {
   const int lane = threadIdx.x & 31;
   const uint32_t group = tile / 32, first = group * 32;
   if (lane == 0) {
     atomicExch(&C.tile[tile], kKnown | total);
     atomicAdd(&C.group[group], 1ull << kGroupShift | total);
   }
-  const long long start = clock64();
-  const auto expired = [&] { return __any_sync(0xFFFFFFFFu, clock64() - start > (1ll << 32)); };
+  PathWait wait;
   uint32_t sum = 0;
   for (int64_t last = int64_t(group) - 1; last >= 0;) {
     // groups last, last - 1, ...: their sums, down to one with the samples before it known
@@ -414,8 +445,7 @@ __device__ __forceinline__ uint32_t samples_before(const TileCounts &C, uint32_t
       }
       last -= 32;
     } else {
-      if (expired()) *failed = 1;
-      if (*failed) return 0;
+      if ((*failed = wait.over(C, limit))) return 0;
       __nanosleep(200);
     }
   }
@@ -425,8 +455,7 @@ __device__ __forceinline__ uint32_t samples_before(const TileCounts &C, uint32_t
     const unsigned long long v = before ? poll(&C.tile[first + lane]) : kKnown;
     if (__all_sync(0xFFFFFFFFu, (v & kKnown) != 0))
       return sum + __reduce_add_sync(0xFFFFFFFFu, before ? uint32_t(v) : 0u);
-    if (expired()) *failed = 1;
-    if (*failed) return 0;
+    if ((*failed = wait.over(C, limit))) return 0;
     __nanosleep(100);
   }
 }
@@ -482,7 +511,7 @@ __host__ __device__ inline uint32_t most_tiles(uint32_t numPaths) {
 }
 __global__ void __launch_bounds__(kPathThreads, kPathBlocksPerSM)
 path_samples_kernel(const PathSegmentRecord *seg, const uint32_t *begin, uint32_t numPaths, float maxDistance,
-                    PathFlags fl, void *counts, uint32_t *offsets, PGLSampleRecord *out) {
+                    PathFlags fl, void *counts, uint32_t waitLimit, uint32_t *offsets, PGLSampleRecord *out) {
   PathShared &S = path_shared();
   const int warp = threadIdx.x >> 5;
   const TileCounts C(counts, most_tiles(numPaths));
@@ -495,7 +524,6 @@ path_samples_kernel(const PathSegmentRecord *seg, const uint32_t *begin, uint32_
     perTile = max(uint32_t(uint64_t(kTileSegments) * numPaths / segments), uint32_t(kMinTilePaths));
   perTile = min(perTile, max((numPaths + gridDim.x - 1) / gridDim.x, uint32_t(kMinTilePaths)));
   const uint32_t tiles = uint32_t((uint64_t(numPaths) + perTile - 1) / perTile);
-  if (threadIdx.x == 0) S.failed = 0;
   if (warp == 1) next_tile(S.tiles[0], C.ticket, tiles, perTile, begin, numPaths);
   __syncthreads();
   for (int buffer = 0; S.tiles[buffer].np > 0; buffer ^= 1) {
@@ -518,32 +546,36 @@ path_samples_kernel(const PathSegmentRecord *seg, const uint32_t *begin, uint32_
       lastA = a;
       lastZ = z;
       lastCount = z > a ? staged_samples(buffer, seg, a, z, maxDistance, fl)
-                        : long_path(seg + T.begin[a], T.n(a), maxDistance, fl, nullptr);
+                        : long_path(seg + T.begin[a], T.n(a), maxDistance, fl, nullptr, C.progress);
       total += lastCount;
       a = z > a ? z : a + 1;
     }
     if (warp == 0) {
-      int failed = 0;
-      const uint32_t before = samples_before(C, T.tile, total, &failed);
+      bool failed = false;
+      const uint32_t before = samples_before(C, T.tile, total, waitLimit, &failed);
       if (threadIdx.x == 0) {
         S.base = before;
         S.failed = failed;
+        if (failed) {  // this total is written after the word, the last tile's before it looks at the word
+          atomicExch(C.failed, 1ull);
+          __threadfence();
+          offsets[numPaths] = ~0u;
+        }
       }
     } else if (warp == 1) {
       next_tile(S.tiles[buffer ^ 1], C.ticket, tiles, perTile, begin, numPaths);
     }
     __syncthreads();
-    const bool failed = S.failed != 0;
+    if (S.failed) return;
     const uint32_t base = S.base;
-    if (threadIdx.x == 0 && T.first + uint32_t(np) == numPaths) at[np] = failed ? ~0u : base + total;
-    if (failed) {
-      for (int p = int(threadIdx.x); p < np; p += kPathThreads) at[p] = ~0u;
-      __syncthreads();
-      continue;
+    if (threadIdx.x == 0 && T.first + uint32_t(np) == numPaths) {
+      at[np] = base + total;
+      __threadfence();
+      if (poll(C.failed) != 0) at[np] = ~0u;
     }
     const auto write_long = [&](int a, uint32_t to) {
       if (threadIdx.x == 0) at[a] = to;
-      return long_path(seg + T.begin[a], T.n(a), maxDistance, fl, out + to);
+      return long_path(seg + T.begin[a], T.n(a), maxDistance, fl, out + to, C.progress);
     };
     if (lastZ > lastA)
       write_staged(S, T, lastA, lastZ, base + total - lastCount, lastCount, at, out);
@@ -570,7 +602,7 @@ path_samples_kernel(const PathSegmentRecord *seg, const uint32_t *begin, uint32_
 size_t path_counts_bytes(uint32_t numPaths) { return TileCounts::words(most_tiles(numPaths)) * sizeof(unsigned long long); }
 cudaError_t launch_path_samples(const PathSegmentRecord *seg, const uint32_t *begin, uint32_t numPaths,
                                 float maxDistance, PathFlags fl, PGLSampleRecord *out, uint32_t *offsets,
-                                void *counts, int numSMs, cudaStream_t s) {
+                                void *counts, int numSMs, cudaStream_t s, uint32_t waitLimit) {
   if (numPaths == 0) return cudaMemsetAsync(offsets, 0, sizeof(uint32_t), s);
   // once per process (thread-safe static initialisation)
   static const cudaError_t attr =
@@ -581,7 +613,7 @@ cudaError_t launch_path_samples(const PathSegmentRecord *seg, const uint32_t *be
   if (e != cudaSuccess) return e;
   count_launch();
   path_samples_kernel<<<most < blocks ? most : blocks, kPathThreads, sizeof(PathShared), s>>>(
-      seg, begin, numPaths, maxDistance, fl, counts, offsets, out);
+      seg, begin, numPaths, maxDistance, fl, counts, waitLimit, offsets, out);
   return cudaGetLastError();
 }
 
