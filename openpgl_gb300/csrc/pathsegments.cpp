@@ -28,10 +28,32 @@ static_assert(offsetof(PGLPathSegmentData, volumeScatter) == offsetof(PathSegmen
 static_assert(sizeof(PGLSampleData) == sizeof(PGLSampleRecord), "sample layout");
 
 // What the blocks of one device batch tell each other lives from a point of the
-// caller's stream to a later one, and each call has its own: calls on several
-// streams may run at the same time, from one thread or many, and a captured call
-// whenever its graph does.  The pool keeps up to 64 MB between calls (a call of
-// 131,072 paths takes 139 KB) and never makes one stream wait for another.
+// caller's stream to a later one: calls on several streams may run at the same
+// time, from one thread or many, and a captured call whenever its graph does.  So a
+// thread keeps a buffer for each of the first few streams that it uses, where
+// calls follow each other (streams by their ids, which are not given again), and
+// any other call, a captured one above all, takes its own from a pool in stream
+// order, which costs it 4 us of host time.  The pool keeps up to 64 MB between calls (a
+// call of 131,072 paths takes 139 KB) and never makes one stream wait for another.
+struct PathCounts {
+  unsigned long long stream = 0;
+  DevArray<unsigned char> kept;
+};
+static void *kept_path_counts(cudaStream_t stream, size_t bytes) {
+  static thread_local PathCounts counts[4];
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  check(cudaStreamIsCapturing(stream, &capture), "path counts");
+  if (capture != cudaStreamCaptureStatusNone) return nullptr;
+  unsigned long long id = 0;
+  check(cudaStreamGetId(stream, &id), "path counts");
+  for (PathCounts &c : counts) {
+    if (c.kept.p && c.stream != id) continue;
+    c.stream = id;
+    c.kept.reserve(bytes);
+    return c.kept.p;
+  }
+  return nullptr;
+}
 static cudaMemPool_t path_counts_pool(int device) {
   static const cudaMemPool_t pool = [&] {  // thread-safe one-time set-up
     cudaMemPoolProps props{};
@@ -253,14 +275,14 @@ OPENPGL_CORE_INTERFACE bool pglPathSegmentsPrepareSamplesDevice(const PGLPathSeg
   if (numPaths >= 0xFFFFFFFFull) throw std::runtime_error("too many paths for one call");
   Context &c = Context::get();
   cudaStream_t st = cudaStream ? static_cast<cudaStream_t>(cudaStream) : c.stream;
-  void *counts = nullptr;
-  check(cudaMallocFromPoolAsync(&counts, path_counts_bytes(uint32_t(numPaths)), path_counts_pool(c.device), st),
-        "path counts");
+  const size_t bytes = path_counts_bytes(uint32_t(numPaths));
+  void *const kept = kept_path_counts(st, bytes), *counts = kept;
+  if (!kept) check(cudaMallocFromPoolAsync(&counts, bytes, path_counts_pool(c.device), st), "path counts");
   const cudaError_t e =
       launch_path_samples(reinterpret_cast<const PathSegmentRecord *>(dSegments), dPathBegin, uint32_t(numPaths),
                           maxDistance, PathFlags{useNEEMiWeights, guideDirectLight, rrAffectsDirectContribution},
                           reinterpret_cast<PGLSampleRecord *>(dSamples), dSampleBegin, counts, c.numSMs, st);
-  const cudaError_t freed = cudaFreeAsync(counts, st);
+  const cudaError_t freed = kept ? cudaSuccess : cudaFreeAsync(counts, st);
   check(e, "path samples");
   check(freed, "path counts");
   return true;

@@ -45,14 +45,16 @@ def _alone(call):
     return to
 
 
-def test_two_streams_of_one_thread():
+# more streams than a thread keeps buffers for, too
+@pytest.mark.parametrize("count", [2, 7])
+def test_streams_of_one_thread(count):
     import torch
 
-    # long and short launches, so that each stream starts one while the other's runs
-    calls = [_call(200000, 51), _call(3000, 52)]
+    # long and short launches, so that each stream starts one while the others' run
+    calls = [_call((200000, 3000, 40000)[i % 3], 51 + i % 3) for i in range(count)]
     want = [_alone(c) for c in calls]
     streams = [torch.cuda.Stream() for _ in calls]
-    got = [[_outputs(c) for c in calls] for _ in range(12)]
+    got = [[_outputs(c) for c in calls] for _ in range(8)]
     for round_ in got:
         for c, to, s in zip(calls, round_, streams):
             _run(c, to, s)
