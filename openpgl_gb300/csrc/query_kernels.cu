@@ -573,13 +573,18 @@ __device__ __forceinline__ GroupInit init_g(const FieldView &f, const Q &q, int 
 // Blocks of a batch that fills the chip, and of one that does not: a small batch
 // takes one query's latency, which is shorter with few warps on an SM, with the
 // registers of few blocks and without the exchange of directions; one with the
-// phase function with a warp per query.  The lines lie where the forms cross
-// (launch by launch, us, large form / few): surface queries 777 10.8 / 10.0, 8,000
-// 12.0 / 11.2, 20,000 22.3 / 20.8 (1,048,576 635 / 706 without the exchange, in
-// blocks of 256); vertices 777 15.0 / 14.3, 8,000 16.2 / 15.6; phase function 300 11.6 / 8.3, 4,000 12.9 / 12.3, 8,000
-// 16.8 / 20.3.
+// phase function with a warp per query.  Surface and volume queries and vertices
+// take the small form while its blocks run in one wave (84 registers: ten blocks of
+// eight queries per SM, 12,160 queries; 72: fourteen, 17,024 vertices): it stays
+// ahead up to there and loses its gain with a second wave.  With the phase
+// function (one wave is 4,864) the forms cross before that.  Launch by launch, us,
+// large form / small:
+//   surface     777 10.8 / 9.9   8,192 12.0 / 11.2  12,000 13.8 / 12.5  13,000 13.9 / 18.6  16,384 16.0 / 19.4
+//   vertices    777 15.0 / 14.3  8,000 16.1 / 15.6  12,000 18.6 / 17.3  16,384 21.8 / 20.8  18,000 22.4 / 28.2
+//   phase fn.   300 11.7 / 8.3   3,000 12.5 / 10.0   4,096 12.9 / 12.3   4,400 12.9 / 13.2   5,200 14.6 / 16.2
+// (1,048,576 surface queries 635 / 706 us without the exchange, in blocks of 256).
 constexpr int kQueryThreads = 256, kQueryBlocks = 4, kFewThreads = 64, kFewBlocks = 4;
-constexpr uint32_t kFewQueries = 16384, kFewHg = 4096;
+constexpr uint32_t kFewQueries = 12160, kFewVertices = 16384, kFewHg = 4096;
 // Batched volume guided queries with the Henyey-Greenstein product, two per
 // warp: Init + product with the phase function's fit + SamplePDF (+ pdfLi).
 // The mixture and its three products are live together, so a lane holds two
@@ -1017,7 +1022,7 @@ cudaError_t launch_query_s4(const QueryParams &p, const QueryInS4 *in, QueryOutS
     query_s4_dqt_kernel<<<unsigned((uint64_t(n) + threads - 1) / threads), threads, 0, s>>>(p, in, out, n);
     return cudaGetLastError();
   }
-  if (n <= kFewQueries)
+  if (n <= kFewVertices)
     query_s4_g_kernel<kFewThreads, kFewBlocks><<<blocks(8, kFewThreads), kFewThreads, 0, s>>>(p, in, out, n);
   else
     query_s4_g_kernel<kQueryThreads, kQueryBlocks><<<blocks(8, kQueryThreads), kQueryThreads, 0, s>>>(p, in, out, n);
