@@ -203,10 +203,15 @@ __device__ __noinline__ uint32_t staged_samples(int buffer, const PathSegmentRec
                                                 float maxDistance, PathFlags fl) {
   PathShared &S = path_shared();
   const PathTile &T = S.tiles[buffer];
+  const uint32_t items = T.items[z] - T.items[a];
+  if (items == 0) {  // paths of one segment have no vertices: nothing to stage
+    if (threadIdx.x == 0) S.before[0] = 0;
+    __syncthreads();
+    return 0;
+  }
   if (threadIdx.x < kDepths) S.depth[threadIdx.x] = 0;
   PathSegmentRecord *stage = stage_segments(S, T, seg, a, z);
   float *words = reinterpret_cast<float *>(stage);
-  const uint32_t items = T.items[z] - T.items[a];
   int at[kPathRounds], bin[kPathRounds];
   uint32_t entry[kPathRounds], place[kPathRounds];
 #pragma unroll
