@@ -261,16 +261,6 @@ __device__ void suff_clear(SuffState &s, uint32_t K) {
   for (int k = 0; k < c * kLanes; ++k) s.dx[k] = s.dy[k] = s.dz[k] = s.w[k] = s.dw[k] = 0.0f;
   s.sumWeights = 0.0f; s.numSamples = 0.0f; s.normalized = 0;
 }
-__device__ void suff_normalize(SuffState &s, float n) {  // WEMFactory.h:553-572
-  int c = vec_count(int(s.K));
-  s.numSamples = n;
-  float sv[kLanes] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int k = 0; k < c * kLanes; ++k) sv[k % kLanes] += s.w[k];
-  s.sumWeights = reduce8(sv);
-  float nrm = n / s.sumWeights;
-  for (int k = 0; k < c * kLanes; ++k) { s.dx[k] *= nrm; s.dy[k] *= nrm; s.dz[k] *= nrm; s.w[k] *= nrm; }
-  s.normalized = 1;
-}
 __device__ void suff_add(SuffState &a, const SuffState &b) {  // WEMFactory.h:575-593
   int c = vec_count(int(a.K));
   a.sumWeights += b.sumWeights;
@@ -349,60 +339,10 @@ __device__ bool split_is_valid(const SplitState &s) {
   return (m & m >> 8 & m >> 16 & m >> 24 & 0xFFu) != 0 && s.K > 0 && s.K <= kMaxK;
 }
 
-// MAP M-step (WEMFactory.h:895-1148); mask == nullptr is the full step.
-__device__ void map_step(VMMState &v, const SuffState &cur, const SuffState &prev, const FieldConfig &cfg, const int *mask) {
-  int c = vec_count(int(v.K));
-  float K = float(v.K);
-  float N = cur.numSamples + prev.numSamples;
-  int rem = int(v.K % kLanes);
-  if (!mask) {
-    for (int k = 0; k < c * kLanes; ++k) {
-      float w = cur.w[k] + prev.w[k];
-      v.w[k] = (cfg.weightPrior + w) / ((cfg.weightPrior * K) + N);
-    }
-  } else {
-    float sw[kLanes] = {0, 0, 0, 0, 0, 0, 0, 0}, sp[kLanes] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < c * kLanes; ++k) {
-      float w = cur.w[k] + prev.w[k];
-      w = (cfg.weightPrior + w) / ((cfg.weightPrior * K) + N);
-      sp[k % kLanes] += mask[k] ? w : 0.0f;
-      sw[k % kLanes] += mask[k] ? 0.0f : v.w[k];
-      v.w[k] = mask[k] ? w : v.w[k];
-    }
-    float inv = 1.0f / reduce8(sp);
-    inv *= 1.0f - reduce8(sw);
-    for (int k = 0; k < c * kLanes; ++k) v.w[k] = mask[k] ? v.w[k] * inv : v.w[k];
-  }
-  if (rem > 0)
-    for (int i = rem; i < kLanes; ++i) v.w[(c - 1) * kLanes + i] = 0.0f;
-
-  float curN = cur.numSamples, prevN = prev.numSamples, NN = curN + prevN;
-  float overallN = cur.numSamples + prev.overallNumSamples;
-  float curW = curN / NN, prevW = 1.0f - curW;
-  for (int k = 0; k < c * kLanes; ++k) {
-    float partialN = v.w[k] * overallN;
-    V3 cm = cur.w[k] > 0.0f ? mk(cur.dx[k] / cur.w[k], cur.dy[k] / cur.w[k], cur.dz[k] / cur.w[k]) : mk(0, 0, 0);
-    V3 pm = prev.w[k] > 0.0f ? mk(prev.dx[k] / prev.w[k], prev.dy[k] / prev.w[k], prev.dz[k] / prev.w[k]) : mk(0, 0, 0);
-    V3 md = cm * curW + pm * prevW;
-    float mc = length(md);
-    bool upd = mask ? (mask[k] != 0) : true;
-    if (upd && mc > 0.0f) { v.mx[k] = md.x / mc; v.my[k] = md.y / mc; v.mz[k] = md.z / mc; }
-    mc = (cfg.mcPrior * cfg.mcPriorStrength + mc * partialN) / (cfg.mcPriorStrength + partialN);
-    mc = emin(cfg.maxMeanCosine, mc);
-    if (upd) { v.mc[k] = mc; v.kappa[k] = mean_cosine_to_kappa(mc); }
-  }
-  if (rem > 0)
-    for (int i = rem; i < kLanes; ++i) {
-      int k = (c - 1) * kLanes + i;
-      v.mx[k] = 0.0f; v.my[k] = 0.0f; v.mz[k] = 1.0f; v.mc[k] = 0.0f; v.kappa[k] = 0.0f;
-      if (!mask) { v.norm[k] = kInv4Pi; v.e2k[k] = 1.0f; }
-    }
-  vmm_calc_norm(v);
-}
-
-// suff_normalize and map_step by one warp, lane k doing lobe k: every lobe's
-// arithmetic is the scalar functions' own; the sums over lobes keep the
-// scalar order (vfloat8 lane sums over k, then the 8-lane reduction) on lane 0.
+// The statistics' normalisation (WEMFactory.h:553-572) and the MAP M-step
+// (WEMFactory.h:895-1148; mask == nullptr is the full step) by one warp, lane k
+// doing lobe k; the sums over lobes keep the reference's order (vfloat8 lane sums
+// over k, then the 8-lane reduction) on lane 0.
 __device__ void suff_normalize_warp(SuffState &s, float n) {
   const unsigned full = 0xFFFFFFFFu;
   const int k = int(threadIdx.x & 31);

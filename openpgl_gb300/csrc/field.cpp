@@ -21,9 +21,6 @@ void check(cudaError_t e, const char *what) {
   if (e != cudaSuccess) throw CudaError(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// The host C library's expf/cosf/sinf exception table (gen_libm_exceptions.cpp),
-// written by the build next to this library as libm_exceptions.bin, copied
-// to device memory that lives until the process exits.
 // The largest distance, relative to the value, between a listed input's value
 // and the rounding boundary beside the host's result (see LibmTables);
 // results that are not normal floats are left out (they are always looked up).
@@ -40,6 +37,9 @@ static float libm_margin(const float2 *v, uint32_t n, F exact) {
   return float(worst * 1.001);
 }
 
+// The host C library's expf/cosf/sinf exception table (gen_libm_exceptions.cpp),
+// written by the build next to this library as libm_exceptions.bin, copied
+// to device memory that lives until the process exits.
 static LibmTables load_libm_tables() {
   Dl_info info{};
   if (!dladdr(reinterpret_cast<void *>(&load_libm_tables), &info) || !info.dli_fname)
@@ -708,7 +708,7 @@ bool SubField::prepare(SampleSide &in) {
   for (DevArray<float4> *a : {&posA_, &posB_, &sP_, &sD_}) a->reserve(n);
   for (DevArray<float> *a : {&sPdf_, &dist_}) a->reserve(n);
   for (DevArray<uint32_t> *a : {&node_, &nodeB_, &jobOf_, &isLeft_, &scanLeft_}) a->reserve(n);
-  keys_.reserve(2 * size_t(n));
+  keys_.reserve(n);
   vals_.reserve(2 * size_t(n));
   keys64_.reserve(2 * size_t(n));
   check(init_posidx(in.P.p, n, posA_.p, stream()), "copy samples");
@@ -796,17 +796,15 @@ bool SubField::prepare(SampleSide &in) {
   std::sort(leafRegions.begin(), leafRegions.end(),
             [&](uint32_t a, uint32_t b) { return regions[a].rb < regions[b].rb; });
   const uint32_t L = uint32_t(leafRegions.size());
-  std::vector<uint32_t> seg(3 * size_t(L));
+  std::vector<uint32_t> seg(2 * size_t(L));
   for (uint32_t k = 0; k < L; ++k) {
     seg[k] = uint32_t(regions[leafRegions[k]].rb);
     seg[L + k] = uint32_t(regions[leafRegions[k]].re);
-    seg[2 * L + k] = uint32_t(regions[leafRegions[k]].re - regions[leafRegions[k]].rb);
   }
   leafSeg_.reserve(seg.size());
   check(cudaMemcpyAsync(leafSeg_.p, seg.data(), seg.size() * 4, cudaMemcpyHostToDevice, stream()), "segments");
-  check(gather_and_order(posA_.p, n, in.P.p, in.D.p, in.pdf.p, leafSeg_.p, leafSeg_.p + 2 * L, L, cfg.deterministic,
-                         vals_.p, keys64_.p, sP_.p, sD_.p, sPdf_.p, scratch_,
-                         stream()),
+  check(gather_and_order(posA_.p, n, in.P.p, in.D.p, in.pdf.p, leafSeg_.p, L, cfg.deterministic, vals_.p,
+                         keys64_.p, sP_.p, sD_.p, sPdf_.p, scratch_, stream()),
         "gather");
 
   // directional fit / update of every region (Field.h:389-511)

@@ -103,9 +103,10 @@ cudaError_t kd_level(const float4 *pos, const uint32_t *jobOf, uint32_t n, const
                      uint32_t *scanLeft, IStatsAcc *acc, float4 *posOut, uint32_t *nodeOut, Scratch &scratch,
                      cudaStream_t s);
 // Gathers samples into leaf order and applies the deterministic per-leaf
-// order (SampleDataLess) when `sorted`; leafBegin/leafCount are device arrays.
+// order (SampleDataLess) when `sorted`; leafBegin (device) holds the
+// leaves' first samples, then their ends.
 cudaError_t gather_and_order(const float4 *posIdx, uint32_t n, const float4 *P, const float4 *D, const float *pdf,
-                             const uint32_t *leafBegin, const uint32_t *leafCount, uint32_t numLeaves, bool sorted,
+                             const uint32_t *leafBegin, uint32_t numLeaves, bool sorted,
                              uint32_t *vals, unsigned long long *keys64, float4 *oP, float4 *oD, float *oPdf, Scratch &scratch,
                              cudaStream_t s);
 cudaError_t copy_regions(RegionDir *regions, const uint32_t *dst, const uint32_t *src, uint32_t n, cudaStream_t s);

@@ -847,7 +847,7 @@ cudaError_t kd_classify(const float4 *pos, const uint32_t *jobOf, uint32_t n, co
 }
 
 cudaError_t gather_and_order(const float4 *posIdx, uint32_t n, const float4 *P, const float4 *D, const float *pdf,
-                             const uint32_t *leafBegin, const uint32_t *leafCount, uint32_t numLeaves, bool sorted,
+                             const uint32_t *leafBegin, uint32_t numLeaves, bool sorted,
                              uint32_t *vals, unsigned long long *keys64, float4 *oP, float4 *oD, float *oPdf, Scratch &scratch,
                              cudaStream_t s) {
   if (n == 0) return cudaSuccess;
@@ -878,7 +878,6 @@ cudaError_t gather_and_order(const float4 *posIdx, uint32_t n, const float4 *P, 
   permute_kernel<<<blocks_for(n, 256), 256, 0, s>>>(valsOut, n, P, D, pdf, oP, oD, oPdf);
   count_launch();
   fix_ties_kernel<<<blocks_for(n, 256), 256, 0, s>>>(keys64Out, n, oP, oD, oPdf);
-  (void)leafCount;
   return cudaGetLastError();
 }
 
