@@ -67,19 +67,6 @@ __device__ __forceinline__ PathShared &path_shared() {
   return *reinterpret_cast<PathShared *>(smem);
 }
 
-// Does a vertex end the run of distances that add up (and what scales them)?
-// The factor of lastDistance, or -1 where it starts again at zero.
-__device__ __forceinline__ float vertex_factor(const PathSegmentRecord &cur) {
-  if (!cur.isDelta && cur.roughness >= 0.3f) return -1.0f;
-  if (cur.eta == 1.0f) return 1.0f;
-  const float cosThetaI = seg_dot(cur.nx, cur.ny, cur.nz, cur.dox, cur.doy, cur.doz);
-  const float cosThetaO = seg_dot(cur.nx, cur.ny, cur.nz, cur.dix, cur.diy, cur.diz);
-  return fabsf(cosThetaI / (cosThetaO * cur.eta));
-}
-__device__ __forceinline__ float vertex_step(const PathSegmentRecord &cur, const PathSegmentRecord &nxt) {
-  const float ex = nxt.px - cur.px, ey = nxt.py - cur.py, ez = nxt.pz - cur.pz;
-  return sqrtf(seg_dot(ex, ey, ez, ex, ey, ez));
-}
 // distance of vertex i: from the next vertex that starts again (or the path's
 // last) down, as the reference's loop from the path's end does
 template <typename Step, typename Factor>
@@ -95,49 +82,6 @@ __device__ __forceinline__ float vertex_distance(int i, int n, float maxDistance
 }
 // rr's reciprocal where div_by takes it
 __device__ __forceinline__ float rr_reciprocal(float rr) { return rr >= 1e-12f && rr <= 1e12f ? rcp_newton(rr) : 0.0f; }
-// The contribution of a path's tail seg[1, n) at its vertex seg[0]
-// (path_prepare_samples' inner loop); rcp(s) is rr_reciprocal of s.rr.
-template <typename Rcp>
-__device__ __forceinline__ void vertex_contribution(const PathSegmentRecord *seg, int n, PathFlags fl, Rcp rcp,
-                                                    float c[3]) {
-  const float maxThroughput = 10.0f;
-  float t[3] = {1.0f, 1.0f, 1.0f}, previousRR = 1.0f;
-  c[0] = c[1] = c[2] = 0.0f;
-  for (int j = 1; j < n; ++j) {
-    const PathSegmentRecord &s = seg[j], &p = seg[j - 1];
-    float ct[3], dc[3] = {s.dc[0], s.dc[1], s.dc[2]};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      t[k] = t[k] * p.tw[k];
-      ct[k] = t[k] < maxThroughput ? t[k] : maxThroughput;  // embree::min
-      c[k] += ct[k] * s.sc[k];
-      if (!fl.rrAffectsDirectContribution) dc[k] *= previousRR;
-    }
-    if (j == 1 && !fl.useNEEMiWeights) {
-      if (fl.guideDirectLight)
-        for (int k = 0; k < 3; ++k) c[k] += ct[k] * dc[k];
-    } else if (j > 1 || fl.guideDirectLight) {
-      for (int k = 0; k < 3; ++k) c[k] += (ct[k] * s.miWeight) * dc[k];
-    }
-    V3 q = mk(t[0] * s.sw[0], t[1] * s.sw[1], t[2] * s.sw[2]);
-    q = s.rr > 0.f ? div3_by(q, s.rr, rcp(s)) : mk(0.0f, 0.0f, 0.0f);
-    t[0] = q.x;
-    t[1] = q.y;
-    t[2] = q.z;
-    previousRR = s.rr;
-  }
-}
-// samples only on non-delta vertices sampled by a non-delta technique
-__device__ __forceinline__ bool vertex_eligible(const PathSegmentRecord &cur) {
-  return !cur.isDelta && cur.roughness > 0.01f;
-}
-__device__ __forceinline__ float vertex_pdf(const PathSegmentRecord &cur) {
-  const float minPDF = 0.1f;
-  return minPDF < cur.pdfDirectionIn ? cur.pdfDirectionIn : minPDF;  // std::max
-}
-__device__ __forceinline__ bool made_sample(const float c[3], float distance) {
-  return (c[0] > 0.0f || c[1] > 0.0f || c[2] > 0.0f) && distance > 0;
-}
 
 // The path of the tile that item x belongs to, among paths [a, z).
 __device__ __forceinline__ int path_of(const PathTile &S, uint32_t x, int a, int z) {
@@ -271,7 +215,7 @@ __device__ __noinline__ uint32_t staged_samples(int buffer, const PathSegmentRec
       const float pdf = vertex_pdf(cur);
       const uint32_t flags = cur.volumeScatter ? 2u : 0u;  // EInsideVolume
       float *w = words + v * kRecordWords;
-      w[kWeight] = ((c[0] + c[1] + c[2]) / 3.0f) / pdf;
+      w[kWeight] = sample_weight(c, pdf);
       w[kPdf] = pdf;
       w[kDistance] = distance;
       w[kFlags] = u2f(flags);
@@ -361,7 +305,7 @@ __device__ __noinline__ uint32_t long_path(const PathSegmentRecord *seg, int n, 
         o.dy = cur.diy;
         o.dz = cur.diz;
         o.pdf = vertex_pdf(cur);
-        o.weight = ((c[0] + c[1] + c[2]) / 3.0f) / o.pdf;
+        o.weight = sample_weight(c, o.pdf);
         o.distance = vertex_distance(i, n, maxDistance, step, factor);
         o.flags = cur.volumeScatter ? 2u : 0u;
         out[total + made_before(S, uint32_t(x))] = o;

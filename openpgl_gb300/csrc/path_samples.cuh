@@ -43,77 +43,94 @@ PGL_HD float seg_dot(float ax, float ay, float az, float bx, float by, float bz)
   return ax * bx + (ay * by + az * bz);
 }
 
+// Does a vertex end the run of distances that add up (and what scales them)?
+// The factor of lastDistance, or -1 where it starts again at zero.
+PGL_HD float vertex_factor(const PathSegmentRecord &cur) {
+  if (!cur.isDelta && cur.roughness >= 0.3f) return -1.0f;
+  if (cur.eta == 1.0f) return 1.0f;
+  const float cosThetaI = seg_dot(cur.nx, cur.ny, cur.nz, cur.dox, cur.doy, cur.doz);
+  const float cosThetaO = seg_dot(cur.nx, cur.ny, cur.nz, cur.dix, cur.diy, cur.diz);
+  return fabsf(cosThetaI / (cosThetaO * cur.eta));
+}
+PGL_HD float vertex_step(const PathSegmentRecord &cur, const PathSegmentRecord &nxt) {
+  const float ex = nxt.px - cur.px, ey = nxt.py - cur.py, ez = nxt.pz - cur.pz;
+  return sqrtf(seg_dot(ex, ey, ez, ex, ey, ez));
+}
+// The contribution of a path's tail seg[1, n) at its vertex seg[0]
+// (Russian roulette's quotients from rcp(s), see div3_by; on the host they divide).
+template <typename Rcp>
+PGL_HD void vertex_contribution(const PathSegmentRecord *seg, int n, PathFlags fl, Rcp rcp, float c[3]) {
+  const float maxThroughput = 10.0f;
+  float t[3] = {1.0f, 1.0f, 1.0f}, previousRR = 1.0f;
+  c[0] = c[1] = c[2] = 0.0f;
+  for (int j = 1; j < n; ++j) {
+    const PathSegmentRecord &s = seg[j], &p = seg[j - 1];
+    float ct[3], dc[3] = {s.dc[0], s.dc[1], s.dc[2]};
+    for (int k = 0; k < 3; ++k) {
+      t[k] = t[k] * p.tw[k];
+      ct[k] = t[k] < maxThroughput ? t[k] : maxThroughput;  // embree::min
+      c[k] += ct[k] * s.sc[k];
+      if (!fl.rrAffectsDirectContribution) dc[k] *= previousRR;
+    }
+    if (j == 1 && !fl.useNEEMiWeights) {
+      if (fl.guideDirectLight)
+        for (int k = 0; k < 3; ++k) c[k] += ct[k] * dc[k];
+    } else if (j > 1 || fl.guideDirectLight) {
+      for (int k = 0; k < 3; ++k) c[k] += (ct[k] * s.miWeight) * dc[k];
+    }
+    V3 q = mk(t[0] * s.sw[0], t[1] * s.sw[1], t[2] * s.sw[2]);
+    q = s.rr > 0.f ? div3_by(q, s.rr, rcp(s)) : mk(0.0f, 0.0f, 0.0f);
+    t[0] = q.x;
+    t[1] = q.y;
+    t[2] = q.z;
+    previousRR = s.rr;
+  }
+}
+// samples only on non-delta vertices sampled by a non-delta technique
+PGL_HD bool vertex_eligible(const PathSegmentRecord &cur) {
+  return !cur.isDelta && cur.roughness > 0.01f;
+}
+PGL_HD float vertex_pdf(const PathSegmentRecord &cur) {
+  const float minPDF = 0.1f;
+  return minPDF < cur.pdfDirectionIn ? cur.pdfDirectionIn : minPDF;  // std::max
+}
+// whether a vertex with these makes a sample, and its weight
+PGL_HD bool made_sample(const float c[3], float distance) {
+  return (c[0] > 0.0f || c[1] > 0.0f || c[2] > 0.0f) && distance > 0;
+}
+PGL_HD float sample_weight(const float c[3], float pdf) { return ((c[0] + c[1] + c[2]) / 3.0f) / pdf; }
+
 // Appends the samples of path seg[0, n) to out (at most cap, counted from
 // out's start); returns how many it would write (the count is exact even
-// when cap is smaller).
-PGL_HD uint32_t path_prepare_samples(const PathSegmentRecord *seg, int n, float maxDistance, PathFlags fl,
+// when cap is smaller).  The host's form; the kernel deals the vertices out.
+inline uint32_t path_prepare_samples(const PathSegmentRecord *seg, int n, float maxDistance, PathFlags fl,
                                      PGLSampleRecord *out, uint32_t cap) {
-  const float minPDF = 0.1f, maxThroughput = 10.0f;
   uint32_t made = 0;
   float lastDistance = 0.0f;
   for (int i = n - 2; i >= 0; --i) {
     const PathSegmentRecord &cur = seg[i];
-    const PathSegmentRecord &nxt = seg[i + 1];
-    const float ex = nxt.px - cur.px, ey = nxt.py - cur.py, ez = nxt.pz - cur.pz;
-    const float currentDistance = sqrtf(seg_dot(ex, ey, ez, ex, ey, ez));
-    const float distance = fminf(currentDistance + lastDistance, 2.0f * maxDistance);
-    if (!cur.isDelta && cur.roughness >= 0.3f) {
-      lastDistance = 0.0f;
-    } else {
-      lastDistance = distance;
-      if (cur.eta != 1.0f) {
-        const float cosThetaI = seg_dot(cur.nx, cur.ny, cur.nz, cur.dox, cur.doy, cur.doz);
-        const float cosThetaO = seg_dot(cur.nx, cur.ny, cur.nz, cur.dix, cur.diy, cur.diz);
-        lastDistance *= fabsf(cosThetaI / (cosThetaO * cur.eta));
-      }
+    const float distance = fminf(vertex_step(cur, seg[i + 1]) + lastDistance, 2.0f * maxDistance);
+    const float factor = vertex_factor(cur);
+    lastDistance = factor == -1.0f ? 0.0f : distance * factor;
+    if (!vertex_eligible(cur)) continue;
+    float c[3];
+    vertex_contribution(&cur, n - i, fl, [](const PathSegmentRecord &) { return 0.0f; }, c);
+    if (!made_sample(c, distance)) continue;
+    if (made < cap) {
+      PGLSampleRecord r;
+      r.px = cur.px;
+      r.py = cur.py;
+      r.pz = cur.pz;
+      r.dx = cur.dix;
+      r.dy = cur.diy;
+      r.dz = cur.diz;
+      r.pdf = vertex_pdf(cur);
+      r.weight = sample_weight(c, r.pdf);
+      r.distance = distance;
+      r.flags = cur.volumeScatter ? 2u : 0u;  // EInsideVolume
+      out[made] = r;
     }
-    // samples only on non-delta vertices sampled by a non-delta technique
-    if (!cur.isDelta && cur.roughness > 0.01f) {
-      const float pdf = minPDF < cur.pdfDirectionIn ? cur.pdfDirectionIn : minPDF;  // std::max
-      float t[3] = {1.0f, 1.0f, 1.0f}, c[3] = {0.0f, 0.0f, 0.0f};
-      float previousRR = 1.0f;
-      for (int j = i + 1; j < n; ++j) {
-        const PathSegmentRecord &s = seg[j];
-        const PathSegmentRecord &p = seg[j - 1];
-        for (int k = 0; k < 3; ++k) t[k] = t[k] * p.tw[k];
-        float ct[3];
-        for (int k = 0; k < 3; ++k) ct[k] = t[k] < maxThroughput ? t[k] : maxThroughput;  // embree::min
-        for (int k = 0; k < 3; ++k) c[k] += ct[k] * s.sc[k];
-        float dc[3] = {s.dc[0], s.dc[1], s.dc[2]};
-        if (!fl.rrAffectsDirectContribution)
-          for (int k = 0; k < 3; ++k) dc[k] *= previousRR;
-        if (j == i + 1 && !fl.useNEEMiWeights) {
-          if (fl.guideDirectLight)
-            for (int k = 0; k < 3; ++k) c[k] += ct[k] * dc[k];
-        } else if (j > i + 1 || fl.guideDirectLight) {
-          for (int k = 0; k < 3; ++k) c[k] += (ct[k] * s.miWeight) * dc[k];
-        }
-        for (int k = 0; k < 3; ++k) t[k] = t[k] * s.sw[k];
-        if (s.rr > 0.f) {
-          for (int k = 0; k < 3; ++k) t[k] /= s.rr;
-        } else {
-          t[0] = t[1] = t[2] = 0.0f;
-        }
-        previousRR = s.rr;
-      }
-      if ((c[0] > 0.0f || c[1] > 0.0f || c[2] > 0.0f) && distance > 0) {
-        if (made < cap) {
-          PGLSampleRecord r;
-          r.px = cur.px;
-          r.py = cur.py;
-          r.pz = cur.pz;
-          r.dx = cur.dix;
-          r.dy = cur.diy;
-          r.dz = cur.diz;
-          r.weight = ((c[0] + c[1] + c[2]) / 3.0f) / pdf;
-          r.pdf = pdf;
-          r.distance = distance;
-          r.flags = cur.volumeScatter ? 2u : 0u;  // EInsideVolume
-          out[made] = r;
-        }
-        ++made;
-      }
-    }
+    ++made;
   }
   return made;
 }
