@@ -39,9 +39,18 @@ namespace pgl {
 constexpr int kDqtThreads = 512;
 constexpr uint32_t kDqtNodes = 768;      // trees up to this many nodes are held in shared memory
 constexpr uint32_t kDqtPool = 10240;     // words for the shares and the masks of a chunk
-constexpr uint32_t kDqtRects = 512;      // leaves whose rectangles are held in shared memory
-constexpr uint32_t kDqtList = 16;        // leaves of a sample that a thread keeps
-constexpr uint32_t kDqtDense = 40;       // leaves up to which a chunk's shares are a matrix
+// Two Updates of 200,000 samples in regions of 16,000, us, by leaves whose rectangles are held
+// in shared memory / leaves of a sample that a thread keeps / leaves up to which a chunk's
+// shares are a matrix (the others at their values below):
+//                                 rects 128  256  512   list 8   16   32   matrix 0   20   40   80
+//   default arguments                  1700 1650 1640     1630 1640 1660     1820 1640 1640 1790
+//   threshold 0.1, 6 levels            1870 1890 1880     1880 1880 1880     2300 1990 1880 1870
+//   threshold 0.002                    2630 2630 2540     2550 2540 2540     2790 2540 2540 2720
+//   threshold 0.02                     2200 2200 2190     2140 2190 2360     2450 2200 2190 2340
+//   footprint 4                        6990 6910 6900     6890 6900 6920     9860 6890 6900 5060
+// (more leaves in the matrix mean fewer samples per chunk: the wide boxes of the last row gain,
+// the ordinary ones lose.)
+constexpr uint32_t kDqtRects = 512, kDqtList = 16, kDqtDense = 40;
 constexpr int kDqtLevels = 40;           // levels of a tree at most
 
 struct DqtShared {

@@ -1303,7 +1303,8 @@ __device__ __forceinline__ EStepShape estep_shape(int cnt, const EmTuning &tune)
 // 30 FP32 operations and about as many issue slots per lobe, 15 cycles per
 // sample at 32 lobes alone on an SM.  A lane per lobe vector and sample, with
 // shuffles between the vectors, held a leaf of 30 lobes that no other block
-// helps at 39 cycles per sample and pass; it now takes 28.
+// helps at 39 cycles per sample and pass; it now takes 28 (18 to 23 at 17 to 24
+// lobes; 12 to 14 where other blocks help).
 template <int kCnt>
 __device__ __noinline__ void produce_estep_rows(const EmShared &S, const EStepShape &e, const float4 *dirw,
                                                 uint32_t count, uint32_t chunk, float *G, int t, int nthreads) {

@@ -8,7 +8,7 @@
 // the blocks before it (a decoupled look-back over per-block counts).
 // 852,000 segments of 131,072 paths are 116 MB in and 17 MB out (19 us at the
 // copy rate).  Two passes with a thread per path took 192 us, this one 77 us
-// (paths of 1 to 24 segments 752 -> 251 us, of 1 or 2 25 -> 25 us): a tile stages
+// (paths of 1 to 24 segments 752 -> 246 us, of 1 or 2 25 -> 25 us): a tile stages
 // for 5,500 cycles, prepares and deals out its vertices for 6,000, adds their
 // contributions for 8,700 (bound by shared-memory reads, 15 words per step) and
 // waits 6,900 for its place in the output.
