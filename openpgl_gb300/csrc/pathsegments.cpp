@@ -273,6 +273,9 @@ OPENPGL_CORE_INTERFACE bool pglPathSegmentsPrepareSamplesDevice(const PGLPathSeg
                                                                 void *cudaStream) {
   PGL_PS_TRY
   if (numPaths >= 0xFFFFFFFFull) throw std::runtime_error("too many paths for one call");
+  // the records are staged by copies of 8 and 16 bytes
+  if (numPaths > 0 && reinterpret_cast<uintptr_t>(dSegments) % alignof(PGLPathSegmentData) != 0)
+    throw std::runtime_error("path segments that are not aligned as PGLPathSegmentData");
   Context &c = Context::get();
   cudaStream_t st = cudaStream ? static_cast<cudaStream_t>(cudaStream) : c.stream;
   const size_t bytes = path_counts_bytes(uint32_t(numPaths));
